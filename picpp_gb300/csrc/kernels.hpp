@@ -137,6 +137,30 @@ void launch_scale(cudaStream_t s, double* v, const double* w, double sc, long lo
 void launch_div(cudaStream_t s, double* v, const double* w, double d, long long n);
 void launch_combine(cudaStream_t s, double* x, const double* V, long long ld, int k, const double* y, double scale,
                     int accumulate, long long n);
+// A whole FP64 GMRES solve in one cooperative launch (gmres_grid.cuh)
+constexpr int kGmresMaxCols = 128;    // Krylov columns its shared-memory triangles reach
+struct GmresArgs {
+    GridP g;
+    OpCoef oc;
+    const double* mu;
+    const double* b;
+    double* x;
+    double* V;        // basis, cols + 1 vectors of 3N
+    double* mx;       // mu v of the operator, 3N
+    double* w;        // vector being orthogonalised, 3N
+    double* r;        // residual, 3N (restarted)
+    double* part;     // partial sums, kNumSM x 2 (cols + 3)
+    unsigned* bar;    // [0] barrier arrivals, [1] set when a barrier gave up
+    double* out;      // GmresOut
+    double tol;       // restarted: relative residual; reference: its bound on the estimate
+    int cols;         // columns per cycle (restarted) / most columns (reference)
+    int max_iter;     // restarted: iterations in all; reference: its limit on n
+    int reference;
+};
+enum GmresOut { kGmStatus = 0, kGmIterations, kGmRestarts, kGmRel, kGmOutLen };
+enum GmresStatus { kGmOk = 0, kGmNotConverged, kGmNonFiniteSystem, kGmNonFiniteResidual };
+cudaError_t launch_gmres_grid(cudaStream_t s, const GmresArgs& a);
+
 // Offsets of the inner solve's FP64 scalars (one array): [0] |v|^2, [1]
 // |v|, then the Hessenberg columns (column j at h + j (S + 1), rows 0..j),
 // the squared norms of the new basis vectors, the least-squares solution y,

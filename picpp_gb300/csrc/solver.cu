@@ -27,7 +27,7 @@ OpCoef make_opcoef(const GridP& g) {
 
 void krylov_free(Krylov& k) {
     cudaFree(k.V); cudaFree(k.Z); cudaFree(k.w); cudaFree(k.mx); cudaFree(k.r); cudaFree(k.hdev); cudaFree(k.ydev);
-    cudaFree(k.part); cudaFree(k.scal);
+    cudaFree(k.part); cudaFree(k.scal); cudaFree(k.bar);
     cudaFree(k.mu32); cudaFree(k.V32); cudaFree(k.w32); cudaFree(k.mx32); cudaFree(k.h32); cudaFree(k.part32);
     cudaFree(k.cnt32);
     k = Krylov{};
@@ -62,6 +62,7 @@ pic_status ensure(SolveCtx& c, int cap, long long L) {
     CKS(cudaMalloc(&k.ydev, sizeof(double) * (size_t)(cap + 2)));
     CKS(cudaMalloc(&k.part, sizeof(double) * (size_t)(cap + 2) * 1024));
     CKS(cudaMalloc(&k.scal, sizeof(double) * 16));
+    CKS(cudaMalloc(&k.bar, sizeof(unsigned) * 2));
     k.cap = cap;
     k.L = L;
     return PIC_OK;
@@ -83,6 +84,58 @@ pic_status check_finite(SolveCtx& c, const double* a, long long n) {
     CKS(cudaStreamSynchronize(c.s));
     if (bad) return err(c, PIC_ERR_NUMERIC, "non-finite value in the Maxwell system");
     return PIC_OK;
+}
+
+// The plain methods with at most kGmresMaxCols Krylov columns: one launch per
+// solve, one read-back.  false: the caller takes the kernel-per-operation form.
+bool one_launch(const GridP& g, const pic_solve_opts& o) {
+    if (o.method == PIC_GMRES_RESTARTED) return (o.restart > 0 ? o.restart : 30) <= kGmresMaxCols;
+    return o.method == PIC_GMRES_REFERENCE && (o.max_iter > 0 ? o.max_iter : 50) <= kGmresMaxCols + 2;
+}
+
+pic_status gmres_one_launch(SolveCtx& c, const OpCoef& oc, const double* rhs, double* x, const pic_solve_opts& o,
+                            pic_solve_info* info) {
+    const GridP& g = *c.g;
+    const long long L = 3 * g.N;
+    const bool ref = o.method == PIC_GMRES_REFERENCE;
+    GmresArgs a{};
+    a.reference = ref ? 1 : 0;
+    pic_status st;
+    if (ref) {
+        const int maxIter = o.max_iter > 0 ? o.max_iter : 50;
+        if ((st = ensure(c, maxIter + 2, L)) != PIC_OK) return st;
+        // matrixDimension of the reference: 3 x its cells (the physical ones of a wall box)
+        const long long dim = g.wall ? 3LL * (g.nx - 2) * g.ny * g.nz : L;
+        a.tol = std::max(o.tol / (double)dim, 1e-15);
+        a.max_iter = (int)std::min<long long>(maxIter, dim + 3);
+        a.cols = std::max(1, a.max_iter - 2);
+    } else {
+        a.cols = std::max(1, o.restart > 0 ? o.restart : 30);
+        if ((st = ensure(c, a.cols + 1, L)) != PIC_OK) return st;
+        a.max_iter = o.max_iter > 0 ? o.max_iter : 1000;
+        a.tol = o.tol > 0 ? o.tol : 1e-8;
+    }
+    Krylov& k = *c.k;
+    a.g = g;
+    a.oc = oc;
+    a.mu = c.mu; a.b = rhs; a.x = x;
+    a.V = k.V; a.mx = k.mx; a.w = k.w; a.r = k.r;
+    a.part = k.part; a.bar = k.bar; a.out = k.scal;
+    CKS(launch_gmres_grid(c.s, a));
+    double out[kGmOutLen] = {};
+    unsigned bar[2] = {};
+    CKS(cudaMemcpyAsync(out, k.scal, sizeof(out), cudaMemcpyDeviceToHost, c.s));
+    CKS(cudaMemcpyAsync(bar, k.bar, sizeof(bar), cudaMemcpyDeviceToHost, c.s));
+    CKS(cudaStreamSynchronize(c.s));
+    if (bar[1]) return err(c, PIC_ERR_CUDA, "a grid barrier of the field solve ran out");
+    if (out[kGmStatus] == kGmNonFiniteSystem) return err(c, PIC_ERR_NUMERIC, "non-finite value in the Maxwell system");
+    if (out[kGmStatus] == kGmNonFiniteResidual) return err(c, PIC_ERR_NUMERIC, "non-finite residual");
+    if (info) {
+        info->iterations = (int)out[kGmIterations];
+        info->restarts = (int)out[kGmRestarts];
+        info->rel_residual = out[kGmRel];
+    }
+    return out[kGmStatus] == kGmOk ? PIC_OK : err(c, PIC_ERR_NOT_CONVERGED, "GMRES did not reach the tolerance");
 }
 
 // generalizedMinimalResidualMethod (PIC++/specialmath.cpp:367-671) semantics.
@@ -430,9 +483,10 @@ pic_status gmres_restarted(SolveCtx& c, const OpCoef& oc, const double* b, doubl
 
 pic_status krylov_solve(SolveCtx& c, const double* rhs, double* x, const pic_solve_opts& o, pic_solve_info* info) {
     const long long L = 3 * c.g->N;
-    pic_status st = check_finite(c, rhs, L);
+    const bool one = one_launch(*c.g, o);   // (that kernel checks its system itself)
+    pic_status st = one ? PIC_OK : check_finite(c, rhs, L);
     if (st != PIC_OK) return st;
-    st = check_finite(c, c.mu, 3 * L);
+    if (!one) st = check_finite(c, c.mu, 3 * L);
     if (st != PIC_OK) return st;
     const OpCoef oc = make_opcoef(*c.g);
     cudaEvent_t e0, e1;
@@ -441,8 +495,12 @@ pic_status krylov_solve(SolveCtx& c, const double* rhs, double* x, const pic_sol
     cudaEventRecord(e0, c.s);
     if (info) *info = pic_solve_info{};
     switch (o.method) {
-        case PIC_GMRES_REFERENCE: st = gmres_reference(c, oc, rhs, x, o, info); break;
-        case PIC_GMRES_RESTARTED: st = gmres_restarted(c, oc, rhs, x, o, info); break;
+        case PIC_GMRES_REFERENCE:
+            st = one ? gmres_one_launch(c, oc, rhs, x, o, info) : gmres_reference(c, oc, rhs, x, o, info);
+            break;
+        case PIC_GMRES_RESTARTED:
+            st = one ? gmres_one_launch(c, oc, rhs, x, o, info) : gmres_restarted(c, oc, rhs, x, o, info);
+            break;
         case PIC_FGMRES_LEARNED:
             if (!c.net || !c.net->ready()) {
                 st = err(c, PIC_ERR_STATE, "learned preconditioner not initialised (pic_nn_init / pic_nn_set_params)");

@@ -19,6 +19,7 @@ struct Krylov {
     double* ydev = nullptr;   // combination coefficients
     double* part = nullptr;   // reduction partials, (cap + 2) * 1024
     double* scal = nullptr;   // scalar results
+    unsigned* bar = nullptr;  // grid barrier of the one-launch solve
     int cap = 0;
     int zcap = 0;
     long long L = 0;
