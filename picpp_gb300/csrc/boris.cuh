@@ -98,6 +98,32 @@ __device__ __forceinline__ void velocity_fast(const float mom[3], float m, float
     v[0] = mom[0] * r; v[1] = mom[1] * r; v[2] = mom[2] * r;
 }
 
+// The same with every rounding fixed (fmadd, common.cuh): the fused tile
+// kernel's push, whose bits so do not depend on the code around it.
+__device__ __forceinline__ float cross1(float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); }
+__device__ __forceinline__ void boris_fixed(float q, float m, float dt, float beta, const float e[3], const float b[3],
+                                           float mom[3]) {
+    const float s = q * dt * 0.5f;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) mom[d] = __fmaf_rn(e[d], s, mom[d]);
+    const float p2 = __fmaf_rn(mom[2], mom[2], __fmaf_rn(mom[0], mom[0], __fmul_rn(mom[1], mom[1])));
+    const float bs = __fmul_rn(beta * m, rsqrtf(__fmaf_rn(m, m, p2)));
+    const float b2 = __fmaf_rn(b[2], b[2], __fmaf_rn(b[0], b[0], __fmul_rn(b[1], b[1])));
+    const float f = __fmul_rn(2.0f, rsqrtf(__fmaf_rn(__fmul_rn(bs, bs), b2, 1.0f)));
+    const float pxb[3] = {cross1(mom[1], b[2], mom[2], b[1]), cross1(mom[2], b[0], mom[0], b[2]),
+                          cross1(mom[0], b[1], mom[1], b[0])};
+    const float tm[3] = {__fmaf_rn(pxb[0], bs, mom[0]), __fmaf_rn(pxb[1], bs, mom[1]), __fmaf_rn(pxb[2], bs, mom[2])};
+    const float txb[3] = {cross1(tm[1], b[2], tm[2], b[1]), cross1(tm[2], b[0], tm[0], b[2]),
+                          cross1(tm[0], b[1], tm[1], b[0])};
+    const float fb = __fmul_rn(f, bs);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) mom[d] = __fadd_rn(mom[d], __fmaf_rn(e[d], s, __fmul_rn(txb[d], fb)));
+}
+__device__ __forceinline__ void velocity_fixed(const float mom[3], float m, float v[3]) {
+    const float r = rsqrtf(__fmaf_rn(mom[2], mom[2], __fmaf_rn(mom[1], mom[1], __fmaf_rn(m, m, __fmul_rn(mom[0], mom[0])))));
+    v[0] = __fmul_rn(mom[0], r); v[1] = __fmul_rn(mom[1], r); v[2] = __fmul_rn(mom[2], r);
+}
+
 // Dispatch: fast forms for FP32 state, reference sequence for FP64.
 template <typename TP>
 __device__ __forceinline__ void boris_t(TP q, TP m, TP dt, TP beta, const TP e[3], const TP b[3], TP mom[3]) {
@@ -112,6 +138,20 @@ template <typename TP>
 __device__ __forceinline__ void velocity_t(const TP mom[3], TP m, TP v[3]) { velocity<TP>(mom, m, v); }
 template <>
 __device__ __forceinline__ void velocity_t<float>(const float mom[3], float m, float v[3]) { velocity_fast(mom, m, v); }
+// ... and of the fused tile kernel (FP32 with fixed roundings).
+template <typename TP>
+__device__ __forceinline__ void boris_tile(TP q, TP m, TP dt, TP beta, const TP e[3], const TP b[3], TP mom[3]) {
+    boris<TP>(q, m, dt, beta, e, b, mom);
+}
+template <>
+__device__ __forceinline__ void boris_tile<float>(float q, float m, float dt, float beta, const float e[3],
+                                                  const float b[3], float mom[3]) {
+    boris_fixed(q, m, dt, beta, e, b, mom);
+}
+template <typename TP>
+__device__ __forceinline__ void velocity_tile(const TP mom[3], TP m, TP v[3]) { velocity<TP>(mom, m, v); }
+template <>
+__device__ __forceinline__ void velocity_tile<float>(const float mom[3], float m, float v[3]) { velocity_fixed(mom, m, v); }
 
 template <typename TP, typename TF>
 __global__ void __launch_bounds__(256) k_boris_push(GridP g, PartView<TP> p, TP q, TP m,

@@ -37,6 +37,7 @@
 #pragma once
 #include "boris.cuh"
 #include "types.cuh"
+#include <type_traits>
 
 namespace pic {
 
@@ -49,7 +50,7 @@ constexpr int kTileThreads = PIC_TILE_THREADS;
 #endif
 
 template <typename TP>
-__device__ __forceinline__ TP lerp(TP a, TP b, TP w) { return a + w * (b - a); }
+__device__ __forceinline__ TP lerp(TP a, TP b, TP w) { return fmadd<TP>(w, subr<TP>(b, a), a); }
 
 // Trilinear value of one staggered component from the staged block: base is
 // the block index of the lower corner, sy/sz the strides, (wx, wy, wz) the
@@ -88,12 +89,36 @@ __device__ __forceinline__ void set_defer_bits(unsigned* __restrict__ mask, long
 // (momentum_collecting.cpp:200-230): Jx at (c, j+dj, k+dk) -> slot 2dk+dj,
 // Jy at (i+di, c, k+dk) -> 4+2dk+di, Jz at (i+di, j+dj, c) -> 8+2dj+di.
 template <typename TP>
-__device__ __forceinline__ void segment_slots(TP Fx, TP Fy, TP Fz, TP Wx, TP Wy, TP Wz, TP a[12]) {
-    const TP ux = TP(1) - Wx, uy = TP(1) - Wy, uz = TP(1) - Wz;
-    a[0] = Fx * uy * uz; a[1] = Fx * Wy * uz; a[2] = Fx * uy * Wz; a[3] = Fx * Wy * Wz;
-    a[4] = Fy * ux * uz; a[5] = Fy * Wx * uz; a[6] = Fy * ux * Wz; a[7] = Fy * Wx * Wz;
-    a[8] = Fz * ux * uy; a[9] = Fz * Wx * uy; a[10] = Fz * ux * Wy; a[11] = Fz * Wx * Wy;
+__device__ __forceinline__ void segment_factors(TP Fx, TP Fy, TP Fz, TP Wx, TP Wy, TP Wz, TP b[12], TP f[12]) {
+    const TP ux = subr<TP>(TP(1), Wx), uy = subr<TP>(TP(1), Wy), uz = subr<TP>(TP(1), Wz);
+    b[0] = b[2] = mulr<TP>(Fx, uy); b[1] = b[3] = mulr<TP>(Fx, Wy);
+    b[4] = b[6] = mulr<TP>(Fy, ux); b[5] = b[7] = mulr<TP>(Fy, Wx);
+    b[8] = b[10] = mulr<TP>(Fz, ux); b[9] = b[11] = mulr<TP>(Fz, Wx);
+    f[0] = f[1] = f[4] = f[5] = uz; f[2] = f[3] = f[6] = f[7] = Wz;
+    f[8] = f[9] = uy; f[10] = f[11] = Wy;
 }
+template <typename TP>
+__device__ __forceinline__ void segment_slots(TP Fx, TP Fy, TP Fz, TP Wx, TP Wy, TP Wz, TP a[12]) {
+    TP b[12], f[12];
+    segment_factors<TP>(Fx, Fy, Fz, Wx, Wy, Wz, b, f);
+#pragma unroll
+    for (int q = 0; q < 12; ++q) a[q] = mulr<TP>(b[q], f[q]);
+}
+// ... added to the terms in a[].
+template <typename TP>
+__device__ __forceinline__ void segment_add(TP Fx, TP Fy, TP Fz, TP Wx, TP Wy, TP Wz, TP a[12]) {
+    TP b[12], f[12];
+    segment_factors<TP>(Fx, Fy, Fz, Wx, Wy, Wz, b, f);
+#pragma unroll
+    for (int q = 0; q < 12; ++q) a[q] = fmadd<TP>(b[q], f[q], a[q]);
+}
+
+// Weight of the upper neighbour at the middle s / 2 of a segment, r cells from
+// the cell it is in: s / (2 d) - r, h = 1 / (2 d).
+template <typename TP>
+__device__ __forceinline__ TP weight_from(TP s, TP d2, TP h, TP r) { return divd<TP>(s, d2, h) - r; }
+template <>
+__device__ __forceinline__ float weight_from<float>(float s, float, float h, float r) { return __fmaf_rn(s, h, -r); }
 
 // Segmented sum of a[] over runs of lanes with equal key; returns true in the
 // first lane of each run, which then holds the run's totals.
@@ -252,11 +277,13 @@ __device__ __forceinline__ void stage_particle(ChunkBuf<TP>* buf, const PartView
 // Tristan mover's reflection and escape and the zigzag wall term
 // (mover.cpp:744-772, momentum_collecting.cpp:93-99); a particle that
 // escaped deposits its current and is marked (cell -1) for the next sort.
-template <typename TP, typename TF, int CT, bool kWall>
+// kParts: several CTAs per tile (parts > 1); without it the loop keeps no
+// register for the stride (64 are all it has).
+template <typename TP, typename TF, int CT, bool kWall, bool kParts>
 __global__ void __launch_bounds__(kTileThreads, PIC_TILE_MIN_BLOCKS) k_push_deposit_tile(GridP g, TileGeom t, TileShape s, SpeciesSet<TP> S,
                                                                        const TF* __restrict__ E, const TF* __restrict__ B,
                                                                        double* __restrict__ Jpart, float fx_scale,
-                                                                       double inv_dt) {
+                                                                       double inv_dt, int nparts) {
     constexpr bool kFixed = sizeof(TP) == sizeof(float);   // FP32 particles: fixed-point block
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int fx = CT ? CT + 4 : s.fx, fy = CT ? CT + 4 : s.fy, fz = CT ? CT + 4 : s.fz;
@@ -284,10 +311,14 @@ __global__ void __launch_bounds__(kTileThreads, PIC_TILE_MIN_BLOCKS) k_push_depo
     const TP dx = TP(g.dx), dy = TP(g.dy), dz = TP(g.dz);
     const TP idx = TP(g.idx), idy = TP(g.idy), idz = TP(g.idz);
     const TP vol = dx * dy * dz;
+    const int parts = kParts ? nparts : 1;
     const int ey = CT ? 1 : (g.y3 ? 1 : 0), ez = CT ? 1 : (g.z3 ? 1 : 0);
     const int fsy = ey ? fx : 0, fsz = ez ? fx * fy : 0;
 
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    // `parts` CTAs share a tile: each takes every parts-th chunk of its
+    // particles and writes a partial block of its own
+    for (int work = blockIdx.x; work < ntiles * parts; work += gridDim.x) {
+        const int tile = work / parts, part = work - tile * parts;
         const int ti = tile % t.ntx, tj = (tile / t.ntx) % t.nty, tk = tile / (t.ntx * t.nty);
         const int lox = ti * tx, loy = tj * ty, loz = tk * tz;
         for (int e = threadIdx.x; e < F; e += blockDim.x) {
@@ -311,14 +342,17 @@ __global__ void __launch_bounds__(kTileThreads, PIC_TILE_MIN_BLOCKS) k_push_depo
             const TP q = S.q[sp], m = S.m[sp];
             const TP beta = q * dt / (TP(2) * m);
             const TP fcd = q * S.w[sp] / vol;
-            const long long pb = S.off[sp][(long long)tile * T3], pe = S.off[sp][(long long)(tile + 1) * T3];
+            // (unsigned: a species holds fewer than 2^31 particles)
+            using IDX = std::conditional_t<kParts, unsigned, long long>;
+            const IDX pb = S.off[sp][(long long)tile * T3] + part * blockDim.x;
+            const IDX pe = S.off[sp][(long long)(tile + 1) * T3];
             // CTA-uniform chunk loop: warp w takes particles cb + 32 w + lane.
             // Each warp's next chunk is copied into its shared buffer while
             // it pushes the current one (the first before the loop).
             if (pb + threadIdx.x < pe) stage_particle(sBuf, P, pb + threadIdx.x, lane);
             cp_async_commit();
-            for (long long cb = pb; cb < pe; cb += blockDim.x) {
-                const long long n = cb + threadIdx.x;
+            for (IDX cb = pb; cb < pe; cb += parts * blockDim.x) {
+                const IDX n = cb + threadIdx.x;
                 TP aB[12];
                 TP s1[6] = {TP(0), TP(0), TP(0), TP(0), TP(0), TP(0)};   // F1 and W1 of the old-side segment
                 int keyA = -1 - lane, keyB = -1 - lane;   // lanes outside a reduction keep unique keys
@@ -329,7 +363,7 @@ __global__ void __launch_bounds__(kTileThreads, PIC_TILE_MIN_BLOCKS) k_push_depo
                 const int cell = n < pe ? sBuf->cell[lane] : -1;
                 TP ox = sBuf->a[0][lane], oy = sBuf->a[1][lane], oz = sBuf->a[2][lane];
                 TP mom[3] = {sBuf->a[3][lane], sBuf->a[4][lane], sBuf->a[5][lane]};
-                if (n + blockDim.x < pe) stage_particle(sBuf, P, n + blockDim.x, lane);
+                if (n + parts * blockDim.x < pe) stage_particle(sBuf, P, n + parts * blockDim.x, lane);
                 cp_async_commit();
                 // (an escaped particle of a wall box waits with cell -1 for the sort)
                 if (n < pe && (!kWall || cell >= 0)) {
@@ -365,19 +399,19 @@ __global__ void __launch_bounds__(kTileThreads, PIC_TILE_MIN_BLOCKS) k_push_depo
                         b3[0] = tri<TP, TF>(sF + 3 * F, c0 + cys + czs, fsy, fsz, ox, wcy, wcz);
                         b3[1] = tri<TP, TF>(sF + 4 * F, c0 + cxs + czs, fsy, fsz, wcx, wny, wcz);
                         b3[2] = tri<TP, TF>(sF + 5 * F, c0 + cxs + cys, fsy, fsz, wcx, wcy, wnz);
-                        boris_t<TP>(q, m, dt, beta, e3, b3, mom);
+                        boris_tile<TP>(q, m, dt, beta, e3, b3, mom);
                         TP v[3];
-                        velocity_t<TP>(mom, m, v);
+                        velocity_tile<TP>(mom, m, v);
                         int ni = i, nj = j, nk = k;
                         int wall_r = 0;
                         if constexpr (kWall) {
-                            wall_r = tristan_wall_x<TP>(g, ni, ox, (v[0] * dt) * idx);
+                            wall_r = tristan_wall_to<TP>(g, ni, ox, fmadd<TP>(mulr<TP>(v[0], dt), idx, ox));
                             if (wall_r & 1) { mom[0] = -mom[0]; v[0] = -v[0]; }   // reflectMomentumX
                         } else {
-                            advance_axis<TP>(ox, ni, (v[0] * dt) * idx, g.nx);
+                            advance_axis<TP>(ox, ni, mulr<TP>(v[0], dt), idx, g.nx);
                         }
-                        advance_axis<TP>(oy, nj, (v[1] * dt) * idy, g.ny);
-                        advance_axis<TP>(oz, nk, (v[2] * dt) * idz, g.nz);
+                        advance_axis<TP>(oy, nj, mulr<TP>(v[1], dt), idy, g.ny);
+                        advance_axis<TP>(oz, nk, mulr<TP>(v[2], dt), idz, g.nz);
                         P.px[n] = mom[0]; P.py[n] = mom[1]; P.pz[n] = mom[2];
                         P.ox[n] = ox; P.oy[n] = oy; P.oz[n] = oz;
                         auto shift = [](int nw, int old, int nn) {
@@ -397,9 +431,9 @@ __global__ void __launch_bounds__(kTileThreads, PIC_TILE_MIN_BLOCKS) k_push_depo
                         const int bz = (ez ? lk + shift(nk, k, g.nz) : 0) + hz;
                         // zigzag split (zig_axis, momentum_collecting.cpp:91-221) in the
                         // new cell's frame: old position P, relay R, relay shift r
-                        const TP X = ox * dx, Y = oy * dy, Z = oz * dz;
-                        TP PX = X - v[0] * dt;
-                        const TP PY = Y - v[1] * dt, PZ = Z - v[2] * dt;
+                        const TP X = mulr<TP>(ox, dx), Y = mulr<TP>(oy, dy), Z = mulr<TP>(oz, dz);
+                        TP PX = subr<TP>(X, mulr<TP>(v[0], dt));
+                        const TP PY = fmadd<TP>(-v[1], dt, Y), PZ = fmadd<TP>(-v[2], dt, Z);
                         if constexpr (kWall) {
                             if (ni == kTristanWallNode && v[0] > TP(0) && PX < TP(0)) PX = -PX;
                         }
@@ -421,11 +455,11 @@ __global__ void __launch_bounds__(kTileThreads, PIC_TILE_MIN_BLOCKS) k_push_depo
                             const TP F1y = divd<TP>(fcd * (RY - PY), dt, idt);
                             const TP F1z = divd<TP>(fcd * (RZ - PZ), dt, idt);
                             const TP F2x = divd<TP>(fcd * (X - RX), dt, idt);
-                            const TP F2y = fcd * v[1] - F1y, F2z = fcd * v[2] - F1z;
+                            const TP F2y = fmadd<TP>(fcd, v[1], -F1y), F2z = fmadd<TP>(fcd, v[2], -F1z);
                             const TP hxx = TP(0.5) * idx, hyy = TP(0.5) * idy, hzz = TP(0.5) * idz;
-                            const TP W1x = divd<TP>(PX + RX, TP(2) * dx, hxx) - TP(rx);
-                            const TP W1y = ey ? divd<TP>(PY + RY, TP(2) * dy, hyy) - TP(ry) : TP(0);
-                            const TP W1z = ez ? divd<TP>(PZ + RZ, TP(2) * dz, hzz) - TP(rz) : TP(0);
+                            const TP W1x = weight_from<TP>(PX + RX, TP(2) * dx, hxx, TP(rx));
+                            const TP W1y = ey ? weight_from<TP>(PY + RY, TP(2) * dy, hyy, TP(ry)) : TP(0);
+                            const TP W1z = ez ? weight_from<TP>(PZ + RZ, TP(2) * dz, hzz, TP(rz)) : TP(0);
                             const TP W2x = divd<TP>(X + RX, TP(2) * dx, hxx);
                             const TP W2y = ey ? divd<TP>(Y + RY, TP(2) * dy, hyy) : TP(0);
                             const TP W2z = ez ? divd<TP>(Z + RZ, TP(2) * dz, hzz) : TP(0);
@@ -457,10 +491,7 @@ __global__ void __launch_bounds__(kTileThreads, PIC_TILE_MIN_BLOCKS) k_push_depo
                 // the old-side pass is left to the particles that crossed (its
                 // 12 values are formed only then, from the six kept in s1)
                 if (keyA == keyB && keyA >= 0) {
-                    TP aA[12];
-                    segment_slots<TP>(s1[0], s1[1], s1[2], s1[3], s1[4], s1[5], aA);
-#pragma unroll
-                    for (int q2 = 0; q2 < 12; ++q2) aB[q2] += aA[q2];
+                    segment_add<TP>(s1[0], s1[1], s1[2], s1[3], s1[4], s1[5], aB);
                     keyA = -1 - lane;
                 }
                 const bool crossed = __any_sync(0xffffffffu, keyA >= 0);
@@ -485,7 +516,7 @@ __global__ void __launch_bounds__(kTileThreads, PIC_TILE_MIN_BLOCKS) k_push_depo
             }
         }
         __syncthreads();
-        double* dst = Jpart + (long long)tile * 3 * JC;
+        double* dst = Jpart + (long long)work * 3 * JC;
         if (kFixed) {
             // the exact block sums as 64-bit integers (k_assemble_j adds
             // them exactly and scales once per cell): integer operations
@@ -569,11 +600,12 @@ __global__ void __launch_bounds__(256) k_push_deposit_deferred(GridP g, SpeciesS
 // periodic images visited in a fixed order (deterministic).  FP32 particles:
 // the partials are 64-bit fixed-point integers, summed exactly and scaled by
 // inv_scale (a power of two) once; FP64 particles: FP64 partials.
-template <typename TP>
+template <typename TP, bool kParts>
 __global__ void __launch_bounds__(256) k_assemble_j(GridP g, TileGeom t, TileShape s, const double* __restrict__ Jpart,
                                                     const double* __restrict__ Jfix, double* __restrict__ J,
-                                                    double inv_scale) {
+                                                    double inv_scale, int nparts) {
     constexpr bool kFixed = sizeof(TP) == sizeof(float);
+    const int parts = kParts ? nparts : 1;
     const long long JC = s.jcells;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.N;
          c += (long long)gridDim.x * blockDim.x) {
@@ -613,16 +645,18 @@ __global__ void __launch_bounds__(256) k_assemble_j(GridP g, TileGeom t, TileSha
                 for (int d = 0; d < cnt[2]; ++d) {
                     long long tile = ((long long)cand_t[2][d] * t.nty + cand_t[1][b]) * t.ntx + cand_t[0][a];
                     long long e = ((long long)cand_l[2][d] * s.jy + cand_l[1][b]) * s.jx + cand_l[0][a];
-                    const double* src = Jpart + tile * 3 * JC;
-                    if constexpr (kFixed) {
-                        const long long* srci = reinterpret_cast<const long long*>(src);
-                        iacc[0] += srci[e];
-                        iacc[1] += srci[JC + e];
-                        iacc[2] += srci[2 * JC + e];
-                    } else {
-                        acc[0] += src[e];
-                        acc[1] += src[JC + e];
-                        acc[2] += src[2 * JC + e];
+                    for (int r = 0; r < parts; ++r) {
+                        const double* src = Jpart + (tile * parts + r) * 3 * JC;
+                        if constexpr (kFixed) {
+                            const long long* srci = reinterpret_cast<const long long*>(src);
+                            iacc[0] += srci[e];
+                            iacc[1] += srci[JC + e];
+                            iacc[2] += srci[2 * JC + e];
+                        } else {
+                            acc[0] += src[e];
+                            acc[1] += src[JC + e];
+                            acc[2] += src[2 * JC + e];
+                        }
                     }
                 }
         if constexpr (kFixed) {

@@ -79,6 +79,18 @@ template <typename T> __device__ __forceinline__ T divd(T a, T d, T invd);
 template <> __device__ __forceinline__ double divd<double>(double a, double d, double) { return a / d; }
 template <> __device__ __forceinline__ float divd<float>(float a, float, float invd) { return a * invd; }
 
+// Fixed roundings of the FP32 push: a * b + c fused, a * b and a - b each
+// rounded, whatever code stands around them.  Left to the compiler, the
+// choice of which product of a sum is fused changes with the surrounding code,
+// and a particle within a rounding of a cell face then takes the other zigzag
+// path.  (FP64: separate operations, as the oracle's.)
+template <typename T> __device__ __forceinline__ T fmadd(T a, T b, T c) { return a * b + c; }
+template <> __device__ __forceinline__ float fmadd<float>(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+template <typename T> __device__ __forceinline__ T mulr(T a, T b) { return a * b; }
+template <> __device__ __forceinline__ float mulr<float>(float a, float b) { return __fmul_rn(a, b); }
+template <typename T> __device__ __forceinline__ T subr(T a, T b) { return a - b; }
+template <> __device__ __forceinline__ float subr<float>(float a, float b) { return __fsub_rn(a, b); }
+
 template <typename T> __device__ __forceinline__ T dev_sqrt(T x);
 template <> __device__ __forceinline__ double dev_sqrt<double>(double x) { return sqrt(x); }
 template <> __device__ __forceinline__ float dev_sqrt<float>(float x) { return sqrtf(x); }
@@ -128,11 +140,10 @@ __device__ __forceinline__ void cell_w(T u, int c, int n, int idx[2], T w[2]) {
     w[0] = wl; w[1] = wr;
 }
 
-// Advance an in-cell offset by du cells and wrap the cell index; identical
-// rule to the oracle's advance_axis.
+// Wraps the offset un of a particle that moved within or out of cell c, and
+// the cell index; identical rule to the oracle's advance_axis.
 template <typename T>
-__device__ __forceinline__ void advance_axis(T& u, int& c, T du, int n) {
-    T un = u + du;
+__device__ __forceinline__ void settle_axis(T un, T& u, int& c, int n) {
     T s = dev_floor(un);
     un = un - s;
     int ci = c + (int)s;
@@ -142,6 +153,11 @@ __device__ __forceinline__ void advance_axis(T& u, int& c, T du, int n) {
     if ((unsigned)w >= (unsigned)n) w = wrap_any(ci, n);   // moved farther than one box length
     c = w;
 }
+// Advance an in-cell offset by du cells / by a length a over cells of size 1 / inv.
+template <typename T>
+__device__ __forceinline__ void advance_axis(T& u, int& c, T du, int n) { settle_axis<T>(u + du, u, c, n); }
+template <typename T>
+__device__ __forceinline__ void advance_axis(T& u, int& c, T a, T inv, int n) { settle_axis<T>(fmadd<T>(a, inv, u), u, c, n); }
 
 constexpr int kRedThreads = 256;
 

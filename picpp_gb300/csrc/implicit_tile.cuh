@@ -357,8 +357,9 @@ __device__ __noinline__ EB6<T> gather_eb_global(const GridP g, int i, int j, int
 // no FP64 conversion per gather).  kStaged: E and B staged in shared memory
 // next to the accumulators (right after a sort, h = 0); a separate
 // instantiation keeps the hot loop's code small.
-template <typename T, typename A, bool kStaged>
-__global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(GridP g, TileGeom t, ImpBlock bk,
+// kSplit: t is the geometry of sub-tiles, cut from the sort's tiles by sp.
+template <typename T, typename A, bool kStaged, bool kSplit>
+__global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(GridP g, TileGeom t, TileSplit sp, ImpBlock bk,
                                                                        ImpSpecies<T> S, const T* __restrict__ E,
                                                                        const T* __restrict__ B,
                                                                        double* __restrict__ J, double* __restrict__ mu,
@@ -392,6 +393,11 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int ti = tile % t.ntx, tj = (tile / t.ntx) % t.nty, tk = tile / (t.ntx * t.nty);
         const int x0 = ti * t.tx, y0 = tj * t.ty, z0 = tk * t.tz;
+        // first key of the sub-tile: its tile's, plus its place in it
+        const int key0 = kSplit ? ((((tk / sp.sz) * (t.nty / sp.sy) + tj / sp.sy) * (t.ntx / sp.sx) + ti / sp.sx) *
+                                       (sp.sx * sp.sy * sp.sz) +
+                                   ((tk % sp.sz) * sp.sy + tj % sp.sy) * sp.sx + ti % sp.sx) * T3
+                                : tile * T3;
         for (int e = threadIdx.x; e < tot; e += blockDim.x) sN[e] = A(0);
         if (kStaged) {   // with h = 0 the blocks cover exactly the stencils of the tile's own cells
             for (int e = threadIdx.x; e < bk.NB; e += blockDim.x) {
@@ -416,7 +422,7 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
             const double cq = qs * ws * ivol;
             const double cm = -(ws * g.theta * g.dt * g.dt * 2 * PI_D * qs * qs / ms) * ivol;
             for (int lc = warp; lc < T3; lc += nwarps) {
-                const int kk = tile * T3 + lc;
+                const int kk = key0 + lc;
                 const int b0 = off[kk], b1 = off[kk + 1];
                 // Right after a sort the particles of this key lie in the key's cell:
                 // the tensor-core sums of all its chunks accumulate and reach the
@@ -619,10 +625,12 @@ struct MoverBlock {
 // and its bit set in S.defer: k_implicit_push_deferred moves it from the
 // FP64 grids (the kernel itself calls nothing out of line, which would cost
 // its hot loop register spills).  Same arithmetic as k_implicit_push.
-template <typename T, bool kWall>
+// kParts: several CTAs per tile (parts > 1); without it the loop keeps no
+// register for the stride.
+template <typename T, bool kWall, bool kParts>
 __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g, TileGeom t, MoverBlock mb, ImpSpecies<T> S,
                                                             const double* __restrict__ E, const double* __restrict__ B,
-                                                            const double* __restrict__ Et) {
+                                                            const double* __restrict__ Et, int nparts) {
     extern __shared__ __align__(16) unsigned char mv_smem[];
     // FP32: E^theta and B^n, gathered two or three times per particle, as
     // float4 nodes / cells (one 16-byte load per corner); E^n, gathered
@@ -661,7 +669,10 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
     const int nn[3] = {g.nx, g.ny, g.nz};
     const T dxT = T(g.dx);
     const T redt = T((1.0 - g.eta) * g.dt);
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int parts = kParts ? nparts : 1;
+    // `parts` CTAs share a tile: each takes every parts-th run of blockDim particles
+    for (int work = blockIdx.x; work < ntiles * parts; work += gridDim.x) {
+        const int tile = work / parts, part = work - tile * parts;
         const int ti = tile % t.ntx, tj = (tile / t.ntx) % t.nty, tk = tile / (t.ntx * t.nty);
         const int x0 = ti * t.tx, y0 = tj * t.ty, z0 = tk * t.tz;
         __syncthreads();   // previous tile's particles are done with the blocks
@@ -695,16 +706,17 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
             const T beta = T(0.5 * qs * g.dt / ms);
             const T qdt = T(qs * g.dt);
             const T mm = T(ms);
-            const int b0 = S.off[s][tile * T3], b1 = S.off[s][(tile + 1) * T3];
+            const int b0 = S.off[s][tile * T3] + part * blockDim.x, b1 = S.off[s][(tile + 1) * T3];
+            const int step = kParts ? parts * blockDim.x : blockDim.x;
             if (b0 + (int)threadIdx.x < b1) stage(p, b0 + threadIdx.x);
             cp_async_commit();
-            for (int n = b0 + threadIdx.x; n < b1; n += blockDim.x) {
+            for (int n = b0 + threadIdx.x; n < b1; n = b1 - n > step ? n + step : b1) {   // (no int overflow)
                 cp_async_wait_all();   // this thread's particle n (its own slot)
                 const int bdim = blockDim.x, me = threadIdx.x;
                 const int cell_n = sPreCell[me];
                 const T pu[3] = {sPre[0 * bdim + me], sPre[1 * bdim + me], sPre[2 * bdim + me]};
                 const T pm[3] = {sPre[3 * bdim + me], sPre[4 * bdim + me], sPre[5 * bdim + me]};
-                if (n + bdim < b1) stage(p, n + bdim);
+                if (b1 - n > step) stage(p, n + step);
                 cp_async_commit();
                 int ci[3];
                 decode(g, cell_n, ci[0], ci[1], ci[2]);

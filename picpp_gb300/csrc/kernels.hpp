@@ -4,6 +4,7 @@
 // (grid.cu).
 #pragma once
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <vector>
 #include "common.cuh"
 #include "types.cuh"
@@ -28,6 +29,14 @@ inline int red_blocks(long long n) {
     return (int)b;
 }
 
+// CTAs that share one tile's particles in the fused explicit kernel and the
+// tiled mover: a box with fewer tiles than two CTAs per SM would leave SMs
+// idle, so the tiles are cut into as many parts as still run in one wave.
+inline int tile_parts(const TileGeom& t) {
+    const int n = t.ntx * t.nty * t.ntz;
+    return std::max(1, 2 * kNumSM / n);
+}
+
 template <typename T>
 struct PK {
     // with GridP::wall the B half step first sets the ghost column left of
@@ -37,15 +46,15 @@ struct PK {
     static void boris_push(cudaStream_t s, const GridP& g, PartView<T> p, double q, double m, const void* E,
                            const void* B);
     static void zigzag(cudaStream_t s, const GridP& g, PartView<T> p, double q, double m, double w, double* J);
-    // fused gather/push/deposit over tiles (boris_tile.cuh); smem bytes and
-    // grid size chosen by the caller
+    // fused gather/push/deposit over tiles (boris_tile.cuh), `parts` CTAs
+    // and partial blocks per tile (tile_parts); smem bytes from the caller
     static void push_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileShape& sh,
                                    const SpeciesSet<T>& S, const void* E, const void* B, double* Jpart, double* Jfix,
-                                   int grid, size_t smem);
+                                   int parts, size_t smem);
     // J from the tile partials and Jfix; inv_scale = 1 / fixed_scale for FP32
     // particles (integer partials), unused for FP64
     static void assemble_j(cudaStream_t s, const GridP& g, const TileGeom& t, const TileShape& sh, const double* Jpart,
-                           const double* Jfix, double* J, double inv_scale);
+                           const double* Jfix, double* J, double inv_scale, int parts);
     static float fixed_scale(const GridP& g, const SpeciesSet<T>& S);
     static size_t tile_smem_bytes(const TileShape& sh);
     static void implicit_deposit(cudaStream_t s, const GridP& g, PartView<T> p, double q, double m, double w,
@@ -55,7 +64,8 @@ struct PK {
     // tile-major sorted particles
     static ImpBlock implicit_block(const GridP& g, const TileGeom& t, int h);
     static size_t implicit_tile_smem(const ImpBlock& bk);
-    static void implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const ImpBlock& bk,
+    static void implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileSplit& sp,
+                                       const ImpBlock& bk,
                                        const ImpSpecies<T>& S, const T* E, const T* B, double* J,
                                        double* mu, double* rho, double* Pi);
     // tiled mover (implicit_tile.cuh): fields staged per tile; needs

@@ -189,28 +189,27 @@ size_t PK<T>::tile_smem_bytes(const TileShape& sh) {
 template <typename T>
 void PK<T>::push_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileShape& sh,
                                const SpeciesSet<T>& S, const void* E, const void* B, double* Jpart, double* Jfix,
-                               int grid, size_t smem) {
+                               int parts, size_t smem) {
     static bool attr_set = false;
     if (!attr_set) {
-        cudaFuncSetAttribute(k_push_deposit_tile<T, T, 8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(k_push_deposit_tile<T, T, 0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(k_push_deposit_tile<T, T, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        for (auto* k : {k_push_deposit_tile<T, T, 8, false, false>, k_push_deposit_tile<T, T, 8, false, true>,
+                        k_push_deposit_tile<T, T, 0, false, false>, k_push_deposit_tile<T, T, 0, false, true>,
+                        k_push_deposit_tile<T, T, 0, true, false>, k_push_deposit_tile<T, T, 0, true, true>})
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         attr_set = true;
     }
     const bool cube8 = t.tx == 8 && t.ty == 8 && t.tz == 8 && g.y3 && g.z3 && sh.fx == 12 && sh.fy == 12 &&
                        sh.fz == 12 && sh.jx == 12 && sh.jy == 12 && sh.jz == 12;
     const float fx_scale = fixed_scale(g, S);
     const double inv_dt = 1.0 / g.dt;
+    const int grid = std::min(t.ntx * t.nty * t.ntz * parts, kNumSM * 8);
     // a wall box runs its own instantiation (run-time tile shape)
-    if (g.wall)
-        k_push_deposit_tile<T, T, 0, true><<<grid, kTileThreads, smem, s>>>(g, t, sh, S, (const T*)E, (const T*)B, Jpart,
-                                                                           fx_scale, inv_dt);
-    else if (cube8)
-        k_push_deposit_tile<T, T, 8, false><<<grid, kTileThreads, smem, s>>>(g, t, sh, S, (const T*)E, (const T*)B, Jpart,
-                                                                            fx_scale, inv_dt);
-    else
-        k_push_deposit_tile<T, T, 0, false><<<grid, kTileThreads, smem, s>>>(g, t, sh, S, (const T*)E, (const T*)B, Jpart,
-                                                                            fx_scale, inv_dt);
+    auto* whole = g.wall ? k_push_deposit_tile<T, T, 0, true, false>
+                         : cube8 ? k_push_deposit_tile<T, T, 8, false, false> : k_push_deposit_tile<T, T, 0, false, false>;
+    auto* shared = g.wall ? k_push_deposit_tile<T, T, 0, true, true>
+                          : cube8 ? k_push_deposit_tile<T, T, 8, false, true> : k_push_deposit_tile<T, T, 0, false, true>;
+    auto* kernel = parts > 1 ? shared : whole;
+    kernel<<<grid, kTileThreads, smem, s>>>(g, t, sh, S, (const T*)E, (const T*)B, Jpart, fx_scale, inv_dt, parts);
     // the particles it left over: one thread per mask word
     long long words = 1;
     for (int q = 0; q < S.ns; ++q) words = std::max(words, (S.p[q].n + 31) / 32 + 1);
@@ -233,8 +232,9 @@ float PK<T>::fixed_scale(const GridP& g, const SpeciesSet<T>& S) {
 
 template <typename T>
 void PK<T>::assemble_j(cudaStream_t s, const GridP& g, const TileGeom& t, const TileShape& sh, const double* Jpart,
-                       const double* Jfix, double* J, double inv_scale) {
-    k_assemble_j<T><<<grid_for(g.N, 256), 256, 0, s>>>(g, t, sh, Jpart, Jfix, J, inv_scale);
+                       const double* Jfix, double* J, double inv_scale, int parts) {
+    auto* kernel = parts > 1 ? k_assemble_j<T, true> : k_assemble_j<T, false>;
+    kernel<<<grid_for(g.N, 256), 256, 0, s>>>(g, t, sh, Jpart, Jfix, J, inv_scale, parts);
 }
 
 template <typename T>
@@ -271,13 +271,14 @@ size_t PK<T>::implicit_tile_smem(const ImpBlock& bk) {
 }
 
 template <typename T>
-void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const ImpBlock& bk,
+void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileSplit& sp, const ImpBlock& bk,
                                    const ImpSpecies<T>& S, const T* E, const T* B, double* J, double* mu,
                                    double* rho, double* Pi) {
     static bool attr_set = false;
     if (!attr_set) {
-        cudaFuncSetAttribute(k_implicit_deposit_tile<T, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        cudaFuncSetAttribute(k_implicit_deposit_tile<T, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        for (auto* k : {k_implicit_deposit_tile<T, T, true, false>, k_implicit_deposit_tile<T, T, true, true>,
+                        k_implicit_deposit_tile<T, T, false, false>})
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         attr_set = true;
     }
     const size_t smem = implicit_tile_smem(bk);
@@ -285,8 +286,10 @@ void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeo
     const int ntiles = t.ntx * t.nty * t.ntz;
     const int grid = ntiles < kNumSM * (per_sm > 0 ? per_sm : 1) ? ntiles : kNumSM * (per_sm > 0 ? per_sm : 1);
     constexpr int nt = imp_threads<T>();
-    if (bk.stage) k_implicit_deposit_tile<T, T, true><<<grid, nt, smem, s>>>(g, t, bk, S, E, B, J, mu, rho, Pi);
-    else k_implicit_deposit_tile<T, T, false><<<grid, nt, smem, s>>>(g, t, bk, S, E, B, J, mu, rho, Pi);
+    const bool split = sp.sx * sp.sy * sp.sz > 1;
+    auto* kernel = !bk.stage ? k_implicit_deposit_tile<T, T, false, false>
+                   : split ? k_implicit_deposit_tile<T, T, true, true> : k_implicit_deposit_tile<T, T, true, false>;
+    kernel<<<grid, nt, smem, s>>>(g, t, sp, bk, S, E, B, J, mu, rho, Pi);
 }
 
 template <typename T>
@@ -311,25 +314,25 @@ bool PK<T>::implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& 
     if (smem > 227 * 1024) return false;
     static bool attr_set = false;
     if (!attr_set) {
-        cudaFuncSetAttribute(k_implicit_push_tile<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        cudaFuncSetAttribute(k_implicit_push_tile<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        for (auto* k : {k_implicit_push_tile<T, false, false>, k_implicit_push_tile<T, false, true>,
+                        k_implicit_push_tile<T, true, false>, k_implicit_push_tile<T, true, true>})
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         attr_set = true;
     }
     const int per_sm = (int)((228 * 1024) / (smem + 1024));
-    const int ntiles = t.ntx * t.nty * t.ntz;
     const int cap = kNumSM * (per_sm > 0 ? per_sm : 1);
+    const int parts = tile_parts(t);
+    const int nwork = t.ntx * t.nty * t.ntz * parts;
     // the wall rules are a separate instantiation: the periodic mover keeps
     // none of their code in its loop
     // the particles it left over: one thread per mask word
     long long words = 1;
     for (int q = 0; q < S.ns; ++q) words = std::max(words, (S.p[q].n + 31) / 32);
-    if (g.wall) {
-        k_implicit_push_tile<T, true><<<ntiles < cap ? ntiles : cap, kMoverThreads, smem, s>>>(g, t, mb, S, E, B, Et);
-        k_implicit_push_deferred<T, true><<<grid_for(words, 128), 128, 0, s>>>(g, S, E, B, Et);
-    } else {
-        k_implicit_push_tile<T, false><<<ntiles < cap ? ntiles : cap, kMoverThreads, smem, s>>>(g, t, mb, S, E, B, Et);
-        k_implicit_push_deferred<T, false><<<grid_for(words, 128), 128, 0, s>>>(g, S, E, B, Et);
-    }
+    auto* kernel = g.wall ? (parts > 1 ? k_implicit_push_tile<T, true, true> : k_implicit_push_tile<T, true, false>)
+                          : (parts > 1 ? k_implicit_push_tile<T, false, true> : k_implicit_push_tile<T, false, false>);
+    kernel<<<nwork < cap ? nwork : cap, kMoverThreads, smem, s>>>(g, t, mb, S, E, B, Et, parts);
+    if (g.wall) k_implicit_push_deferred<T, true><<<grid_for(words, 128), 128, 0, s>>>(g, S, E, B, Et);
+    else k_implicit_push_deferred<T, false><<<grid_for(words, 128), 128, 0, s>>>(g, S, E, B, Et);
     return true;
 }
 

@@ -21,6 +21,13 @@ struct TileGeom {
     int lx, ly, lz;      // log2 of the extents when all three are powers of two, else -1
 };
 
+// Sub-tiles of the staged implicit deposit: each tile of the sort key cut into
+// sx, sy, sz pieces per axis whose cells are consecutive keys (y is cut only
+// when z is cut down to single layers, x only when y is).
+struct TileSplit {
+    int sx, sy, sz;
+};
+
 // Shared-memory blocks of the fused explicit kernel (boris_tile.cuh).
 struct TileShape {
     int fx, fy, fz;   // staged field block (tile + 1 halo each side on active axes)

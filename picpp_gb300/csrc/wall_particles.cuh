@@ -84,9 +84,8 @@ __device__ __forceinline__ int wall_final_x(const GridP& g, int& c, T& u, T disp
 // this step, then leaves).  c, u: cell and offset of x^n on entry, of the
 // result on return.
 template <typename T>
-__device__ __forceinline__ int tristan_wall_x(const GridP& g, int& c, T& u, T disp) {
+__device__ __forceinline__ int tristan_wall_to(const GridP& g, int& c, T& u, T s) {   // s = u + disp
     const int W = kTristanWallNode;
-    const T s = u + disp;
     const T fl = dev_floor(s);
     int cn = c + (int)fl;
     T un = s - fl;
@@ -101,6 +100,10 @@ __device__ __forceinline__ int tristan_wall_x(const GridP& g, int& c, T& u, T di
     c = cn;
     u = un;
     return r;
+}
+template <typename T>
+__device__ __forceinline__ int tristan_wall_x(const GridP& g, int& c, T& u, T disp) {
+    return tristan_wall_to<T>(g, c, u, u + disp);
 }
 
 // True for a particle that left a wall box through the open boundary: its
