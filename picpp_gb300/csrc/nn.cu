@@ -70,22 +70,31 @@ void conv(cudaStream_t s, int ci, int co, const bf16* x, const bf16* W, const fl
 #undef PIC_CONV
 }
 
-template <int CI, int CO>
+// CC input channels per CTA: as many as 96 accumulators a thread hold.
+template <int CI, int CO, int CC>
 void wgrad_t(cudaStream_t s, const bf16* x, const bf16* g, Dims d, float* dW, float* db) {
     static bool attr = false;
-    const size_t sm = (size_t)nn::kWgVox * (CI + CO) * sizeof(float);
+    const int sm = 2 * nn::wg_stage(CC, CO);
     if (!attr) {
-        cudaFuncSetAttribute(nn::k_wgrad<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaFuncSetAttribute(nn::k_wgrad<CI, CO, CC>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
         attr = true;
     }
-    dim3 grid((unsigned)((d.vox() + nn::kWgVox - 1) / nn::kWgVox), 27);
-    nn::k_wgrad<CI, CO><<<grid, 256, sm, s>>>(x, g, d, dW, db);
+    const int bricks = d.N * ((d.D + nn::kWgD - 1) / nn::kWgD) * ((d.H + nn::kWgH - 1) / nn::kWgH) *
+                       ((d.W + nn::kWgW - 1) / nn::kWgW);
+    // one CTA per SM: with two, the sums they add at their end cost as much as
+    // the second hides (forward and backward of 4 x 16x64x64 voxels 1,219
+    // against 1,207 us).  Before: the same pass 9,020 us, its weight gradients
+    // 0.90 (16/16), 2.68 (48/16), 1.01 (96/32) and 0.26 ms (32/32) each on
+    // CUDA cores; 0.028, 0.075, 0.036 and 0.031 ms here.
+    const int most = std::max(1, kNumSM / (CI / CC));
+    nn::k_wgrad<CI, CO, CC><<<dim3(std::min(bricks, most), CI / CC), nn::kWgThreads, sm, s>>>(x, g, d, dW, db);
 }
 
 void wgrad(cudaStream_t s, int ci, int co, const bf16* x, const bf16* g, Dims d, float* dW, float* db) {
-#define PIC_WG(A, B) \
-    if (ci == A && co == B) return wgrad_t<A, B>(s, x, g, d, dW, db)
-    PIC_WG(16, 16); PIC_WG(16, 32); PIC_WG(32, 32); PIC_WG(32, 64); PIC_WG(64, 64); PIC_WG(96, 32); PIC_WG(48, 16);
+#define PIC_WG(A, B, C) \
+    if (ci == A && co == B) return wgrad_t<A, B, C>(s, x, g, d, dW, db)
+    PIC_WG(16, 16, 16); PIC_WG(16, 32, 16); PIC_WG(32, 32, 32); PIC_WG(32, 64, 16); PIC_WG(64, 64, 16);
+    PIC_WG(96, 32, 32); PIC_WG(48, 16, 48);
 #undef PIC_WG
 }
 
@@ -479,7 +488,7 @@ pic_status Net::loss_grad_host(cudaStream_t s, int n, int d, int h, int w, const
     forward(s, *b);
     NCK(cudaMemsetAsync(loss_, 0, sizeof(double), s));
     NCK(cudaMemsetAsync(g_, 0, sizeof(float) * param_count(), s));
-    nn::k_mse<<<gs(V * 16), 256, 0, s>>>(b->out, b->tgt, b->A0, V, 16, 3, 1.f, loss_);
+    nn::k_mse<<<gs(V), 256, 0, s>>>(b->out, b->tgt, b->A0, V, 16, 3, 1.f, loss_);
     backward(s, *b);
     NCK(cudaMemcpyAsync(loss, loss_, sizeof(double), cudaMemcpyDeviceToHost, s));
     NCK(cudaMemcpyAsync(grad, g_, sizeof(float) * param_count(), cudaMemcpyDeviceToHost, s));

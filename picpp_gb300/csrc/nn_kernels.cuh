@@ -18,60 +18,133 @@ struct Dims {
     __host__ __device__ long long vox() const { return (long long)N * D * H * W; }
 };
 
-// dW[tap][co][ci] += sum_v x[v + off(tap)][ci] * gy[v][co], and (blocks of
-// tap 0) db[co] += sum_v gy[v][co]; FP32 partial sums over a chunk of 128
-// voxels per CTA, added with global atomics.
-constexpr int kWgVox = 128;
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(256) k_wgrad(const bf16* __restrict__ x, const bf16* __restrict__ gy, Dims dm,
-                                               float* __restrict__ dW, float* __restrict__ db) {
-    constexpr int PER = CIN * COUT / 256;
+// Weight gradients dW[tap][co][ci] += sum_v gy[v][co] x[v + off(tap)][ci] and
+// db[co] += sum_v gy[v][co] on the tensor cores: per tap a COUT x CC product
+// with the voxels as the inner dimension.
+//
+// A CTA takes output bricks of 2 x 4 x 16 voxels (d, h, w): the brick of gy
+// and, with its halo, of CC channels of x arrive in shared memory by cp.async,
+// the next brick's while this one is multiplied.  Warp (kd, kh) keeps the
+// three taps kw of its row in FP32 accumulators over all the CTA's bricks: a
+// tap is only another row of the staged x, so x is read from memory once for
+// 27 taps, and an A fragment (16 voxels of gy) serves three taps.  mma.sync
+// m16n8k16 (BF16 in, FP32 accumulator): tcgen05.mma takes at least 64 rows of
+// A, four times the 16 output channels of the layers that cost most, and its
+// operands would have to be transposed copies of these; both fragments come
+// from the voxel-major rows by ldmatrix.trans here.  Rows are padded by 16
+// bytes, so that eight of them lie in distinct banks.  Each CTA adds its sums
+// to dW once, at its end.
+// The FP32 kernel this replaces converted 128-voxel chunks of x for every tap
+// and multiplied them on CUDA cores, adding every chunk's sums with atomics;
+// times of both at the launcher (nn.cu).
+constexpr int kWgD = 2, kWgH = 4, kWgW = 16;                              // output brick
+constexpr int kWgXv = (kWgD + 2) * (kWgH + 2) * (kWgW + 2);               // its x with halo
+constexpr int kWgGv = kWgD * kWgH * kWgW;
+constexpr int kWgThreads = 9 * 32;
+__host__ __device__ constexpr int wg_row(int c) { return 2 * c + 16; }    // bytes of a padded row of c channels
+__host__ __device__ constexpr int wg_stage(int cc, int co) { return kWgXv * wg_row(cc) + kWgGv * wg_row(co); }
+
+__device__ __forceinline__ void wg_cp16(unsigned dst, const void* src, bool in) {
+    const int n = in ? 16 : 0;   // 0: zeros
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void wg_ldsm(unsigned r[4], unsigned addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void wg_mma(float d[4], const unsigned a[4], unsigned b0, unsigned b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+template <int CIN, int COUT, int CC>
+__global__ void __launch_bounds__(kWgThreads) k_wgrad(const bf16* __restrict__ x, const bf16* __restrict__ gy, Dims dm,
+                                                      float* __restrict__ dW, float* __restrict__ db) {
+    static_assert(CIN % CC == 0 && CC % 16 == 0 && COUT % 16 == 0, "channel counts");
+    constexpr int XS = wg_row(CC), GS = wg_row(COUT), kStage = wg_stage(CC, COUT);
     extern __shared__ __align__(16) unsigned char wg_smem[];
-    float* sx = reinterpret_cast<float*>(wg_smem);   // [kWgVox][CIN]
-    float* sg = sx + kWgVox * CIN;                   // [kWgVox][COUT]
-    const int tap = blockIdx.y;
-    const int kd = tap / 9 - 1, kh = (tap / 3) % 3 - 1, kw = tap % 3 - 1;
-    const long long V = dm.vox();
-    const long long v0 = (long long)blockIdx.x * kWgVox;
-    for (int e = threadIdx.x; e < kWgVox * CIN; e += 256) {
-        const int vi = e / CIN, ci = e % CIN;
-        const long long v = v0 + vi;
-        float val = 0.f;
-        if (v < V) {
-            const int w = (int)(v % dm.W), h = (int)((v / dm.W) % dm.H), d = (int)((v / ((long long)dm.W * dm.H)) % dm.D);
-            const long long nn = v / ((long long)dm.W * dm.H * dm.D);
-            const int dd = d + kd, hh = h + kh, ww = w + kw;
-            if (dd >= 0 && dd < dm.D && hh >= 0 && hh < dm.H && ww >= 0 && ww < dm.W)
-                val = __bfloat162float(x[(((nn * dm.D + dd) * dm.H + hh) * dm.W + ww) * CIN + ci]);
+    const unsigned base = (unsigned)__cvta_generic_to_shared(wg_smem);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int kd = warp / 3, kh = warp % 3;
+    const int c0 = blockIdx.y * CC;   // first input channel
+    const int bw = (dm.W + kWgW - 1) / kWgW, bh = (dm.H + kWgH - 1) / kWgH, bd = (dm.D + kWgD - 1) / kWgD;
+    const int bricks = dm.N * bd * bh * bw;
+    auto load = [&](int brick, int buf) {
+        const int w0 = brick % bw * kWgW, h0 = brick / bw % bh * kWgH, d0 = brick / (bw * bh) % bd * kWgD;
+        const long long n = brick / (bw * bh * bd);
+        const unsigned sx = base + buf * kStage, sg = sx + kWgXv * XS;
+        for (int e = threadIdx.x; e < kWgXv * (CC / 8); e += kWgThreads) {
+            const int p = e % (CC / 8), v = e / (CC / 8);
+            const int w = w0 + v % (kWgW + 2) - 1, h = h0 + v / (kWgW + 2) % (kWgH + 2) - 1,
+                      d = d0 + v / ((kWgW + 2) * (kWgH + 2)) - 1;
+            const bool in = w >= 0 && w < dm.W && h >= 0 && h < dm.H && d >= 0 && d < dm.D;
+            const long long vox = in ? ((n * dm.D + d) * dm.H + h) * dm.W + w : 0;
+            wg_cp16(sx + v * XS + p * 16, x + vox * CIN + c0 + p * 8, in);
         }
-        sx[e] = val;
-    }
-    for (int e = threadIdx.x; e < kWgVox * COUT; e += 256) {
-        const long long v = v0 + e / COUT;
-        sg[e] = v < V ? __bfloat162float(gy[v * COUT + e % COUT]) : 0.f;
-    }
-    __syncthreads();
-    float acc[PER];
+        for (int e = threadIdx.x; e < kWgGv * (COUT / 8); e += kWgThreads) {
+            const int p = e % (COUT / 8), v = e / (COUT / 8);
+            const int w = w0 + v % kWgW, h = h0 + v / kWgW % kWgH, d = d0 + v / (kWgW * kWgH);
+            const bool in = w < dm.W && h < dm.H && d < dm.D;
+            const long long vox = in ? ((n * dm.D + d) * dm.H + h) * dm.W + w : 0;
+            wg_cp16(sg + v * GS + p * 16, gy + vox * COUT + p * 8, in);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[3][COUT / 16][CC / 8][4] = {};
+    float bias = 0.f;
+    constexpr int kStrands = kWgThreads / COUT;   // threads per output channel of db
+    const int bco = threadIdx.x % COUT, strand = threadIdx.x / COUT;
+    // this lane's row and column in the four 8 x 8 matrices of a fragment load
+    const int r8 = lane & 7, m8 = lane >> 3;
+    const int ka = r8 + (m8 >> 1) * 8, ma = (m8 & 1) * 8;   // A: k, co
+    const int kb = r8 + (m8 & 1) * 8, nb8 = (m8 >> 1) * 8;  // B: k, ci
+    int buf = 0;
+    if ((int)blockIdx.x < bricks) load(blockIdx.x, 0);
+    for (int brick = blockIdx.x; brick < bricks; brick += gridDim.x, buf ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();   // this brick is there, and the other buffer's is used up
+        if (brick + (int)gridDim.x < bricks) load(brick + gridDim.x, buf ^ 1);
+        const unsigned sx = base + buf * kStage, sg = sx + kWgXv * XS;
+#pragma unroll 1
+        for (int s = 0; s < kWgD * kWgH; ++s) {
+            unsigned a[COUT / 16][4];
 #pragma unroll
-    for (int j = 0; j < PER; ++j) acc[j] = 0.f;
-    for (int vi = 0; vi < kWgVox; ++vi) {
+            for (int m = 0; m < COUT / 16; ++m) wg_ldsm(a[m], sg + (s * kWgW + ka) * GS + (m * 16 + ma) * 2);
+            const int row = ((s / kWgH + kd) * (kWgH + 2) + s % kWgH + kh) * (kWgW + 2);
 #pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const int el = threadIdx.x + 256 * j;
-            const int co = el / CIN, ci = el % CIN;
-            acc[j] += sx[vi * CIN + ci] * sg[vi * COUT + co];
+            for (int kw = 0; kw < 3; ++kw)
+#pragma unroll
+                for (int q = 0; q < CC / 16; ++q) {
+                    unsigned b[4];
+                    wg_ldsm(b, sx + (row + kw + kb) * XS + (q * 16 + nb8) * 2);
+#pragma unroll
+                    for (int m = 0; m < COUT / 16; ++m) {
+                        wg_mma(acc[kw][m][2 * q], a[m], b[0], b[1]);
+                        wg_mma(acc[kw][m][2 * q + 1], a[m], b[2], b[3]);
+                    }
+                }
+        }
+        if (blockIdx.y == 0 && strand < kStrands) {
+            const unsigned char* g = wg_smem + buf * kStage + kWgXv * XS + bco * 2;
+            for (int v = strand; v < kWgGv; v += kStrands)
+                bias += __bfloat162float(*reinterpret_cast<const bf16*>(g + v * GS));
         }
     }
+    if ((int)blockIdx.x >= bricks) return;
+    const int gq = lane >> 2, t = lane & 3;
 #pragma unroll
-    for (int j = 0; j < PER; ++j) {
-        const int el = threadIdx.x + 256 * j;
-        atomicAdd(&dW[(size_t)tap * COUT * CIN + el], acc[j]);
-    }
-    if (tap == 0 && threadIdx.x < COUT) {
-        float s = 0.f;
-        for (int vi = 0; vi < kWgVox; ++vi) s += sg[vi * COUT + threadIdx.x];
-        atomicAdd(&db[threadIdx.x], s);
-    }
+    for (int kw = 0; kw < 3; ++kw)
+#pragma unroll
+        for (int m = 0; m < COUT / 16; ++m)
+#pragma unroll
+            for (int q = 0; q < CC / 8; ++q)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int co = m * 16 + gq + (i >> 1) * 8, ci = c0 + q * 8 + 2 * t + (i & 1);
+                    atomicAdd(&dW[((size_t)(warp * 3 + kw) * COUT + co) * CIN + ci], acc[kw][m][q][i]);
+                }
+    if (blockIdx.y == 0 && strand < kStrands) atomicAdd(&db[bco], bias);
 }
 
 // 2x2x2 average pooling (NDHWC, C channels), dims of the input.
@@ -178,21 +251,29 @@ __global__ void k_relu_bwd(const float* __restrict__ g32, const bf16* __restrict
 // Weighted mean-squared loss over the first OC channels of out (C channels
 // per voxel): g[v][c] = 2 w (out - t) / (OC V) for c < OC, else 0; w times
 // the mean square added to *loss.
+// One thread per voxel: the FP64 squares of three channels in every lane,
+// where a thread per element left 13 of 16 lanes of the slow FP64 pipe idle
+// (42 -> 11 us at 262,144 voxels).  C a multiple of 4.
 __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t, float* __restrict__ g, long long V,
                       int C, int OC, float w, double* __restrict__ loss) {
     double s = 0.0;
     const float sc = 2.f * w / (float)(OC * V);
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < V * C; e += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(e % C);
-        const long long v = e / C;
-        float gv = 0.f;
-        if (c < OC) {
-            const float d = out[e] - t[v * OC + c];
-            s += (double)d * d;
-            gv = sc * d;
+    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x)
+        for (int c = 0; c < C; c += 4) {
+            float gv[4] = {0.f, 0.f, 0.f, 0.f};
+            if (c < OC) {
+                const float4 o4 = *reinterpret_cast<const float4*>(out + v * C + c);
+                const float o[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (c + i < OC) {
+                        const float d = o[i] - t[v * OC + c + i];
+                        s += (double)d * d;
+                        gv[i] = sc * d;
+                    }
+            }
+            *reinterpret_cast<float4*>(g + v * C + c) = make_float4(gv[0], gv[1], gv[2], gv[3]);
         }
-        g[e] = gv;
-    }
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0 && s != 0.0) atomicAdd(loss, (double)w * s / (double)(OC * V));
 }
