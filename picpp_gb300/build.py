@@ -3,7 +3,8 @@
     python -m picpp_gb300.build        (or picpp_gb300.build.build())
 
 Translation units compile in parallel with nvcc; the FP64 particle kernels
-use --fmad=false so that their arithmetic rounds like the CPU oracle.
+(but the per-tile ones) use --fmad=false so that their arithmetic rounds like
+the CPU oracle.
 """
 from __future__ import annotations
 
@@ -32,6 +33,7 @@ UNITS = {
     "grid.cu": [],
     "kernels_f32.cu": [],
     "kernels_f64.cu": ["--fmad=false"],
+    "kernels_f64_tile.cu": [],
     "energy_noalloc.cu": [],
     "init.cu": [],
     "nn.cu": [],

@@ -274,6 +274,10 @@ pic_status smooth_moments(pic_ctx* ctx) {
 }
 
 // -------------------------------------------------------------- explicit
+// CTAs per tile of the fused kernel: two CTAs per SM run at once with FP32
+// particles, one with FP64 ones.
+int explicit_parts(const TileGeom& t, int preal) { return tile_parts(t, preal ? kNumSM : 2 * kNumSM, preal != 0); }
+
 template <typename T>
 pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
     cudaStream_t s = ctx->s;
@@ -298,7 +302,7 @@ pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
                 S.defer[q] = ctx->sp[q].defer;
                 S.dwords[q] = ctx->sp[q].dwords;
             }
-            const int parts = tile_parts(ctx->tg);
+            const int parts = explicit_parts(ctx->tg, ctx->preal);
             {
                 Phase ph(ctx, PIC_PHASE_PUSH_DEPOSIT, 2);   // the fused kernel and its deferred pass
                 PK<T>::push_deposit_tiled(s, g, ctx->tg, ctx->ts, S, ctx->E, ctx->B, (double*)ctx->Jpart, ctx->Jfix,
@@ -600,7 +604,7 @@ pic_status pic_create(const pic_config* cfg, pic_ctx** out) {
         ok = ok && A(&ctx->B, ctx->rsz * 3 * N);
         ok = ok && A(&ctx->J, sizeof(double) * 3 * N);
         ok = ok && A(&ctx->Jfix, sizeof(double) * 3 * N);
-        ok = ok && A(&ctx->Jpart, sizeof(double) * 3 * (size_t)ts.jcells * ctx->ntiles * tile_parts(t));
+        ok = ok && A(&ctx->Jpart, sizeof(double) * 3 * (size_t)ts.jcells * ctx->ntiles * explicit_parts(t, ctx->preal));
     } else {
         ctx->pi_len = c.pressure_compat ? 9LL * ga.cex * ga.cey * ga.cez : 9 * N;
         ctx->jg_len = c.pressure_compat ? 3LL * ctx->nex * ctx->ney * ctx->nez : 3 * N;

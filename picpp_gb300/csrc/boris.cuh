@@ -139,9 +139,22 @@ __device__ __forceinline__ void velocity_t(const TP mom[3], TP m, TP v[3]) { vel
 template <>
 __device__ __forceinline__ void velocity_t<float>(const float mom[3], float m, float v[3]) { velocity_fast(mom, m, v); }
 // ... and of the fused tile kernel (FP32 with fixed roundings).
+// The FP64 form: the same with two reciprocal square roots where boris() has
+// three divisions and two square roots (about ten FP64 instructions each).
 template <typename TP>
 __device__ __forceinline__ void boris_tile(TP q, TP m, TP dt, TP beta, const TP e[3], const TP b[3], TP mom[3]) {
-    boris<TP>(q, m, dt, beta, e, b, mom);
+    const TP s = q * dt * TP(0.5);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) mom[d] = fma(e[d], s, mom[d]);
+    const TP p2 = mom[0] * mom[0] + mom[1] * mom[1] + mom[2] * mom[2];
+    const TP bs = (beta * m) * rsqrt(m * m + p2);
+    const TP b2 = b[0] * b[0] + b[1] * b[1] + b[2] * b[2];
+    const TP fb = (TP(2) * bs) * rsqrt(TP(1) + (bs * bs) * b2);
+    const TP tm[3] = {fma(mom[1] * b[2] - mom[2] * b[1], bs, mom[0]), fma(mom[2] * b[0] - mom[0] * b[2], bs, mom[1]),
+                      fma(mom[0] * b[1] - mom[1] * b[0], bs, mom[2])};
+    const TP txb[3] = {tm[1] * b[2] - tm[2] * b[1], tm[2] * b[0] - tm[0] * b[2], tm[0] * b[1] - tm[1] * b[0]};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) mom[d] += fma(txb[d], fb, e[d] * s);
 }
 template <>
 __device__ __forceinline__ void boris_tile<float>(float q, float m, float dt, float beta, const float e[3],
@@ -149,7 +162,10 @@ __device__ __forceinline__ void boris_tile<float>(float q, float m, float dt, fl
     boris_fixed(q, m, dt, beta, e, b, mom);
 }
 template <typename TP>
-__device__ __forceinline__ void velocity_tile(const TP mom[3], TP m, TP v[3]) { velocity<TP>(mom, m, v); }
+__device__ __forceinline__ void velocity_tile(const TP mom[3], TP m, TP v[3]) {
+    const TP r = rsqrt(m * m + mom[0] * mom[0] + mom[1] * mom[1] + mom[2] * mom[2]);
+    v[0] = mom[0] * r; v[1] = mom[1] * r; v[2] = mom[2] * r;
+}
 template <>
 __device__ __forceinline__ void velocity_tile<float>(const float mom[3], float m, float v[3]) { velocity_fixed(mom, m, v); }
 

@@ -48,6 +48,9 @@ constexpr int kTileThreads = PIC_TILE_THREADS;
 #ifndef PIC_TILE_MIN_BLOCKS
 #define PIC_TILE_MIN_BLOCKS 2   // CTAs per SM the register budget is sized for
 #endif
+// FP64: one CTA per SM (its blocks fill the shared memory), so 128 registers
+template <typename TP>
+__host__ __device__ constexpr int tile_ctas() { return sizeof(TP) == sizeof(float) ? PIC_TILE_MIN_BLOCKS : 1; }
 
 template <typename TP>
 __device__ __forceinline__ TP lerp(TP a, TP b, TP w) { return fmadd<TP>(w, subr<TP>(b, a), a); }
@@ -112,13 +115,6 @@ __device__ __forceinline__ void segment_add(TP Fx, TP Fy, TP Fz, TP Wx, TP Wy, T
 #pragma unroll
     for (int q = 0; q < 12; ++q) a[q] = fmadd<TP>(b[q], f[q], a[q]);
 }
-
-// Weight of the upper neighbour at the middle s / 2 of a segment, r cells from
-// the cell it is in: s / (2 d) - r, h = 1 / (2 d).
-template <typename TP>
-__device__ __forceinline__ TP weight_from(TP s, TP d2, TP h, TP r) { return divd<TP>(s, d2, h) - r; }
-template <>
-__device__ __forceinline__ float weight_from<float>(float s, float, float h, float r) { return __fmaf_rn(s, h, -r); }
 
 // Segmented sum of a[] over runs of lanes with equal key; returns true in the
 // first lane of each run, which then holds the run's totals.
@@ -280,7 +276,7 @@ __device__ __forceinline__ void stage_particle(ChunkBuf<TP>* buf, const PartView
 // kParts: several CTAs per tile (parts > 1); without it the loop keeps no
 // register for the stride (64 are all it has).
 template <typename TP, typename TF, int CT, bool kWall, bool kParts>
-__global__ void __launch_bounds__(kTileThreads, PIC_TILE_MIN_BLOCKS) k_push_deposit_tile(GridP g, TileGeom t, TileShape s, SpeciesSet<TP> S,
+__global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_tile(GridP g, TileGeom t, TileShape s, SpeciesSet<TP> S,
                                                                        const TF* __restrict__ E, const TF* __restrict__ B,
                                                                        double* __restrict__ Jpart, float fx_scale,
                                                                        double inv_dt, int nparts) {
@@ -437,12 +433,12 @@ __global__ void __launch_bounds__(kTileThreads, PIC_TILE_MIN_BLOCKS) k_push_depo
                         if constexpr (kWall) {
                             if (ni == kTristanWallNode && v[0] > TP(0) && PX < TP(0)) PX = -PX;
                         }
-                        const int rx = (int)dev_floor(divd<TP>(PX, dx, idx));
-                        const int ry = ey ? (int)dev_floor(divd<TP>(PY, dy, idy)) : 0;
-                        const int rz = ez ? (int)dev_floor(divd<TP>(PZ, dz, idz)) : 0;
-                        const TP RX = rx == 0 ? (X + PX) / TP(2) : TP(rx > 0 ? rx : 0) * dx;
-                        const TP RY = ry == 0 ? (Y + PY) / TP(2) : TP(ry > 0 ? ry : 0) * dy;
-                        const TP RZ = rz == 0 ? (Z + PZ) / TP(2) : TP(rz > 0 ? rz : 0) * dz;
+                        const int rx = (int)dev_floor((PX) * idx);
+                        const int ry = ey ? (int)dev_floor((PY) * idy) : 0;
+                        const int rz = ez ? (int)dev_floor((PZ) * idz) : 0;
+                        const TP RX = rx == 0 ? (X + PX) * TP(0.5) : TP(rx > 0 ? rx : 0) * dx;
+                        const TP RY = ry == 0 ? (Y + PY) * TP(0.5) : TP(ry > 0 ? ry : 0) * dy;
+                        const TP RZ = rz == 0 ? (Z + PZ) * TP(0.5) : TP(rz > 0 ? rz : 0) * dz;
                         const int ax = bx + rx, ay = by + ry, az = bz + rz;   // block cell of the old-side segment
                         // unsigned compares: (unsigned)x < n is 0 <= x < n
                         const bool inblock = nearx && (unsigned)(rx + 1) <= 2u && (unsigned)(ry + 1) <= 2u &&
@@ -451,18 +447,18 @@ __global__ void __launch_bounds__(kTileThreads, PIC_TILE_MIN_BLOCKS) k_push_depo
                                              (unsigned)by < (unsigned)(jy - ey) && (unsigned)az < (unsigned)(jz - ez) &&
                                              (unsigned)bz < (unsigned)(jz - ez);
                         if (inblock) {
-                            const TP F1x = divd<TP>(fcd * (RX - PX), dt, idt);
-                            const TP F1y = divd<TP>(fcd * (RY - PY), dt, idt);
-                            const TP F1z = divd<TP>(fcd * (RZ - PZ), dt, idt);
-                            const TP F2x = divd<TP>(fcd * (X - RX), dt, idt);
+                            const TP F1x = (fcd * (RX - PX)) * idt;
+                            const TP F1y = (fcd * (RY - PY)) * idt;
+                            const TP F1z = (fcd * (RZ - PZ)) * idt;
+                            const TP F2x = (fcd * (X - RX)) * idt;
                             const TP F2y = fmadd<TP>(fcd, v[1], -F1y), F2z = fmadd<TP>(fcd, v[2], -F1z);
                             const TP hxx = TP(0.5) * idx, hyy = TP(0.5) * idy, hzz = TP(0.5) * idz;
-                            const TP W1x = weight_from<TP>(PX + RX, TP(2) * dx, hxx, TP(rx));
-                            const TP W1y = ey ? weight_from<TP>(PY + RY, TP(2) * dy, hyy, TP(ry)) : TP(0);
-                            const TP W1z = ez ? weight_from<TP>(PZ + RZ, TP(2) * dz, hzz, TP(rz)) : TP(0);
-                            const TP W2x = divd<TP>(X + RX, TP(2) * dx, hxx);
-                            const TP W2y = ey ? divd<TP>(Y + RY, TP(2) * dy, hyy) : TP(0);
-                            const TP W2z = ez ? divd<TP>(Z + RZ, TP(2) * dz, hzz) : TP(0);
+                            const TP W1x = fmadd<TP>(PX + RX, hxx, -TP(rx));
+                            const TP W1y = ey ? fmadd<TP>(PY + RY, hyy, -TP(ry)) : TP(0);
+                            const TP W1z = ez ? fmadd<TP>(PZ + RZ, hzz, -TP(rz)) : TP(0);
+                            const TP W2x = (X + RX) * hxx;
+                            const TP W2y = ey ? (Y + RY) * hyy : TP(0);
+                            const TP W2z = ez ? (Z + RZ) * hzz : TP(0);
                             segment_slots<TP>(F2x, F2y, F2z, W2x, W2y, W2z, aB);
                             s1[0] = F1x; s1[1] = F1y; s1[2] = F1z; s1[3] = W1x; s1[4] = W1y; s1[5] = W1z;
                             keyA = (az * jy + ay) * jx + ax;

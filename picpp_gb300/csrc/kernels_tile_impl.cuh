@@ -1,0 +1,166 @@
+// kernels_tile_impl.cuh -- launchers of the per-tile particle kernels (fused
+// explicit step, tiled implicit deposit and mover) for one particle precision
+// T; instantiated by kernels_f32.cu and kernels_f64_tile.cu.
+#pragma once
+#include <algorithm>
+#include <cmath>
+#include "boris_tile.cuh"
+#include "implicit_tile.cuh"
+#include "kernels.hpp"
+
+namespace pic {
+
+template <typename T>
+size_t PK<T>::tile_smem_bytes(const TileShape& sh) {
+    size_t F = (size_t)sh.fx * sh.fy * sh.fz;
+    // FP32: the current block is 64-bit fixed point in two 32-bit words,
+    // followed by the warps' scratch for spreading the run heads' adds
+    const size_t fixed_scratch = sizeof(T) == 4 ? (size_t)(kTileThreads / 32) * kSpreadBytes : 0;
+    // and every warp's staged chunk of particles
+    return ((6 * F * sizeof(T) + 15) & ~size_t(15)) + ((3 * (size_t)sh.jcells * 8 + 15) & ~size_t(15)) + fixed_scratch +
+           (size_t)(kTileThreads / 32) * sizeof(ChunkBuf<T>);
+}
+
+template <typename T>
+void PK<T>::push_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileShape& sh,
+                               const SpeciesSet<T>& S, const void* E, const void* B, double* Jpart, double* Jfix,
+                               int parts, size_t smem) {
+    static bool attr_set = false;
+    if (!attr_set) {
+        for (auto* k : {k_push_deposit_tile<T, T, 8, false, false>, k_push_deposit_tile<T, T, 8, false, true>,
+                        k_push_deposit_tile<T, T, 0, false, false>, k_push_deposit_tile<T, T, 0, false, true>,
+                        k_push_deposit_tile<T, T, 0, true, false>, k_push_deposit_tile<T, T, 0, true, true>})
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        attr_set = true;
+    }
+    const bool cube8 = t.tx == 8 && t.ty == 8 && t.tz == 8 && g.y3 && g.z3 && sh.fx == 12 && sh.fy == 12 &&
+                       sh.fz == 12 && sh.jx == 12 && sh.jy == 12 && sh.jz == 12;
+    const float fx_scale = fixed_scale(g, S);
+    const double inv_dt = 1.0 / g.dt;
+    const int grid = std::min(t.ntx * t.nty * t.ntz * parts, kNumSM * 8);
+    // a wall box runs its own instantiation (run-time tile shape)
+    auto* whole = g.wall ? k_push_deposit_tile<T, T, 0, true, false>
+                         : cube8 ? k_push_deposit_tile<T, T, 8, false, false> : k_push_deposit_tile<T, T, 0, false, false>;
+    auto* shared = g.wall ? k_push_deposit_tile<T, T, 0, true, true>
+                          : cube8 ? k_push_deposit_tile<T, T, 8, false, true> : k_push_deposit_tile<T, T, 0, false, true>;
+    auto* kernel = parts > 1 ? shared : whole;
+    kernel<<<grid, kTileThreads, smem, s>>>(g, t, sh, S, (const T*)E, (const T*)B, Jpart, fx_scale, inv_dt, parts);
+    // the particles it left over: one thread per mask word
+    long long words = 1;
+    for (int q = 0; q < S.ns; ++q) words = std::max(words, (S.p[q].n + 31) / 32 + 1);
+    k_push_deposit_deferred<T, T><<<grid_for(words, 256), 256, 0, s>>>(g, S, (const T*)E, (const T*)B, Jfix);
+}
+
+// Fixed-point scale of the FP32 current block: the power of two with
+// max_species |q w / V| * scale <= 2^35 (every zigzag term is bounded by
+// q w / V because |v| < c = 1, so a run total of up to 32 terms stays below
+// 2^40; a tile entry takes at most two terms per particle of the tile, and
+// a cell's sum of at most 27 tile partials stays below 2^63 up to about five
+// million particles per tile).
+template <typename T>
+float PK<T>::fixed_scale(const GridP& g, const SpeciesSet<T>& S) {
+    double fmax = 0;
+    for (int q = 0; q < S.ns; ++q)
+        fmax = std::max(fmax, std::fabs((double)S.q[q] * (double)S.w[q] / (g.dx * g.dy * g.dz)));
+    return fmax > 0 ? (float)std::ldexp(1.0, 35 - (int)std::ceil(std::log2(fmax))) : 1.0f;
+}
+
+template <typename T>
+void PK<T>::assemble_j(cudaStream_t s, const GridP& g, const TileGeom& t, const TileShape& sh, const double* Jpart,
+                       const double* Jfix, double* J, double inv_scale, int parts) {
+    auto* kernel = parts > 1 ? k_assemble_j<T, true> : k_assemble_j<T, false>;
+    kernel<<<grid_for(g.N, 256), 256, 0, s>>>(g, t, sh, Jpart, Jfix, J, inv_scale, parts);
+}
+
+template <typename T>
+ImpBlock PK<T>::implicit_block(const GridP& g, const TileGeom& t, int h) {
+    ImpBlock b{};
+    b.h = h;
+    b.nbx = g.nx > 1 ? t.tx + 2 * h + 1 : 1;
+    b.nby = g.y3 ? t.ty + 2 * h + 1 : 1;
+    b.nbz = g.z3 ? t.tz + 2 * h + 1 : 1;
+    b.cbx = g.nx > 1 ? t.tx + 2 * h + 2 : 1;
+    b.cby = g.y3 ? t.ty + 2 * h + 2 : 1;
+    b.cbz = g.z3 ? t.tz + 2 * h + 2 : 1;
+    b.NB = b.nbx * b.nby * b.nbz;
+    b.CB = b.cbx * b.cby * b.cbz;
+    return b;
+}
+
+template <typename T>
+size_t PK<T>::implicit_tile_smem(const ImpBlock& bk) {
+    // FP32 accumulators add the per-warp rows of the tensor-core run sums
+    // and their 32-entry lane table
+    const size_t scratch = sizeof(T) == sizeof(float)
+                               ? (size_t)(imp_threads<T>() / 32) * kScrParticles * kScrRow * sizeof(float) + 32 * sizeof(TcLane)
+                               : 0;
+    return (12 * (size_t)bk.NB + 7 * (size_t)bk.CB + (bk.stage ? 3 * ((size_t)bk.NB + bk.CB) : 0)) * sizeof(T) + scratch;
+}
+
+template <typename T>
+void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileSplit& sp, const ImpBlock& bk,
+                                   const ImpSpecies<T>& S, const T* E, const T* B, double* J, double* mu,
+                                   double* rho, double* Pi) {
+    static bool attr_set = false;
+    if (!attr_set) {
+        for (auto* k : {k_implicit_deposit_tile<T, T, true, false>, k_implicit_deposit_tile<T, T, true, true>,
+                        k_implicit_deposit_tile<T, T, false, false>})
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        attr_set = true;
+    }
+    const size_t smem = implicit_tile_smem(bk);
+    const int per_sm = (int)((227 * 1024) / (smem + 1024));
+    const int ntiles = t.ntx * t.nty * t.ntz;
+    const int grid = ntiles < kNumSM * (per_sm > 0 ? per_sm : 1) ? ntiles : kNumSM * (per_sm > 0 ? per_sm : 1);
+    constexpr int nt = imp_threads<T>();
+    const bool split = sp.sx * sp.sy * sp.sz > 1;
+    auto* kernel = !bk.stage ? k_implicit_deposit_tile<T, T, false, false>
+                   : split ? k_implicit_deposit_tile<T, T, true, true> : k_implicit_deposit_tile<T, T, true, false>;
+    kernel<<<grid, nt, smem, s>>>(g, t, sp, bk, S, E, B, J, mu, rho, Pi);
+}
+
+template <typename T>
+bool PK<T>::implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const ImpSpecies<T>& S,
+                                const double* E, const double* B, const double* Et) {
+    MoverBlock mb{};
+    const int H = kMoverHalo;
+    mb.nbx = g.nx > 1 ? t.tx + 2 * H + 1 : 1;
+    mb.nby = g.y3 ? t.ty + 2 * H + 1 : 1;
+    mb.nbz = g.z3 ? t.tz + 2 * H + 1 : 1;
+    mb.cbx = g.nx > 1 ? t.tx + 2 * H + 2 : 1;
+    mb.cby = g.y3 ? t.ty + 2 * H + 2 : 1;
+    mb.cbz = g.z3 ? t.tz + 2 * H + 2 : 1;
+    mb.NB = mb.nbx * mb.nby * mb.nbz;
+    mb.CB = mb.cbx * mb.cby * mb.cbz;
+    // FP32: E^theta and B^n as float4 nodes / cells, E^n as three planes
+    const size_t fld = sizeof(T) == sizeof(float)
+                           ? ((size_t)mb.NB + (size_t)mb.CB) * 16 + 3 * (size_t)mb.NB * sizeof(float)
+                           : (6 * (size_t)mb.NB + 3 * (size_t)mb.CB) * sizeof(T);
+    // plus every thread's staged next particle (6 values and a cell)
+    const size_t smem = ((fld + 15) & ~size_t(15)) + (size_t)kMoverThreads * (6 * sizeof(T) + sizeof(int));
+    if (smem > 227 * 1024) return false;
+    static bool attr_set = false;
+    if (!attr_set) {
+        for (auto* k : {k_implicit_push_tile<T, false, false>, k_implicit_push_tile<T, false, true>,
+                        k_implicit_push_tile<T, true, false>, k_implicit_push_tile<T, true, true>})
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        attr_set = true;
+    }
+    const int per_sm = (int)((228 * 1024) / (smem + 1024));
+    const int cap = kNumSM * (per_sm > 0 ? per_sm : 1);
+    const int parts = tile_parts(t, 2 * kNumSM, false);
+    const int nwork = t.ntx * t.nty * t.ntz * parts;
+    // the wall rules are a separate instantiation: the periodic mover keeps
+    // none of their code in its loop
+    // the particles it left over: one thread per mask word
+    long long words = 1;
+    for (int q = 0; q < S.ns; ++q) words = std::max(words, (S.p[q].n + 31) / 32);
+    auto* kernel = g.wall ? (parts > 1 ? k_implicit_push_tile<T, true, true> : k_implicit_push_tile<T, true, false>)
+                          : (parts > 1 ? k_implicit_push_tile<T, false, true> : k_implicit_push_tile<T, false, false>);
+    kernel<<<nwork < cap ? nwork : cap, kMoverThreads, smem, s>>>(g, t, mb, S, E, B, Et, parts);
+    if (g.wall) k_implicit_push_deferred<T, true><<<grid_for(words, 128), 128, 0, s>>>(g, S, E, B, Et);
+    else k_implicit_push_deferred<T, false><<<grid_for(words, 128), 128, 0, s>>>(g, S, E, B, Et);
+    return true;
+}
+
+}  // namespace pic
