@@ -246,11 +246,8 @@ pic_status smooth_current(pic_ctx* ctx) {
     if (ctx->cfg.smoothing_count <= 0) return PIC_OK;
     pic_status st = ensure_smooth_tmp(ctx);
     if (st != PIC_OK) return st;
-    const size_t L = 3 * (size_t)ctx->g.N;
-    for (int q = 0; q < ctx->cfg.smoothing_count; ++q) {
+    for (int q = 0; q < ctx->cfg.smoothing_count; ++q)
         launch_smooth(ctx->s, ctx->g, ctx->J, ctx->smooth_tmp, 3, ctx->cfg.smoothing_parameter);
-        CK(cudaMemcpyAsync(ctx->J, ctx->smooth_tmp, sizeof(double) * L, cudaMemcpyDeviceToDevice, ctx->s));
-    }
     return PIC_OK;
 }
 
@@ -266,9 +263,7 @@ pic_status smooth_moments(pic_ctx* ctx) {
         launch_smooth_rho_ext(s, g, ctx->rho_ext, ctx->smooth_tmp, ctx->ex, ctx->ey, ctx->ez, sp);
         CK(cudaMemcpyAsync(ctx->rho_ext, ctx->smooth_tmp, sizeof(double) * ctx->rho_ext_len, cudaMemcpyDeviceToDevice, s));
         launch_smooth(s, g, ctx->Jh, ctx->smooth_tmp, 3, sp);
-        CK(cudaMemcpyAsync(ctx->Jh, ctx->smooth_tmp, sizeof(double) * 3 * g.N, cudaMemcpyDeviceToDevice, s));
         launch_smooth(s, g, ctx->mu, ctx->smooth_tmp, 9, sp);
-        CK(cudaMemcpyAsync(ctx->mu, ctx->smooth_tmp, sizeof(double) * 9 * g.N, cudaMemcpyDeviceToDevice, s));
     }
     return PIC_OK;
 }
@@ -331,7 +326,7 @@ pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
             for (auto& sp : ctx->sp) PK<T>::zigzag(s, g, view<T>(sp), sp.q, sp.m, sp.w, ctx->J);
         }
         {
-            Phase ph(ctx, PIC_PHASE_FIELDS, 2 * ctx->cfg.smoothing_count + 1);
+            Phase ph(ctx, PIC_PHASE_FIELDS, 2 * ctx->cfg.smoothing_count + 1);   // two passes a smoothing, the E step
             pic_status st = smooth_current(ctx);
             if (st != PIC_OK) return st;
             PK<T>::yee_e(s, g, ctx->E, ctx->B, ctx->J, ctx->e_right);

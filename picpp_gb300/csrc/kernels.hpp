@@ -139,7 +139,8 @@ void launch_maxwell_apply_t(cudaStream_t s, const GridP& g, const OpCoef& oc, co
                             double* out);
 void launch_field_update(cudaStream_t s, const GridP& g, const double* Et, const double* E, const double* B,
                          double* En, double* Bn, int doE, int doB);
-void launch_smooth(cudaStream_t s, const GridP& g, const double* src, double* dst, int ncomp, double sp);
+// a smoothed in place, tmp: scratch of the same size
+void launch_smooth(cudaStream_t s, const GridP& g, double* a, double* tmp, int ncomp, double sp);
 void launch_smooth_rho_ext(cudaStream_t s, const GridP& g, const double* src, double* dst, int ex, int ey, int ez,
                            double sp);
 void launch_density_finish(cudaStream_t s, long long N, double q, const double* conc, const double* energy,

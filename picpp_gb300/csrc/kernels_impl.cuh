@@ -48,22 +48,23 @@ __global__ void k_gather_payload(const int* __restrict__ perm, long long n, Part
 
 // Kinetic energy and momentum of one species: partials[q*P + block],
 // q = 0: sum w (gamma - 1) m, 1..3: sum w p (updateEnergy,
-// PIC++/simulation.cpp:1590-1600).
+// PIC++/simulation.cpp:1590-1600); the constant factors at the end, once.
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads) k_particle_sums(PartView<T> p, double m, double w, double* __restrict__ partials,
                                                                int P) {
     __shared__ double sh[32];
     double s[4] = {0, 0, 0, 0};
+    const double im2 = 1.0 / (m * m);
     for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < p.n; n += (long long)gridDim.x * blockDim.x) {
-        double px = p.px[n], py = p.py[n], pz = p.pz[n];
-        double p2 = px * px + py * py + pz * pz;
-        double gam = sqrt(p2 / (m * m) + 1.0);
-        s[0] += (gam - 1) * m * w;
-        s[1] += px * w; s[2] += py * w; s[3] += pz * w;
+        const double px = p.px[n], py = p.py[n], pz = p.pz[n];
+        const double u2 = fma(px, px, fma(py, py, pz * pz)) * im2;
+        s[0] += sqrt(u2 + 1.0) - 1.0;
+        s[1] += px; s[2] += py; s[3] += pz;
     }
+    const double f[4] = {m * w, w, w, w};
     for (int q = 0; q < 4; ++q) {
         double r = block_sum(s[q], sh);
-        if (threadIdx.x == 0) partials[q * P + blockIdx.x] = r;
+        if (threadIdx.x == 0) partials[q * P + blockIdx.x] = r * f[q];
     }
 }
 
