@@ -94,20 +94,47 @@ __device__ __forceinline__ T tri_block(const T* __restrict__ F, int base, int sx
                  wy * (ux * F[base + sz + sy] + wx * F[base + sz + sy + sx]));
 }
 
-// The same trilinear form on a block of float4 nodes or cells (x, y, z, unused):
-// one 16-byte load per corner for all three components, each component
-// evaluated in exactly tri_block's order.
-__device__ __forceinline__ void tri_block4(const float4* __restrict__ F, int base, int sx, int sy, int sz, float wx,
-                                           float wy, float wz, float out[3]) {
-    const float ux = 1.f - wx, uy = 1.f - wy, uz = 1.f - wz;
-    const float4 f000 = F[base], f100 = F[base + sx], f010 = F[base + sy], f110 = F[base + sy + sx];
-    const float4 f001 = F[base + sz], f101 = F[base + sz + sx], f011 = F[base + sz + sy], f111 = F[base + sz + sy + sx];
-    out[0] = uz * (uy * (ux * f000.x + wx * f100.x) + wy * (ux * f010.x + wx * f110.x)) +
-             wz * (uy * (ux * f001.x + wx * f101.x) + wy * (ux * f011.x + wx * f111.x));
-    out[1] = uz * (uy * (ux * f000.y + wx * f100.y) + wy * (ux * f010.y + wx * f110.y)) +
-             wz * (uy * (ux * f001.y + wx * f101.y) + wy * (ux * f011.y + wx * f111.y));
-    out[2] = uz * (uy * (ux * f000.z + wx * f100.z) + wy * (ux * f010.z + wx * f110.z)) +
-             wz * (uy * (ux * f001.z + wx * f101.z) + wy * (ux * f011.z + wx * f111.z));
+// Weights of the eight corners (x fastest) from the upper weight of each axis.
+template <typename T>
+__device__ __forceinline__ void corners(T wx, T wy, T wz, T w[8]) {
+    const T ux = T(1) - wx, uy = T(1) - wy, uz = T(1) - wz;
+    const T yz[4] = {uy * uz, wy * uz, uy * wz, wy * wz};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) { w[2 * q] = ux * yz[q]; w[2 * q + 1] = wx * yz[q]; }
+}
+// Three components gathered with corner weights that they share (12 products
+// and 24 multiply-adds; the nested form above has 14 operations and the lower
+// weights per component): from three planes of a staged block, `plane`
+// entries apart, or from a block of float4 nodes or cells (x, y, z, unused),
+// one 16-byte load per corner.
+template <typename T>
+__device__ __forceinline__ void gather3(const T* __restrict__ F, int plane, int base, int sx, int sy, int sz,
+                                        const T w[8], T out[3]) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const T* f = F + q * plane + base;
+        T v = w[0] * f[0];
+        v = fma(w[1], f[sx], v);
+        v = fma(w[2], f[sy], v);
+        v = fma(w[3], f[sy + sx], v);
+        v = fma(w[4], f[sz], v);
+        v = fma(w[5], f[sz + sx], v);
+        v = fma(w[6], f[sz + sy], v);
+        out[q] = fma(w[7], f[sz + sy + sx], v);
+    }
+}
+__device__ __forceinline__ void gather3(const float4* __restrict__ F, int base, int sx, int sy, int sz, const float w[8],
+                                        float out[3]) {
+    const float4* f = F + base;
+    const int at[8] = {0, sx, sy, sy + sx, sz, sz + sx, sz + sy, sz + sy + sx};
+    out[0] = out[1] = out[2] = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const float4 v = f[at[q]];
+        out[0] = fmaf(w[q], v.x, out[0]);
+        out[1] = fmaf(w[q], v.y, out[1]);
+        out[2] = fmaf(w[q], v.z, out[2]);
+    }
 }
 
 // ---- tensor-core reduction of one run (FP32 accumulators) -------------------
@@ -617,6 +644,14 @@ struct MoverBlock {
     int cbx, cby, cbz, CB;
 };
 
+// The tiled mover's constants in the particle precision.
+template <typename T>
+struct MoverSet {
+    T dt, eta, edt, redt, dx2;   // dx2: dx squared (Picard test)
+    T id[3];
+    T beta[kMaxSpecies], qdt[kMaxSpecies], m[kMaxSpecies];
+};
+
 // moveParticle (PIC++/mover.cpp:194-491), one CTA per tile of tile-ordered
 // particles: E^n and E^{n+theta} (nodes) and B^n (cells) of the tile and a
 // two-cell halo are staged in shared memory in the particle precision, so
@@ -629,6 +664,7 @@ struct MoverBlock {
 // register for the stride.
 template <typename T, bool kWall, bool kParts>
 __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g, TileGeom t, MoverBlock mb, ImpSpecies<T> S,
+                                                            const __grid_constant__ MoverSet<T> K,
                                                             const double* __restrict__ E, const double* __restrict__ B,
                                                             const double* __restrict__ Et, int nparts) {
     extern __shared__ __align__(16) unsigned char mv_smem[];
@@ -664,11 +700,12 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
     const int hx = ax ? kMoverHalo : 0, hy = ay ? kMoverHalo : 0, hz = az ? kMoverHalo : 0;
     const int nsx = ax ? 1 : 0, nsy = ay ? mb.nbx : 0, nsz = az ? mb.nbx * mb.nby : 0;
     const int csx = ax ? 1 : 0, csy = ay ? mb.cbx : 0, csz = az ? mb.cbx * mb.cby : 0;
-    const T dt = T(g.dt), eta = T(g.eta), edt = T(g.eta * g.dt);
-    const T id[3] = {T(g.idx), T(g.idy), T(g.idz)};
+    // (in the particle precision already: conversions from the FP64 grid
+    // parameters run on the FP64 pipe, and the compiler repeats them in the
+    // loop rather than hold their results)
+    const T dt = K.dt, eta = K.eta, edt = K.edt, redt = K.redt;
+    const T id[3] = {K.id[0], K.id[1], K.id[2]};
     const int nn[3] = {g.nx, g.ny, g.nz};
-    const T dxT = T(g.dx);
-    const T redt = T((1.0 - g.eta) * g.dt);
     const int parts = kParts ? nparts : 1;
     // `parts` CTAs share a tile: each takes every parts-th run of blockDim particles
     for (int work = blockIdx.x; work < ntiles * parts; work += gridDim.x) {
@@ -702,10 +739,7 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
         __syncthreads();
         for (int s = 0; s < S.ns; ++s) {
             const PartView<T> p = S.p[s];
-            const double qs = S.q[s], ms = S.m[s];
-            const T beta = T(0.5 * qs * g.dt / ms);
-            const T qdt = T(qs * g.dt);
-            const T mm = T(ms);
+            const T beta = K.beta[s], qdt = K.qdt[s], mm = K.m[s];
             const int b0 = S.off[s][tile * T3] + part * blockDim.x, b1 = S.off[s][(tile + 1) * T3];
             const int step = kParts ? parts * blockDim.x : blockDim.x;
             if (b0 + (int)threadIdx.x < b1) stage(p, b0 + threadIdx.x);
@@ -737,14 +771,13 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
                     int lo[3];
 #pragma unroll
                     for (int a = 0; a < 3; ++a) {
-                        T w2[2];
-                        int idx[2];
-                        node_w<T>(u[a], l[a], nn[a], idx, w2);
-                        L.wn[a] = w2[1];
-                        cell_w<T>(u[a], l[a], nn[a], idx, w2);
-                        L.wc[a] = w2[1];
-                        // lower cell of the pair: c - 1 below the centre, c above
-                        lo[a] = (nn[a] > 1 && u[a] < T(0.5)) ? l[a] - 1 : l[a];
+                        // upper weights: u of the nodes (c, c + 1); of the cell
+                        // pair (c - 1, c) below the centre u + 1/2, (c, c + 1)
+                        // above it u - 1/2
+                        const bool act = nn[a] > 1, below = act && u[a] < T(0.5);
+                        L.wn[a] = act ? u[a] : T(0);
+                        L.wc[a] = act ? u[a] + (below ? T(0.5) : T(-0.5)) : T(0);
+                        lo[a] = below ? l[a] - 1 : l[a];
                     }
                     L.nbase = (l[2] + hz) * nsz + (l[1] + hy) * nsy + (l[0] + hx) * nsx;
                     const int ex = ax ? 1 : 0, ey = ay ? 1 : 0, ez = az ? 1 : 0;
@@ -759,33 +792,24 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
                     }
                     locate_l(l, u, L);
                 };
-                // gathers at a located position inside the block
-                auto gat = [&](const Loc& L, const T* __restrict__ blkN, bool node, T out[3]) {
-                    if (node) {
-#pragma unroll
-                        for (int q = 0; q < 3; ++q)
-                            out[q] = tri_block<T>(blkN + q * mb.NB, L.nbase, nsx, nsy, nsz, L.wn[0], L.wn[1], L.wn[2]);
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 3; ++q)
-                            out[q] = tri_block<T>(blkN + q * mb.CB, L.cbase, csx, csy, csz, L.wc[0], L.wc[1], L.wc[2]);
-                    }
-                };
-                // E^theta (node) and B^n (cell): float4 blocks for FP32
-                auto gatEt = [&](const Loc& L, T out[3]) {
-                    if constexpr (kVec) tri_block4(sEt4, L.nbase, nsx, nsy, nsz, L.wn[0], L.wn[1], L.wn[2], out);
-                    else gat(L, sEt, true, out);
+                // gathers at a located position inside the block: E^theta
+                // (nodes, corner weights w) and B^n (cells), float4 blocks for FP32
+                auto gatEt = [&](const Loc& L, const T w[8], T out[3]) {
+                    if constexpr (kVec) gather3(sEt4, L.nbase, nsx, nsy, nsz, w, out);
+                    else gather3<T>(sEt, mb.NB, L.nbase, nsx, nsy, nsz, w, out);
                 };
                 auto gatB = [&](const Loc& L, T out[3]) {
-                    if constexpr (kVec) tri_block4(sB4, L.cbase, csx, csy, csz, L.wc[0], L.wc[1], L.wc[2], out);
-                    else gat(L, sB, false, out);
+                    T w[8];
+                    corners<T>(L.wc[0], L.wc[1], L.wc[2], w);
+                    if constexpr (kVec) gather3(sB4, L.cbase, csx, csy, csz, w, out);
+                    else gather3<T>(sB, mb.CB, L.cbase, csx, csy, csz, w, out);
                 };
                 auto defer = [&]() { atomicOr(&S.defer[s][n >> 5], 1u << (n & 31)); };
                 T u0[3] = {pu[0], pu[1], pu[2]};
                 T mom0[3] = {pm[0], pm[1], pm[2]};
                 T gam, v[3];
                 gamma_vel<T>(mom0, mm, gam, v);
-                T e[3], b[3], al[9];
+                T e[3], e0[3], b[3], al[9];
                 Loc L0;
                 int l0[3];
                 locate(ci, u0, L0, l0);
@@ -793,10 +817,14 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
                     defer();
                     continue;
                 }
-                gat(L0, sE, true, e);
+                {
+                    T w[8];
+                    corners<T>(L0.wn[0], L0.wn[1], L0.wn[2], w);
+                    gather3<T>(sE, mb.NB, L0.nbase, nsx, nsy, nsz, w, e0);
+                    gatEt(L0, w, e);
+                }
                 gatB(L0, b);
-                alpha_tensor<T>(beta, v, gam, e, b, al);
-                gatEt(L0, e);
+                alpha_tensor<T>(beta, v, gam, e0, b, al);
                 T vxb[3] = {v[1] * b[2] - v[2] * b[1], -v[0] * b[2] + v[2] * b[0], v[0] * b[1] - v[1] * b[0]};
                 T pnew[3];
 #pragma unroll
@@ -822,7 +850,7 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
                 const T momNorm = (mom0[0] * mom0[0] + mom0[1] * mom0[1] + mom0[2] * mom0[2]);
                 T err = ((mom0[0] - pnew[0]) * (mom0[0] - pnew[0]) + (mom0[1] - pnew[1]) * (mom0[1] - pnew[1]) +
                                  (mom0[2] - pnew[2]) * (mom0[2] - pnew[2]));
-                const T dxN = dxT * dxT;
+                const T dxN = K.dx2;
                 T cerr = dxN;
                 T newDisp[3] = {mv[0] * edt, mv[1] * edt, mv[2] * edt};
                 T prevDisp[3];
@@ -867,7 +895,11 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
                         left = true;
                         break;
                     }
-                    gatEt(L1, e);
+                    {
+                        T w[8];
+                        corners<T>(L1.wn[0], L1.wn[1], L1.wn[2], w);
+                        gatEt(L1, w, e);
+                    }
                     gatB(L1, b);
                     const T mvxb[3] = {mv[1] * b[2] - mv[2] * b[1], -mv[0] * b[2] + mv[2] * b[0], mv[0] * b[1] - mv[1] * b[0]};
 #pragma unroll

@@ -157,7 +157,16 @@ bool PK<T>::implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& 
     for (int q = 0; q < S.ns; ++q) words = std::max(words, (S.p[q].n + 31) / 32);
     auto* kernel = g.wall ? (parts > 1 ? k_implicit_push_tile<T, true, true> : k_implicit_push_tile<T, true, false>)
                           : (parts > 1 ? k_implicit_push_tile<T, false, true> : k_implicit_push_tile<T, false, false>);
-    kernel<<<nwork < cap ? nwork : cap, kMoverThreads, smem, s>>>(g, t, mb, S, E, B, Et, parts);
+    MoverSet<T> K{};
+    K.dt = T(g.dt); K.eta = T(g.eta); K.edt = T(g.eta * g.dt); K.redt = T((1.0 - g.eta) * g.dt);
+    K.dx2 = T(g.dx) * T(g.dx);
+    K.id[0] = T(g.idx); K.id[1] = T(g.idy); K.id[2] = T(g.idz);
+    for (int q = 0; q < S.ns; ++q) {
+        K.beta[q] = T(0.5 * S.q[q] * g.dt / S.m[q]);
+        K.qdt[q] = T(S.q[q] * g.dt);
+        K.m[q] = T(S.m[q]);
+    }
+    kernel<<<nwork < cap ? nwork : cap, kMoverThreads, smem, s>>>(g, t, mb, S, K, E, B, Et, parts);
     if (g.wall) k_implicit_push_deferred<T, true><<<grid_for(words, 128), 128, 0, s>>>(g, S, E, B, Et);
     else k_implicit_push_deferred<T, false><<<grid_for(words, 128), 128, 0, s>>>(g, S, E, B, Et);
     return true;
