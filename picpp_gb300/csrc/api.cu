@@ -341,17 +341,23 @@ pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
 // -------------------------------------------------------------- implicit
 // Sub-tiles of the staged deposit: tiles are cut (z first, then y, then x, by
 // the smallest prime factor, so that a sub-tile's keys stay consecutive)
-// until there is one sub-tile per SM.  Returns the sub-tiles' geometry.  More
-// cuts do not help: the pairs plane of 32x32x1 (16 tiles, FP64) deposits in
-// 1.73 ms per step uncut, 0.34 ms cut to 256 sub-tiles, 0.5 ms at 1024 (each
+// until there is one sub-tile per SM and two fit into an SM's shared memory.
+// More cuts do not help: the pairs plane of 32x32x1 (16 tiles, FP64) deposited
+// in 1.73 ms per step uncut, 0.34 ms cut to 256 sub-tiles, 0.5 ms at 1024 (each
 // sub-tile flushes a block of its own).
-TileGeom split_tiles(const TileGeom& t, TileSplit& sp) {
+template <typename T>
+TileGeom split_tiles(const GridP& g, const TileGeom& t, TileSplit& sp) {
     TileGeom w = t;
     int* ext[3] = {&w.tz, &w.ty, &w.tx};
     int* cnt[3] = {&w.ntz, &w.nty, &w.ntx};
     int* cut[3] = {&sp.sz, &sp.sy, &sp.sx};
+    auto fits = [&]() {
+        ImpBlock bk = PK<T>::implicit_block(g, w, 0);
+        bk.stage = 1;
+        return PK<T>::implicit_tile_smem(bk, w.tx * w.ty * w.tz) <= (size_t)(227 * 1024) / 2 - 1024;
+    };
     for (int a = 0; a < 3; ++a)
-        while (*ext[a] > 1 && w.ntx * w.nty * w.ntz < kNumSM) {
+        while (*ext[a] > 1 && (w.ntx * w.nty * w.ntz < kNumSM || !fits())) {
             int f = 2;
             while (*ext[a] % f) ++f;
             *ext[a] /= f;
@@ -377,18 +383,18 @@ pic_status implicit_moments(pic_ctx* ctx) {
     // the block fits in shared memory
     // right after a sort every particle is in its tile: no halo, and E, B
     // staged next to the accumulators; otherwise a one-cell halo for drift
-    // (staged: over sub-tiles when the box has few tiles)
+    // (staged: over sub-tiles, split_tiles)
     TileSplit sp{1, 1, 1};
-    TileGeom wt = split_tiles(ctx->tg, sp);
+    TileGeom wt = split_tiles<T>(g, ctx->tg, sp);
     ImpBlock bk = PK<T>::implicit_block(g, wt, 0);
     bk.stage = 1;
-    if (!ctx->fresh_sort || PK<T>::implicit_tile_smem(bk) > 227 * 1024) {
+    if (!ctx->fresh_sort || PK<T>::implicit_tile_smem(bk, wt.tx * wt.ty * wt.tz) > 227 * 1024) {
         wt = ctx->tg;
         sp = TileSplit{1, 1, 1};
         bk = PK<T>::implicit_block(g, ctx->tg, 1);
-        if (PK<T>::implicit_tile_smem(bk) > 227 * 1024) bk = PK<T>::implicit_block(g, ctx->tg, 0);
+        if (PK<T>::implicit_tile_smem(bk, ctx->T3) > 227 * 1024) bk = PK<T>::implicit_block(g, ctx->tg, 0);
     }
-    if (!compat && all_sorted(ctx) && PK<T>::implicit_tile_smem(bk) <= 227 * 1024) {
+    if (!compat && all_sorted(ctx) && PK<T>::implicit_tile_smem(bk, wt.tx * wt.ty * wt.tz) <= 227 * 1024) {
         ImpSpecies<T> S{};
         S.ns = (int)ctx->sp.size();
         for (int q = 0; q < S.ns; ++q) {

@@ -249,25 +249,6 @@ __device__ __forceinline__ void add_runs_fx(unsigned* __restrict__ lo, int* __re
     __syncwarp();
 }
 
-// A warp's staged chunk of particles: cell, then ox oy oz px py pz, 32 each.
-template <typename TP>
-struct ChunkBuf {
-    TP a[6][32];
-    int cell[32];
-};
-
-// Starts the copy of particle n (this lane's slot) into the warp's buffer.
-template <typename TP>
-__device__ __forceinline__ void stage_particle(ChunkBuf<TP>* buf, const PartView<TP>& P, long long n, int lane) {
-    cp_async<4>(&buf->cell[lane], P.cell + n);
-    cp_async<sizeof(TP)>(&buf->a[0][lane], P.ox + n);
-    cp_async<sizeof(TP)>(&buf->a[1][lane], P.oy + n);
-    cp_async<sizeof(TP)>(&buf->a[2][lane], P.oz + n);
-    cp_async<sizeof(TP)>(&buf->a[3][lane], P.px + n);
-    cp_async<sizeof(TP)>(&buf->a[4][lane], P.py + n);
-    cp_async<sizeof(TP)>(&buf->a[5][lane], P.pz + n);
-}
-
 // CT: compile-time tile extent of a cubic 3-D tile (8), or 0 for shapes read
 // from TileShape at run time.  kWall: conductor-wall box (GridP::wall), the
 // Tristan mover's reflection and escape and the zigzag wall term

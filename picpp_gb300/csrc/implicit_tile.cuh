@@ -61,15 +61,17 @@ __device__ __forceinline__ A xpose_sum(A v[32], int lane) {
     return v[0];
 }
 
-// Node / cell weights of one axis (node_w and cell_w of common.cuh, in the
-// three-slot form c-1, c, c+1 for cells).
+// Node weights (c, c + 1) and cell weights (c - 1, c, c + 1) of one axis
+// (node_w and cell_w of common.cuh without branches).
 template <typename T>
 __device__ __forceinline__ void axis_weights(T u, bool act, T wn[2], T wc[3]) {
     if (!act) { wn[0] = T(1); wn[1] = T(0); wc[0] = T(0); wc[1] = T(1); wc[2] = T(0); return; }
-    if (u < T(0.5)) { wn[0] = T(0.5) + (T(0.5) - u); wn[1] = T(1) - wn[0]; }
-    else            { wn[1] = T(0.5) + (u - T(0.5)); wn[0] = T(1) - wn[1]; }
-    if (u < T(0.5)) { wc[1] = T(0.5) + u; wc[0] = T(1) - wc[1]; wc[2] = T(0); }
-    else            { wc[1] = T(0.5) + (T(1) - u); wc[2] = T(1) - wc[1]; wc[0] = T(0); }
+    wn[0] = T(1) - u;
+    wn[1] = u;
+    const T d = u - T(0.5);
+    wc[0] = d < T(0) ? -d : T(0);
+    wc[1] = T(1) - (d < T(0) ? -d : d);
+    wc[2] = d < T(0) ? T(0) : d;
 }
 
 // Local index of global cell index c on an axis of n cells relative to a
@@ -83,17 +85,6 @@ __device__ __forceinline__ bool local_axis(int c, int x0, int t, int h, int n, i
     return false;
 }
 
-// Trilinear gather from a staged block: base = block index of the lower
-// corner, (sx, sy, sz) strides (0 on a single-cell axis), weights of the
-// upper corners.
-template <typename T>
-__device__ __forceinline__ T tri_block(const T* __restrict__ F, int base, int sx, int sy, int sz, T wx, T wy, T wz) {
-    const T ux = T(1) - wx, uy = T(1) - wy, uz = T(1) - wz;
-    return uz * (uy * (ux * F[base] + wx * F[base + sx]) + wy * (ux * F[base + sy] + wx * F[base + sy + sx])) +
-           wz * (uy * (ux * F[base + sz] + wx * F[base + sz + sx]) +
-                 wy * (ux * F[base + sz + sy] + wx * F[base + sz + sy + sx]));
-}
-
 // Weights of the eight corners (x fastest) from the upper weight of each axis.
 template <typename T>
 __device__ __forceinline__ void corners(T wx, T wy, T wz, T w[8]) {
@@ -103,8 +94,7 @@ __device__ __forceinline__ void corners(T wx, T wy, T wz, T w[8]) {
     for (int q = 0; q < 4; ++q) { w[2 * q] = ux * yz[q]; w[2 * q + 1] = wx * yz[q]; }
 }
 // Three components gathered with corner weights that they share (12 products
-// and 24 multiply-adds; the nested form above has 14 operations and the lower
-// weights per component): from three planes of a staged block, `plane`
+// and 24 multiply-adds; nested interpolations are 14 operations per component): from three planes of a staged block, `plane`
 // entries apart, or from a block of float4 nodes or cells (x, y, z, unused),
 // one 16-byte load per corner.
 template <typename T>
@@ -380,14 +370,84 @@ __device__ __noinline__ EB6<T> gather_eb_global(const GridP g, int i, int j, int
     return r;
 }
 
+// The run sums of the lanes `me` (one stencil base) with FP64 accumulators: a
+// butterfly per 32 products, one shared atomic per lane and pass.
+template <typename A, typename T>
+__device__ __forceinline__ void butterfly_sums(const T row[kScrRow], bool me, double cq, double cm, A* __restrict__ sN,
+                                               A* __restrict__ sC, int NB, int CB, int nb, int cb, int oxn, int oyn,
+                                               int ozn, int oxc, int oyc, int ozc, int lane) {
+    A QN[12], QC[7], wn[8], wc[27];
+    run_quantities<A, T>(row, cq, cm, QN, QC);
+    run_weights<A, T>(row, wn, wc);
+    A vv[32];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+#pragma unroll
+        for (int x = 0; x < 32; ++x) vv[x] = me ? QN[4 * r + x / 8] * wn[x % 8] : A(0);
+        const A sum = xpose_sum<A>(vv, lane);
+        const int q = 4 * r + lane / 8, c = lane % 8;
+        if (sum != A(0))
+            atomicAdd(&sN[q * NB + nb + (c & 1) * oxn + ((c >> 1) & 1) * oyn + (c >> 2) * ozn],
+                      sum);
+    }
+#pragma unroll
+    for (int r = 0; r < 6; ++r) {
+#pragma unroll
+        for (int x = 0; x < 32; ++x) {
+            const int idx = 32 * r + x;
+            vv[x] = (idx < 189 && me) ? QC[idx / 27] * wc[idx % 27] : A(0);
+        }
+        const A sum = xpose_sum<A>(vv, lane);
+        const int idx = 32 * r + lane;
+        if (idx < 189 && sum != A(0)) {
+            const int q = idx / 27, sl = idx % 27;
+            atomicAdd(&sC[q * CB + cb + (sl % 3) * oxc + ((sl / 3) % 3) * oyc + (sl / 9) * ozc],
+                      sum);
+        }
+    }
+}
+
+// A particle outside the block (rare): its raw row into the FP64 grids.
+template <typename A, typename T>
+__device__ __forceinline__ void deposit_row_global(const GridP& g, int cell, T ox, T oy, T oz, const T row[kScrRow],
+                                                   double cq, double cm, double* __restrict__ J, double* __restrict__ mu,
+                                                   double* __restrict__ rho, double* __restrict__ Pi) {
+    int i, j, k;
+    decode(g, cell, i, j, k);
+    A QN[12], QC[7];
+    run_quantities<A, T>(row, cq, cm, QN, QC);
+    double qn[12], qc[7];
+#pragma unroll
+    for (int d = 0; d < 12; ++d) qn[d] = double(QN[d]);
+#pragma unroll
+    for (int d = 0; d < 7; ++d) qc[d] = double(QC[d]);
+    imp_deposit_global<T>(g, i, j, k, ox, oy, oz, qn, qc, J, mu, rho, Pi);
+}
+
+// The tiled deposit's constants per species: beta and m in the particle
+// precision, the factors of J-hat, rho-hat, Pi (q w / V) and of mu.
+template <typename T>
+struct DepositSet {
+    T beta[kMaxSpecies], m[kMaxSpecies];
+    double cq[kMaxSpecies], cm[kMaxSpecies];
+};
+
 // E and B come in the particle precision (FP32 copies for the FP32 path:
-// no FP64 conversion per gather).  kStaged: E and B staged in shared memory
-// next to the accumulators (right after a sort, h = 0); a separate
-// instantiation keeps the hot loop's code small.
+// no FP64 conversion per gather).
+// kStaged (right after a sort, h = 0): a particle of key k lies in cell k, so a
+// chunk of 32 particles of one key has one stencil base; E and B are staged in
+// shared memory next to the accumulators (FP32: float4 nodes and cells, one
+// 16-byte load per corner), the keys' offsets too, and each warp copies its
+// next chunk of particles with cp.async while it works on the current one.
+// What bounds it is instruction issue at 16 warps per SM (two CTAs: the run
+// sums' accumulators take 128 registers); tiles are cut so that two fit
+// (split_tiles, api.cu).
 // kSplit: t is the geometry of sub-tiles, cut from the sort's tiles by sp.
 template <typename T, typename A, bool kStaged, bool kSplit>
 __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(GridP g, TileGeom t, TileSplit sp, ImpBlock bk,
-                                                                       ImpSpecies<T> S, const T* __restrict__ E,
+                                                                       ImpSpecies<T> S,
+                                                                       const __grid_constant__ DepositSet<T> K,
+                                                                       const T* __restrict__ E,
                                                                        const T* __restrict__ B,
                                                                        double* __restrict__ J, double* __restrict__ mu,
                                                                        double* __restrict__ rho,
@@ -395,13 +455,15 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
     extern __shared__ __align__(16) unsigned char imp_smem[];
     A* sN = reinterpret_cast<A*>(imp_smem);   // [12][NB]
     A* sC = sN + 12 * bk.NB;                  // [7][CB]
-    T* sE = reinterpret_cast<T*>(sC + 7 * bk.CB);   // [3][NB] when staged
-    T* sB = sE + 3 * bk.NB;                          // [3][CB] when staged
+    // staged E and B: three planes each, FP32 one float4 per node / cell
+    constexpr bool kVec = sizeof(T) == sizeof(float);
+    T* sE = reinterpret_cast<T*>(imp_smem + bk.stage_at());
+    T* sB = sE + 3 * bk.NB;
+    float4* sE4 = reinterpret_cast<float4*>(sE);
+    float4* sB4 = sE4 + bk.NB;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int T3 = t.tx * t.ty * t.tz;
     const int ntiles = t.ntx * t.nty * t.ntz;
-    const double PI_D = 3.14159265358979323846;
-    const double ivol = 1.0 / (g.dx * g.dy * g.dz);
     const bool ax = g.nx > 1, ay = g.y3, az = g.z3;
     const int hx = ax ? bk.h : 0, hy = ay ? bk.h : 0, hz = az ? bk.h : 0;
     const int nsy = bk.nbx, nsz = bk.nbx * bk.nby;
@@ -410,11 +472,14 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
     const int oxc = ax ? 1 : 0, oyc = ay ? csy : 0, ozc = az ? csz : 0;   // slot strides
     const int tot = 12 * bk.NB + 7 * bk.CB;
     constexpr bool kTc = sizeof(A) == sizeof(float);   // FP32 accumulators: tensor-core run sums
-    float* scr0 = reinterpret_cast<float*>(imp_smem + (size_t)tot * sizeof(A) +
-                                           (kStaged ? (size_t)3 * (bk.NB + bk.CB) * sizeof(T) : 0));
+    unsigned char* after = imp_smem + bk.scratch_at();
+    float* scr0 = reinterpret_cast<float*>(after);
     float* scr = scr0 + warp * (kScrParticles * kScrRow);
     // the lane table of tc_run_sums follows the scratch rows of all warps
     TcLane* s_lane = reinterpret_cast<TcLane*>(scr0 + nwarps * (kScrParticles * kScrRow));
+    // staged: every warp's next chunk, then the keys' offsets of all species
+    ChunkBuf<T>* buf = reinterpret_cast<ChunkBuf<T>*>(kTc ? reinterpret_cast<unsigned char*>(s_lane + 32) : after) + warp;
+    int* sOff = reinterpret_cast<int*>(buf - warp + nwarps);
     if (kTc && threadIdx.x < 32) s_lane[threadIdx.x] = tc_lane(threadIdx.x);
 
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -430,39 +495,132 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
             for (int e = threadIdx.x; e < bk.NB; e += blockDim.x) {
                 const int lx = e % bk.nbx, ly = (e / bk.nbx) % bk.nby, lz = e / (bk.nbx * bk.nby);
                 const long long id = linw(g, x0 + lx, y0 + ly, z0 + lz);
+                if constexpr (kVec) {
+                    sE4[e] = make_float4(E[id], E[g.N + id], E[2 * g.N + id], 0.f);
+                } else {
 #pragma unroll
-                for (int c = 0; c < 3; ++c) sE[c * bk.NB + e] = E[c * g.N + id];
+                    for (int c = 0; c < 3; ++c) sE[c * bk.NB + e] = E[c * g.N + id];
+                }
             }
             for (int e = threadIdx.x; e < bk.CB; e += blockDim.x) {
                 const int lx = e % bk.cbx, ly = (e / bk.cbx) % bk.cby, lz = e / (bk.cbx * bk.cby);
                 const long long id = linw(g, x0 - (ax ? 1 : 0) + lx, y0 - (ay ? 1 : 0) + ly, z0 - (az ? 1 : 0) + lz);
+                if constexpr (kVec) {
+                    sB4[e] = make_float4(B[id], B[g.N + id], B[2 * g.N + id], 0.f);
+                } else {
 #pragma unroll
-                for (int c = 0; c < 3; ++c) sB[c * bk.CB + e] = B[c * g.N + id];
+                    for (int c = 0; c < 3; ++c) sB[c * bk.CB + e] = B[c * g.N + id];
+                }
             }
+            for (int s = 0; s < S.ns; ++s)
+                for (int e = threadIdx.x; e <= T3; e += blockDim.x) sOff[s * (T3 + 1) + e] = S.off[s][key0 + e];
         }
         __syncthreads();
         for (int s = 0; s < S.ns; ++s) {
             const PartView<T> p = S.p[s];
+            const double cq = K.cq[s], cm = K.cm[s];
+            const T beta = K.beta[s], ms = K.m[s];
+            if constexpr (kStaged) {
+                const int* __restrict__ of = sOff + s * (T3 + 1);
+                // the warp's chunks: keys warp, warp + nwarps, ... of the tile
+                // (empty ones skipped), each 32 particles at a time
+                auto next_key = [&](int lc) {
+                    while (lc < T3 && of[lc] == of[lc + 1]) lc += nwarps;
+                    return lc;
+                };
+                int lc = next_key(warp), c0 = lc < T3 ? of[lc] : 0;
+                if (lc < T3 && c0 + lane < of[lc + 1]) stage_particle(buf, p, c0 + lane, lane);
+                cp_async_commit();
+                int key = -1, cellK = 0, nbK = 0, cbK = 0;
+                float an[4] = {0.f, 0.f, 0.f, 0.f}, ac[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                while (lc < T3) {
+                    if (lc != key) {
+                        key = lc;
+                        const int li = lc % t.tx, q = lc / t.tx, lj = q % t.ty, lk = q / t.ty;
+                        nbK = lk * nsz + lj * nsy + li;
+                        cbK = lk * csz + lj * csy + li;
+                        cellK = (int)lin(g, x0 + li, y0 + lj, z0 + lk);
+                    }
+                    const bool valid = c0 + lane < of[lc + 1];
+                    cp_async_wait_all();   // a lane's own slots
+                    const int cell = buf->cell[lane];
+                    const T ox = buf->a[0][lane], oy = buf->a[1][lane], oz = buf->a[2][lane];
+                    const T mom[3] = {buf->a[3][lane], buf->a[4][lane], buf->a[5][lane]};
+                    int nlc = lc, nc0 = c0 + 32;
+                    if (nc0 >= of[lc + 1]) {
+                        nlc = next_key(lc + nwarps);
+                        nc0 = nlc < T3 ? of[nlc] : 0;
+                    }
+                    if (nlc < T3 && nc0 + lane < of[nlc + 1]) stage_particle(buf, p, nc0 + lane, lane);
+                    cp_async_commit();
+                    // raw quantities: rv (3), alpha (9), node weights x/y/z (2 each), cell weights x/y/z (3 each)
+                    T row[kScrRow];
+                    const bool mine = valid && cell == cellK;   // (always, after a sort)
+                    if (valid) {
+                        T gam, v[3];
+                        gamma_vel<T>(mom, ms, gam, v);
+                        T* nw = row + 12;
+                        T* cw = row + 18;
+                        axis_weights<T>(ox, ax, nw, cw);
+                        axis_weights<T>(oy, ay, nw + 2, cw + 3);
+                        axis_weights<T>(oz, az, nw + 4, cw + 6);
+                        T e[3], bf[3];
+                        if (mine) {
+                            T w[8];
+                            corners<T>(nw[1], nw[3], nw[5], w);
+                            if constexpr (kVec) gather3(sE4, nbK, oxn, oyn, ozn, w, e);
+                            else gather3<T>(sE, bk.NB, nbK, oxn, oyn, ozn, w, e);
+                            // cell pair (c - 1, c) below the centre, (c, c + 1) above
+                            const bool bx = ox < T(0.5), by = oy < T(0.5), bz = oz < T(0.5);
+                            corners<T>(bx ? cw[1] : cw[2], by ? cw[4] : cw[5], bz ? cw[7] : cw[8], w);
+                            const int cbase = cbK + (bx ? 0 : oxc) + (by ? 0 : oyc) + (bz ? 0 : ozc);
+                            if constexpr (kVec) gather3(sB4, cbase, oxc, oyc, ozc, w, bf);
+                            else gather3<T>(sB, bk.CB, cbase, oxc, oyc, ozc, w, bf);
+                        } else {
+                            int i, j, k;
+                            decode(g, cell, i, j, k);
+                            const EB6<T> r = gather_eb_global<T>(g, i, j, k, ox, oy, oz, E, B);
+#pragma unroll
+                            for (int c = 0; c < 3; ++c) { e[c] = r.e[c]; bf[c] = r.b[c]; }
+                        }
+                        T al[9];
+                        alpha_tensor<T>(beta, v, gam, e, bf, al);
+                        const T vg[3] = {v[0] * gam, v[1] * gam, v[2] * gam};
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) row[a] = al[3 * a] * vg[0] + al[3 * a + 1] * vg[1] + al[3 * a + 2] * vg[2];
+#pragma unroll
+                        for (int d = 0; d < 9; ++d) row[3 + d] = al[d];
+                        if (!mine) deposit_row_global<A, T>(g, cell, ox, oy, oz, row, cq, cm, J, mu, rho, Pi);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < kScrRow; ++q) row[q] = T(0);
+                    }
+                    const unsigned mm = __ballot_sync(0xffffffffu, mine);
+                    if constexpr (kTc) {
+                        if (mm) tc_run_sums(scr, lane, mine, mm, row, an, ac, s_lane[lane]);
+                        if (nlc != lc) {   // the key's sums reach the block once
+                            add_run_sums(sN, sC, bk.NB, bk.CB, nbK, cbK, oxn, oyn, ozn, oxc, oyc, ozc, lane, an, ac, float(cq),
+                                         float(cm));
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) an[q] = 0.f;
+#pragma unroll
+                            for (int q = 0; q < 8; ++q) ac[q] = 0.f;
+                        }
+                    } else if (__popc(mm) >= kXposeMin) {
+                        butterfly_sums<A, T>(row, mine, cq, cm, sN, sC, bk.NB, bk.CB, nbK, cbK, oxn, oyn, ozn, oxc, oyc, ozc,
+                                             lane);
+                    } else if (mine) {
+                        imp_deposit_direct<A, T>(row, cq, cm, sN, sC, bk.NB, bk.CB, nbK, cbK, oxn, oyn, ozn, oxc, oyc, ozc);
+                    }
+                    lc = nlc;
+                    c0 = nc0;
+                }
+                continue;
+            }
             const int* __restrict__ off = S.off[s];
-            const double qs = S.q[s], ms = S.m[s], ws = S.w[s];
-            const T beta = T(0.5 * qs * g.dt / ms);
-            const double cq = qs * ws * ivol;
-            const double cm = -(ws * g.theta * g.dt * g.dt * 2 * PI_D * qs * qs / ms) * ivol;
             for (int lc = warp; lc < T3; lc += nwarps) {
                 const int kk = key0 + lc;
                 const int b0 = off[kk], b1 = off[kk + 1];
-                // Right after a sort the particles of this key lie in the key's cell:
-                // the tensor-core sums of all its chunks accumulate and reach the
-                // block once.
-                constexpr bool kCellAcc = kStaged && kTc;
-                float an[4] = {0.f, 0.f, 0.f, 0.f}, ac[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                bool acc_any = false;
-                int nbK = 0, cbK = 0;
-                if constexpr (kCellAcc) {
-                    const int li = lc % t.tx, lj = (lc / t.tx) % t.ty, lk = lc / (t.tx * t.ty);
-                    nbK = (lk + hz) * nsz + (lj + hy) * nsy + (li + hx);
-                    cbK = (lk + hz) * csz + (lj + hy) * csy + (li + hx);
-                }
                 for (int c0 = b0; c0 < b1; c0 += 32) {
                     const int n = c0 + lane;
                     const bool valid = n < b1;
@@ -479,7 +637,7 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
                         const T ox = p.ox[n], oy = p.oy[n], oz = p.oz[n];
                         T mom[3] = {p.px[n], p.py[n], p.pz[n]};
                         T gam, v[3];
-                        gamma_vel<T>(mom, T(ms), gam, v);
+                        gamma_vel<T>(mom, ms, gam, v);
                         T* nw = row + 12;
                         T* cw = row + 18;
                         axis_weights<T>(ox, ax, nw, cw);
@@ -493,25 +651,8 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
                             cb = (lk + hz) * csz + (lj + hy) * csy + (li + hx);
                         }
                         T e[3], bf[3];
-                        if (kStaged && inb) {
-                            // node pair (c, c+1); cell pair (c-1, c) below the centre, (c, c+1) above
-                            const int cbase = cb + (ox < T(0.5) ? 0 : oxc) + (oy < T(0.5) ? 0 : oyc) + (oz < T(0.5) ? 0 : ozc);
-                            const T ux = ox < T(0.5) ? cw[1] : cw[2];
-                            const T uy = oy < T(0.5) ? cw[4] : cw[5];
-                            const T uz = oz < T(0.5) ? cw[7] : cw[8];
-#pragma unroll
-                            for (int c = 0; c < 3; ++c) {
-                                e[c] = tri_block<T>(sE + c * bk.NB, nb, oxn, oyn, ozn, nw[1], nw[3], nw[5]);
-                                bf[c] = tri_block<T>(sB + c * bk.CB, cbase, oxc, oyc, ozc, ux, uy, uz);
-                            }
-                        } else if (kStaged) {
-                            const EB6<T> r = gather_eb_global<T>(g, i, j, k, ox, oy, oz, E, B);
-#pragma unroll
-                            for (int c = 0; c < 3; ++c) { e[c] = r.e[c]; bf[c] = r.b[c]; }
-                        } else {
-                            gather_node<T, T>(g, i, j, k, ox, oy, oz, E, e);
-                            gather_cell<T, T>(g, i, j, k, ox, oy, oz, B, bf);
-                        }
+                        gather_node<T, T>(g, i, j, k, ox, oy, oz, E, e);
+                        gather_cell<T, T>(g, i, j, k, ox, oy, oz, B, bf);
                         T al[9];
                         alpha_tensor<T>(beta, v, gam, e, bf, al);
                         const T vg[3] = {v[0] * gam, v[1] * gam, v[2] * gam};
@@ -519,27 +660,9 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
                         for (int a = 0; a < 3; ++a) row[a] = al[3 * a] * vg[0] + al[3 * a + 1] * vg[1] + al[3 * a + 2] * vg[2];
 #pragma unroll
                         for (int d = 0; d < 9; ++d) row[3 + d] = al[d];
-                        if (!inb) {
-                            A QN[12], QC[7];
-                            run_quantities<A, T>(row, cq, cm, QN, QC);
-                            double qn[12], qc[7];
-#pragma unroll
-                            for (int d = 0; d < 12; ++d) qn[d] = double(QN[d]);
-#pragma unroll
-                            for (int d = 0; d < 7; ++d) qc[d] = double(QC[d]);
-                            imp_deposit_global<T>(g, i, j, k, ox, oy, oz, qn, qc, J, mu, rho, Pi);
-                        }
+                        if (!inb) deposit_row_global<A, T>(g, cell, ox, oy, oz, row, cq, cm, J, mu, rho, Pi);
                     }
                     unsigned pending = __ballot_sync(0xffffffffu, valid && inb);
-                    if constexpr (kCellAcc) {
-                        const bool mine = valid && inb && nb == nbK;
-                        const unsigned mm = __ballot_sync(0xffffffffu, mine);
-                        if (mm) {
-                            tc_run_sums(scr, lane, mine, mm, row, an, ac, s_lane[lane]);
-                            acc_any = true;
-                        }
-                        pending &= ~mm;
-                    }
                     while (pending) {
                         const int leader = __ffs(pending) - 1;
                         const int lcell = __shfl_sync(0xffffffffu, cell, leader);
@@ -555,45 +678,13 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
                                 add_run_sums(sN, sC, bk.NB, bk.CB, nbL, cbL, oxn, oyn, ozn, oxc, oyc, ozc, lane, dn, dc,
                                              float(cq), float(cm));
                             } else {
-                                A QN[12], QC[7], wn[8], wc[27];
-                                run_quantities<A, T>(row, cq, cm, QN, QC);
-                                run_weights<A, T>(row, wn, wc);
-                                A vv[32];
-#pragma unroll
-                                for (int r = 0; r < 3; ++r) {
-#pragma unroll
-                                    for (int x = 0; x < 32; ++x) vv[x] = me ? QN[4 * r + x / 8] * wn[x % 8] : A(0);
-                                    const A sum = xpose_sum<A>(vv, lane);
-                                    const int q = 4 * r + lane / 8, c = lane % 8;
-                                    if (sum != A(0))
-                                        atomicAdd(&sN[q * bk.NB + nbL + (c & 1) * oxn + ((c >> 1) & 1) * oyn + (c >> 2) * ozn],
-                                                  sum);
-                                }
-#pragma unroll
-                                for (int r = 0; r < 6; ++r) {
-#pragma unroll
-                                    for (int x = 0; x < 32; ++x) {
-                                        const int idx = 32 * r + x;
-                                        vv[x] = (idx < 189 && me) ? QC[idx / 27] * wc[idx % 27] : A(0);
-                                    }
-                                    const A sum = xpose_sum<A>(vv, lane);
-                                    const int idx = 32 * r + lane;
-                                    if (idx < 189 && sum != A(0)) {
-                                        const int q = idx / 27, sl = idx % 27;
-                                        atomicAdd(&sC[q * bk.CB + cbL + (sl % 3) * oxc + ((sl / 3) % 3) * oyc + (sl / 9) * ozc],
-                                                  sum);
-                                    }
-                                }
+                                butterfly_sums<A, T>(row, me, cq, cm, sN, sC, bk.NB, bk.CB, nbL, cbL, oxn, oyn, ozn, oxc, oyc, ozc,
+                                                     lane);
                             }
                         } else if (me) {
                             imp_deposit_direct<A, T>(row, cq, cm, sN, sC, bk.NB, bk.CB, nb, cb, oxn, oyn, ozn, oxc, oyc, ozc);
                         }
                     }
-                }
-                if constexpr (kCellAcc) {
-                    if (acc_any)
-                        add_run_sums(sN, sC, bk.NB, bk.CB, nbK, cbK, oxn, oyn, ozn, oxc, oyc, ozc, lane, an, ac, float(cq),
-                                     float(cm));
                 }
             }
         }

@@ -74,7 +74,7 @@ struct PK {
     // tiled deposit (implicit_tile.cuh), periodic pressure placement; needs
     // tile-major sorted particles
     static ImpBlock implicit_block(const GridP& g, const TileGeom& t, int h);
-    static size_t implicit_tile_smem(const ImpBlock& bk);
+    static size_t implicit_tile_smem(const ImpBlock& bk, int keys);   // keys per (sub-)tile
     static void implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileSplit& sp,
                                        const ImpBlock& bk,
                                        const ImpSpecies<T>& S, const T* E, const T* B, double* J,

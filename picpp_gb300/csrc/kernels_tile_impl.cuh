@@ -76,6 +76,7 @@ template <typename T>
 ImpBlock PK<T>::implicit_block(const GridP& g, const TileGeom& t, int h) {
     ImpBlock b{};
     b.h = h;
+    b.areal = sizeof(T);
     b.nbx = g.nx > 1 ? t.tx + 2 * h + 1 : 1;
     b.nby = g.y3 ? t.ty + 2 * h + 1 : 1;
     b.nbz = g.z3 ? t.tz + 2 * h + 1 : 1;
@@ -88,13 +89,15 @@ ImpBlock PK<T>::implicit_block(const GridP& g, const TileGeom& t, int h) {
 }
 
 template <typename T>
-size_t PK<T>::implicit_tile_smem(const ImpBlock& bk) {
-    // FP32 accumulators add the per-warp rows of the tensor-core run sums
-    // and their 32-entry lane table
-    const size_t scratch = sizeof(T) == sizeof(float)
-                               ? (size_t)(imp_threads<T>() / 32) * kScrParticles * kScrRow * sizeof(float) + 32 * sizeof(TcLane)
-                               : 0;
-    return (12 * (size_t)bk.NB + 7 * (size_t)bk.CB + (bk.stage ? 3 * ((size_t)bk.NB + bk.CB) : 0)) * sizeof(T) + scratch;
+size_t PK<T>::implicit_tile_smem(const ImpBlock& bk, int keys) {
+    // FP32 accumulators: the per-warp rows of the tensor-core run sums and
+    // their 32-entry lane table; staged: every warp's next chunk of particles
+    // and the offsets of the sub-tile's keys for all species
+    size_t n = bk.scratch_at();
+    if (sizeof(T) == sizeof(float))
+        n += (size_t)(imp_threads<T>() / 32) * kScrParticles * kScrRow * sizeof(float) + 32 * sizeof(TcLane);
+    if (bk.stage) n += (size_t)(imp_threads<T>() / 32) * sizeof(ChunkBuf<T>) + (size_t)kMaxSpecies * (keys + 1) * sizeof(int);
+    return n;
 }
 
 template <typename T>
@@ -108,7 +111,7 @@ void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeo
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         attr_set = true;
     }
-    const size_t smem = implicit_tile_smem(bk);
+    const size_t smem = implicit_tile_smem(bk, t.tx * t.ty * t.tz);
     const int per_sm = (int)((227 * 1024) / (smem + 1024));
     const int ntiles = t.ntx * t.nty * t.ntz;
     const int grid = ntiles < kNumSM * (per_sm > 0 ? per_sm : 1) ? ntiles : kNumSM * (per_sm > 0 ? per_sm : 1);
@@ -116,7 +119,16 @@ void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeo
     const bool split = sp.sx * sp.sy * sp.sz > 1;
     auto* kernel = !bk.stage ? k_implicit_deposit_tile<T, T, false, false>
                    : split ? k_implicit_deposit_tile<T, T, true, true> : k_implicit_deposit_tile<T, T, true, false>;
-    kernel<<<grid, nt, smem, s>>>(g, t, sp, bk, S, E, B, J, mu, rho, Pi);
+    const double PI_D = 3.14159265358979323846;
+    const double ivol = 1.0 / (g.dx * g.dy * g.dz);
+    DepositSet<T> K{};
+    for (int q = 0; q < S.ns; ++q) {
+        K.beta[q] = T(0.5 * S.q[q] * g.dt / S.m[q]);
+        K.m[q] = T(S.m[q]);
+        K.cq[q] = S.q[q] * S.w[q] * ivol;
+        K.cm[q] = -(S.w[q] * g.theta * g.dt * g.dt * 2 * PI_D * S.q[q] * S.q[q] / S.m[q]) * ivol;
+    }
+    kernel<<<grid, nt, smem, s>>>(g, t, sp, bk, S, K, E, B, J, mu, rho, Pi);
 }
 
 template <typename T>
