@@ -50,6 +50,8 @@ struct pic_ctx {
     GridP g{};
     TileGeom tg{};
     TileShape ts{};
+    TileGeom wg{};          // work tiles of the fused explicit kernel (merge_geom) and their shape
+    TileShape ws{};
     GhostAxes ga{};
     int nkeys = 0, ntiles = 0, T3 = 0;
     int preal = 0;
@@ -273,6 +275,27 @@ pic_status smooth_moments(pic_ctx* ctx) {
 // particles, one with FP64 ones.
 int explicit_parts(const TileGeom& t, int preal) { return tile_parts(t, preal ? kNumSM : 2 * kNumSM, preal != 0); }
 
+// Work tiles of the fused explicit kernel: 8^3 cells, several of the sort's
+// tiles each, where the caller left the tiles to the library and some axis is
+// no multiple of 8 (its default tile is then smaller).  At 100x60x54 (4x4x2
+// tiles of 288 particles per species) a CTA per tile spent its time staging
+// and flushing halo: 428 us per step, 273 us with work tiles.  Axes below 8 cells
+// keep the sort's tiles: a work tile would wrap onto itself.
+void merge_geom(const pic_config& c, const TileGeom& t, TileGeom& w, TileShape& ws) {
+    const int n[3] = {c.nx, c.ny, c.nz}, e[3] = {t.tx, t.ty, t.tz};
+    bool small = false;
+    for (int a = 0; a < 3; ++a) {
+        if (c.tile[a] > 0 || n[a] < 8 || 8 % e[a] != 0) return;
+        small = small || e[a] < 8;
+    }
+    if (!small || c.boundary_x != PIC_BOUNDARY_PERIODIC) return;
+    w.tx = w.ty = w.tz = 8;
+    w.ntx = (n[0] + 7) / 8; w.nty = (n[1] + 7) / 8; w.ntz = (n[2] + 7) / 8;
+    w.lx = w.ly = w.lz = 3;
+    ws.fx = ws.fy = ws.fz = ws.jx = ws.jy = ws.jz = 12;
+    ws.jcells = 12 * 12 * 12;
+}
+
 template <typename T>
 pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
     cudaStream_t s = ctx->s;
@@ -297,11 +320,11 @@ pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
                 S.defer[q] = ctx->sp[q].defer;
                 S.dwords[q] = ctx->sp[q].dwords;
             }
-            const int parts = explicit_parts(ctx->tg, ctx->preal);
+            const int parts = explicit_parts(ctx->wg, ctx->preal);
             {
                 Phase ph(ctx, PIC_PHASE_PUSH_DEPOSIT, 2);   // the fused kernel and its deferred pass
-                PK<T>::push_deposit_tiled(s, g, ctx->tg, ctx->ts, S, ctx->E, ctx->B, (double*)ctx->Jpart, ctx->Jfix,
-                                          parts, PK<T>::tile_smem_bytes(ctx->ts));
+                PK<T>::push_deposit_tiled(s, g, ctx->wg, ctx->tg, ctx->ws, S, ctx->E, ctx->B, (double*)ctx->Jpart,
+                                          ctx->Jfix, parts);
             }
             {
                 Phase ph(ctx, PIC_PHASE_FIELDS, 1);
@@ -309,7 +332,7 @@ pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
             }
             {
                 Phase ph(ctx, PIC_PHASE_ASSEMBLE, 1);
-                PK<T>::assemble_j(s, g, ctx->tg, ctx->ts, (const double*)ctx->Jpart, ctx->Jfix, ctx->J,
+                PK<T>::assemble_j(s, g, ctx->wg, ctx->ws, (const double*)ctx->Jpart, ctx->Jfix, ctx->J,
                                   1.0 / (double)PK<T>::fixed_scale(g, S), parts);
             }
         } else {
@@ -576,10 +599,13 @@ pic_status pic_create(const pic_config* cfg, pic_ctx** out) {
     ts.jcells = (long long)ts.jx * ts.jy * ts.jz;
     // the fused explicit kernel holds the tile's fields and current in shared memory
     if (c.solver == PIC_SOLVER_BUNEMAN &&
-        (ctx->preal ? PK<double>::tile_smem_bytes(ts) : PK<float>::tile_smem_bytes(ts)) > 200 * 1024) {
+        (ctx->preal ? PK<double>::tile_smem_bytes(ts, false) : PK<float>::tile_smem_bytes(ts, false)) > 200 * 1024) {
         delete ctx;
         return PIC_ERR_ARG;
     }
+    ctx->wg = t;
+    ctx->ws = ts;
+    merge_geom(c, t, ctx->wg, ctx->ws);
     GhostAxes& ga = ctx->ga;
     ga.cex = c.nx > 1 ? c.nx + 4 : 1; ga.cey = c.ny > 1 ? c.ny + 4 : 1; ga.cez = c.nz > 1 ? c.nz + 4 : 1;
     ga.gx = c.nx > 1 ? 2 : 0; ga.gy = c.ny > 1 ? 2 : 0; ga.gz = c.nz > 1 ? 2 : 0;
@@ -605,7 +631,8 @@ pic_status pic_create(const pic_config* cfg, pic_ctx** out) {
         ok = ok && A(&ctx->B, ctx->rsz * 3 * N);
         ok = ok && A(&ctx->J, sizeof(double) * 3 * N);
         ok = ok && A(&ctx->Jfix, sizeof(double) * 3 * N);
-        ok = ok && A(&ctx->Jpart, sizeof(double) * 3 * (size_t)ts.jcells * ctx->ntiles * explicit_parts(t, ctx->preal));
+        ok = ok && A(&ctx->Jpart, sizeof(double) * 3 * (size_t)ctx->ws.jcells * ctx->wg.ntx * ctx->wg.nty * ctx->wg.ntz *
+                                   explicit_parts(ctx->wg, ctx->preal));
     } else {
         ctx->pi_len = c.pressure_compat ? 9LL * ga.cex * ga.cey * ga.cez : 9 * N;
         ctx->jg_len = c.pressure_compat ? 3LL * ctx->nex * ctx->ney * ctx->nez : 3 * N;

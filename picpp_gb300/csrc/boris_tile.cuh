@@ -249,6 +249,56 @@ __device__ __forceinline__ void add_runs_fx(unsigned* __restrict__ lo, int* __re
     __syncwarp();
 }
 
+// The fused kernel's constants in the particle precision.
+template <typename TP>
+struct PushSet {
+    TP dt, idt, d[3], id[3], hid[3];
+    TP q[kMaxSpecies], m[kMaxSpecies], beta[kMaxSpecies], fcd[kMaxSpecies];
+    float fx_scale;   // fixed-point scale (FP32)
+    int parts;        // CTAs per tile
+};
+
+// The tiles of a work tile (kMerge), x fastest: chunks of 32 particles in the
+// tiles before each, first particle and count.
+constexpr int kMergeTiles = 512;   // tiles of one cell in 8^3
+struct MergeTable {
+    int before[kMergeTiles + 1];
+    unsigned first[kMergeTiles], count[kMergeTiles];
+    int warp_total[kTileThreads / 32];
+};
+// Fills the table for one species (all threads; a thread per tile).
+__device__ __forceinline__ void merge_table(MergeTable* M, const int* __restrict__ off, const TileGeom& o, int ti, int tj,
+                                            int tk) {
+    static_assert(kTileThreads == kMergeTiles, "a thread per tile");
+    const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
+    const int gx = 8 / o.tx, gy = 8 / o.ty, gz = 8 / o.tz;
+    const int a = ti * gx + e % gx, b = tj * gy + e / gx % gy, c = tk * gz + e / (gx * gy);
+    int first = 0, count = 0;
+    if (e < gx * gy * gz && a < o.ntx && b < o.nty && c < o.ntz) {
+        const int T3 = o.tx * o.ty * o.tz;
+        const long long k0 = ((long long)(c * o.nty + b) * o.ntx + a) * T3;
+        first = off[k0];
+        count = off[k0 + T3] - first;
+    }
+    const int mine = (count + 31) / 32;
+    int x = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= d) x += y;
+    }
+    __syncthreads();   // the species before is done with the table
+    if (lane == 31) M->warp_total[warp] = x;
+    __syncthreads();
+    int base = 0;
+    for (int w = 0; w < warp; ++w) base += M->warp_total[w];
+    M->before[e] = base + x - mine;
+    M->first[e] = (unsigned)first;
+    M->count[e] = (unsigned)count;
+    if (e == kMergeTiles - 1) M->before[kMergeTiles] = base + x;
+    __syncthreads();
+}
+
 // CT: compile-time tile extent of a cubic 3-D tile (8), or 0 for shapes read
 // from TileShape at run time.  kWall: conductor-wall box (GridP::wall), the
 // Tristan mover's reflection and escape and the zigzag wall term
@@ -256,11 +306,20 @@ __device__ __forceinline__ void add_runs_fx(unsigned* __restrict__ lo, int* __re
 // escaped deposits its current and is marked (cell -1) for the next sort.
 // kParts: several CTAs per tile (parts > 1); without it the loop keeps no
 // register for the stride (64 are all it has).
-template <typename TP, typename TF, int CT, bool kWall, bool kParts>
-__global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_tile(GridP g, TileGeom t, TileShape s, SpeciesSet<TP> S,
+// kMerge: t holds work tiles of CT^3 cells, each several of the sort's tiles o
+// (ragged at the box's upper ends): a box whose axes no 8-cell tile divides is
+// sorted by smaller tiles, and a CTA per such tile would stage and flush more
+// cells of halo than it has of its own.  A warp's 32 particles always come from
+// one of the sort's tiles, counted from its first, and a particle's distance
+// is measured from that tile, so the sums of a run, and which particles are
+// left to the deferred pass, are those of a CTA per tile, bit for bit (FP32).
+// At 100x60x54, 9 per species and cell (tiles of 4x4x2): 428 -> 273 us.
+template <typename TP, typename TF, int CT, bool kWall, bool kParts, bool kMerge>
+__global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_tile(GridP g, TileGeom t, TileGeom o, TileShape s,
+                                                                       SpeciesSet<TP> S,
+                                                                       const __grid_constant__ PushSet<TP> K,
                                                                        const TF* __restrict__ E, const TF* __restrict__ B,
-                                                                       double* __restrict__ Jpart, float fx_scale,
-                                                                       double inv_dt, int nparts) {
+                                                                       double* __restrict__ Jpart) {
     constexpr bool kFixed = sizeof(TP) == sizeof(float);   // FP32 particles: fixed-point block
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int fx = CT ? CT + 4 : s.fx, fy = CT ? CT + 4 : s.fy, fz = CT ? CT + 4 : s.fz;
@@ -279,16 +338,21 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
     float* sW = reinterpret_cast<float*>(after_j + (threadIdx.x >> 5) * kSpreadBytes);
     ChunkBuf<TP>* sBuf = reinterpret_cast<ChunkBuf<TP>*>(after_j + (kFixed ? (blockDim.x >> 5) * kSpreadBytes : 0)) +
                          (threadIdx.x >> 5);
+    // kMerge: of the work tile's tiles, the chunks before each and its first
+    // particle and count of this species
+    MergeTable* sM = reinterpret_cast<MergeTable*>(reinterpret_cast<unsigned char*>(sBuf - (threadIdx.x >> 5)) +
+                                                   (kTileThreads / 32) * sizeof(ChunkBuf<TP>));
     const int ntiles = t.ntx * t.nty * t.ntz;
-    const int T3 = tx * ty * tz;
     const long long N = g.N;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // reciprocals from the host (no FP64 division per thread)
-    const TP dt = TP(g.dt), idt = TP(inv_dt);
-    const TP dx = TP(g.dx), dy = TP(g.dy), dz = TP(g.dz);
-    const TP idx = TP(g.idx), idy = TP(g.idy), idz = TP(g.idz);
-    const TP vol = dx * dy * dz;
-    const int parts = kParts ? nparts : 1;
+    // (in the particle precision already: of the FP64 grid parameters the
+    // compiler repeats four conversions per chunk, on the FP64 pipe)
+    const TP dt = K.dt, idt = K.idt;
+    const TP dx = K.d[0], dy = K.d[1], dz = K.d[2];
+    const TP idx = K.id[0], idy = K.id[1], idz = K.id[2];
+    const int parts = kParts ? K.parts : 1;
+    // extents of the sort's tiles
+    const int otx = kMerge ? o.tx : tx, oty = kMerge ? o.ty : ty, otz = kMerge ? o.tz : tz;
     const int ey = CT ? 1 : (g.y3 ? 1 : 0), ez = CT ? 1 : (g.z3 ? 1 : 0);
     const int fsy = ey ? fx : 0, fsz = ez ? fx * fy : 0;
 
@@ -316,20 +380,43 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
 
         for (int sp = 0; sp < S.ns; ++sp) {
             const PartView<TP> P = S.p[sp];
-            const TP q = S.q[sp], m = S.m[sp];
-            const TP beta = q * dt / (TP(2) * m);
-            const TP fcd = q * S.w[sp] / vol;
-            // (unsigned: a species holds fewer than 2^31 particles)
-            using IDX = std::conditional_t<kParts, unsigned, long long>;
-            const IDX pb = S.off[sp][(long long)tile * T3] + part * blockDim.x;
-            const IDX pe = S.off[sp][(long long)(tile + 1) * T3];
-            // CTA-uniform chunk loop: warp w takes particles cb + 32 w + lane.
-            // Each warp's next chunk is copied into its shared buffer while
-            // it pushes the current one (the first before the loop).
-            if (pb + threadIdx.x < pe) stage_particle(sBuf, P, pb + threadIdx.x, lane);
+            const TP q = K.q[sp], m = K.m[sp], beta = K.beta[sp], fcd = K.fcd[sp];
+            // A warp takes chunks of 32 consecutive particles of a tile: chunk
+            // warp, warp + nwarps * parts, ... (n0: its first particle, pe: the
+            // end of its tile's).  Each warp's next chunk is copied into its
+            // shared buffer while it pushes the current one.  (IDX unsigned: a
+            // species holds fewer than 2^31 particles.)
+            unsigned n0, pe;
+            int at = 0, c = part * (kTileThreads / 32) + warp, chunks = 0;   // kMerge: tile of the table, chunk, their number
+            auto seek = [&]() {   // kMerge: n0 and pe of chunk c, at or after tile `at`
+                unsigned passed;
+                do {
+                    const int i = at + 1 + lane;
+                    passed = __ballot_sync(0xffffffffu, i <= kMergeTiles && sM->before[i < kMergeTiles ? i : kMergeTiles] <= c);
+                    at += __popc(passed);
+                } while (passed == 0xffffffffu);
+                n0 = sM->first[at] + 32u * (unsigned)(c - sM->before[at]);
+                pe = sM->first[at] + sM->count[at];
+            };
+            if constexpr (kMerge) {
+                merge_table(sM, S.off[sp], o, ti, tj, tk);
+                chunks = sM->before[kMergeTiles];
+                n0 = pe = 0;
+                if (c < chunks) seek();
+            } else {
+                const long long k0 = (long long)tile * (tx * ty * tz);
+                n0 = S.off[sp][k0] + part * kTileThreads + 32 * warp;
+                pe = S.off[sp][k0 + tx * ty * tz];
+            }
+            if (n0 + lane < pe) stage_particle(sBuf, P, n0 + lane, lane);
             cp_async_commit();
-            for (IDX cb = pb; cb < pe; cb += parts * blockDim.x) {
-                const IDX n = cb + threadIdx.x;
+            while (n0 < pe) {
+                const unsigned nb = n0, n = n0 + lane;
+                const bool here = n < pe;
+                // the tile's place in the work tile
+                const int px = kMerge ? (at & (CT / otx - 1)) * otx : 0;
+                const int py = kMerge ? (at / (CT / otx) & (CT / oty - 1)) * oty : 0;
+                const int pz = kMerge ? at / (CT / otx * (CT / oty)) * otz : 0;
                 TP aB[12];
                 TP s1[6] = {TP(0), TP(0), TP(0), TP(0), TP(0), TP(0)};   // F1 and W1 of the old-side segment
                 int keyA = -1 - lane, keyB = -1 - lane;   // lanes outside a reduction keep unique keys
@@ -337,13 +424,20 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
                 // a lane reads and refills only its own slots, and the wait
                 // covers the copies it started itself
                 cp_async_wait_all();
-                const int cell = n < pe ? sBuf->cell[lane] : -1;
+                const int cell = here ? sBuf->cell[lane] : -1;
                 TP ox = sBuf->a[0][lane], oy = sBuf->a[1][lane], oz = sBuf->a[2][lane];
                 TP mom[3] = {sBuf->a[3][lane], sBuf->a[4][lane], sBuf->a[5][lane]};
-                if (n + parts * blockDim.x < pe) stage_particle(sBuf, P, n + parts * blockDim.x, lane);
+                if constexpr (kMerge) {
+                    c += parts * (kTileThreads / 32);
+                    if (c < chunks) seek();
+                    else n0 = pe;
+                } else {
+                    n0 += parts * kTileThreads;
+                }
+                if (n0 + lane < pe) stage_particle(sBuf, P, n0 + lane, lane);
                 cp_async_commit();
                 // (an escaped particle of a wall box waits with cell -1 for the sort)
-                if (n < pe && (!kWall || cell >= 0)) {
+                if (here && (!kWall || cell >= 0)) {
                     int i, j, k;
                     decode(g, cell, i, j, k);
                     auto local = [](int c, int lo, int te, int nn) {
@@ -352,17 +446,17 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
                         if (l < -1) l += nn;
                         return l;
                     };
-                    const int li = local(i, lox, tx, g.nx);
-                    const int lj = ey ? local(j, loy, ty, g.ny) : 0;
-                    const int lk = ez ? local(k, loz, tz, g.nz) : 0;
-                    const bool fast = li >= -1 && li <= tx && lj >= -ey && lj <= ty * ey && lk >= -ez && lk <= tz * ez;
+                    const int li = local(i, lox + px, otx, g.nx);
+                    const int lj = ey ? local(j, loy + py, oty, g.ny) : 0;
+                    const int lk = ez ? local(k, loz + pz, otz, g.nz) : 0;
+                    const bool fast = li >= -1 && li <= otx && lj >= -ey && lj <= oty * ey && lk >= -ez && lk <= otz * ez;
                     push_later = !fast;
                     if (fast) {
                         TP e3[3], b3[3];
                         // upper-neighbour weights: node grids (c, c+1) with weight u;
                         // cell-centred grids (c-1, c) with u + 1/2 below the centre,
                         // (c, c+1) with u - 1/2 above it (correlation.cpp:471-496)
-                        const int c0 = (lk + hz) * fsz + (lj + hy) * fsy + (li + hx);
+                        const int c0 = (lk + pz + hz) * fsz + (lj + py + hy) * fsy + (li + px + hx);
                         const int cxs = ox < TP(0.5) ? -1 : 0;
                         const int cys = (ey && oy < TP(0.5)) ? -fsy : 0;
                         const int czs = (ez && oz < TP(0.5)) ? -fsz : 0;
@@ -414,26 +508,27 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
                         if constexpr (kWall) {
                             if (ni == kTristanWallNode && v[0] > TP(0) && PX < TP(0)) PX = -PX;
                         }
-                        const int rx = (int)dev_floor((PX) * idx);
-                        const int ry = ey ? (int)dev_floor((PY) * idy) : 0;
-                        const int rz = ez ? (int)dev_floor((PZ) * idz) : 0;
+                        const TP fxr = dev_floor(PX * idx), fyr = ey ? dev_floor(PY * idy) : TP(0),
+                                 fzr = ez ? dev_floor(PZ * idz) : TP(0);
+                        const int rx = (int)fxr, ry = (int)fyr, rz = (int)fzr;
                         const TP RX = rx == 0 ? (X + PX) * TP(0.5) : TP(rx > 0 ? rx : 0) * dx;
                         const TP RY = ry == 0 ? (Y + PY) * TP(0.5) : TP(ry > 0 ? ry : 0) * dy;
                         const TP RZ = rz == 0 ? (Z + PZ) * TP(0.5) : TP(rz > 0 ? rz : 0) * dz;
                         const int ax = bx + rx, ay = by + ry, az = bz + rz;   // block cell of the old-side segment
                         // unsigned compares: (unsigned)x < n is 0 <= x < n
+                        const int ex_ = kMerge ? otx + 4 : jx, ey_ = kMerge ? oty + 4 : jy, ez_ = kMerge ? otz + 4 : jz;
                         const bool inblock = nearx && (unsigned)(rx + 1) <= 2u && (unsigned)(ry + 1) <= 2u &&
-                                             (unsigned)(rz + 1) <= 2u && (unsigned)ax < (unsigned)(jx - 1) &&
-                                             (unsigned)bx < (unsigned)(jx - 1) && (unsigned)ay < (unsigned)(jy - ey) &&
-                                             (unsigned)by < (unsigned)(jy - ey) && (unsigned)az < (unsigned)(jz - ez) &&
-                                             (unsigned)bz < (unsigned)(jz - ez);
+                                             (unsigned)(rz + 1) <= 2u && (unsigned)ax < (unsigned)(ex_ - 1) &&
+                                             (unsigned)bx < (unsigned)(ex_ - 1) && (unsigned)ay < (unsigned)(ey_ - ey) &&
+                                             (unsigned)by < (unsigned)(ey_ - ey) && (unsigned)az < (unsigned)(ez_ - ez) &&
+                                             (unsigned)bz < (unsigned)(ez_ - ez);
                         if (inblock) {
                             const TP F1x = (fcd * (RX - PX)) * idt;
                             const TP F1y = (fcd * (RY - PY)) * idt;
                             const TP F1z = (fcd * (RZ - PZ)) * idt;
                             const TP F2x = (fcd * (X - RX)) * idt;
                             const TP F2y = fmadd<TP>(fcd, v[1], -F1y), F2z = fmadd<TP>(fcd, v[2], -F1z);
-                            const TP hxx = TP(0.5) * idx, hyy = TP(0.5) * idy, hzz = TP(0.5) * idz;
+                            const TP hxx = K.hid[0], hyy = K.hid[1], hzz = K.hid[2];   // half reciprocals
                             const TP W1x = fmadd<TP>(PX + RX, hxx, -TP(rx));
                             const TP W1y = ey ? fmadd<TP>(PY + RY, hyy, -TP(ry)) : TP(0);
                             const TP W1z = ez ? fmadd<TP>(PZ + RZ, hzz, -TP(rz)) : TP(0);
@@ -442,8 +537,8 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
                             const TP W2z = ez ? (Z + RZ) * hzz : TP(0);
                             segment_slots<TP>(F2x, F2y, F2z, W2x, W2y, W2z, aB);
                             s1[0] = F1x; s1[1] = F1y; s1[2] = F1z; s1[3] = W1x; s1[4] = W1y; s1[5] = W1z;
-                            keyA = (az * jy + ay) * jx + ax;
-                            keyB = (bz * jy + by) * jx + bx;
+                            keyA = ((az + pz) * jy + ay + py) * jx + ax + px;
+                            keyB = ((bz + pz) * jy + by + py) * jx + bx + px;
                         }
                         deposit_later = !inblock;
                         // an escaped particle is marked once its current is
@@ -455,8 +550,8 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
                     const unsigned mp = __ballot_sync(0xffffffffu, push_later);
                     const unsigned md = __ballot_sync(0xffffffffu, deposit_later);
                     if ((mp | md) && lane == 0) {
-                        set_defer_bits(S.defer[sp], cb + 32LL * warp, mp);
-                        set_defer_bits(S.defer[sp] + S.dwords[sp], cb + 32LL * warp, md);
+                        set_defer_bits(S.defer[sp], nb, mp);
+                        set_defer_bits(S.defer[sp] + S.dwords[sp], nb, md);
                     }
                 }
                 if (keyB < 0) {
@@ -474,7 +569,7 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
                 const bool crossed = __any_sync(0xffffffffu, keyA >= 0);
                 if constexpr (kFixed) {
                     const bool hb = run_sum<TP>(keyB, aB);
-                    add_runs_fx(sLo, sHi, (int)JC, jx, jx * jy, ey, ez, hb, keyB, (const float*)aB, fx_scale, sW);
+                    add_runs_fx(sLo, sHi, (int)JC, jx, jx * jy, ey, ez, hb, keyB, (const float*)aB, K.fx_scale, sW);
                 } else {
                     if (run_sum<TP>(keyB, aB) && keyB >= 0) add_slots<TP>(sJ, JC, keyB, jx, jx * jy, ey, ez, aB);
                 }
@@ -485,7 +580,7 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
                     segment_slots<TP>(s1[0], s1[1], s1[2], s1[3], s1[4], s1[5], aA);
                     if constexpr (kFixed) {
                         const bool ha = run_sum<TP>(keyA, aA);
-                        add_runs_fx(sLo, sHi, (int)JC, jx, jx * jy, ey, ez, ha, keyA, (const float*)aA, fx_scale, sW);
+                        add_runs_fx(sLo, sHi, (int)JC, jx, jx * jy, ey, ez, ha, keyA, (const float*)aA, K.fx_scale, sW);
                     } else {
                         if (run_sum<TP>(keyA, aA) && keyA >= 0) add_slots<TP>(sJ, JC, keyA, jx, jx * jy, ey, ez, aA);
                     }

@@ -57,17 +57,18 @@ struct PK {
     static void boris_push(cudaStream_t s, const GridP& g, PartView<T> p, double q, double m, const void* E,
                            const void* B);
     static void zigzag(cudaStream_t s, const GridP& g, PartView<T> p, double q, double m, double w, double* J);
-    // fused gather/push/deposit over tiles (boris_tile.cuh), `parts` CTAs
-    // and partial blocks per tile (tile_parts); smem bytes from the caller
-    static void push_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileShape& sh,
+    // fused gather/push/deposit over work tiles t of shape sh (boris_tile.cuh),
+    // each one or several tiles o of the sort, `parts` CTAs and partial blocks
+    // per work tile (tile_parts)
+    static void push_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileGeom& o, const TileShape& sh,
                                    const SpeciesSet<T>& S, const void* E, const void* B, double* Jpart, double* Jfix,
-                                   int parts, size_t smem);
+                                   int parts);
     // J from the tile partials and Jfix; inv_scale = 1 / fixed_scale for FP32
     // particles (integer partials), unused for FP64
     static void assemble_j(cudaStream_t s, const GridP& g, const TileGeom& t, const TileShape& sh, const double* Jpart,
                            const double* Jfix, double* J, double inv_scale, int parts);
     static float fixed_scale(const GridP& g, const SpeciesSet<T>& S);
-    static size_t tile_smem_bytes(const TileShape& sh);
+    static size_t tile_smem_bytes(const TileShape& sh, bool merge);
     static void implicit_deposit(cudaStream_t s, const GridP& g, PartView<T> p, double q, double m, double w,
                                  const double* E, const double* B, double* J, double* mu, double* rho, double* Pi,
                                  int compat, const GhostAxes& ga);

@@ -2,10 +2,9 @@
 // multiply-adds: their time is the number of FP64 instructions.
 #include "kernels_tile_impl.cuh"
 namespace pic {
-template size_t PK<double>::tile_smem_bytes(const TileShape&);
-template void PK<double>::push_deposit_tiled(cudaStream_t, const GridP&, const TileGeom&, const TileShape&,
-                                             const SpeciesSet<double>&, const void*, const void*, double*, double*, int,
-                                             size_t);
+template size_t PK<double>::tile_smem_bytes(const TileShape&, bool);
+template void PK<double>::push_deposit_tiled(cudaStream_t, const GridP&, const TileGeom&, const TileGeom&, const TileShape&,
+                                             const SpeciesSet<double>&, const void*, const void*, double*, double*, int);
 template float PK<double>::fixed_scale(const GridP&, const SpeciesSet<double>&);
 template void PK<double>::assemble_j(cudaStream_t, const GridP&, const TileGeom&, const TileShape&, const double*,
                                      const double*, double*, double, int);

@@ -11,40 +11,60 @@
 namespace pic {
 
 template <typename T>
-size_t PK<T>::tile_smem_bytes(const TileShape& sh) {
+size_t PK<T>::tile_smem_bytes(const TileShape& sh, bool merge) {
     size_t F = (size_t)sh.fx * sh.fy * sh.fz;
     // FP32: the current block is 64-bit fixed point in two 32-bit words,
     // followed by the warps' scratch for spreading the run heads' adds
     const size_t fixed_scratch = sizeof(T) == 4 ? (size_t)(kTileThreads / 32) * kSpreadBytes : 0;
     // and every warp's staged chunk of particles
     return ((6 * F * sizeof(T) + 15) & ~size_t(15)) + ((3 * (size_t)sh.jcells * 8 + 15) & ~size_t(15)) + fixed_scratch +
-           (size_t)(kTileThreads / 32) * sizeof(ChunkBuf<T>);
+           (size_t)(kTileThreads / 32) * sizeof(ChunkBuf<T>) + (merge ? sizeof(MergeTable) : 0);
 }
 
 template <typename T>
-void PK<T>::push_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileShape& sh,
+void PK<T>::push_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileGeom& o, const TileShape& sh,
                                const SpeciesSet<T>& S, const void* E, const void* B, double* Jpart, double* Jfix,
-                               int parts, size_t smem) {
+                               int parts) {
     static bool attr_set = false;
     if (!attr_set) {
-        for (auto* k : {k_push_deposit_tile<T, T, 8, false, false>, k_push_deposit_tile<T, T, 8, false, true>,
-                        k_push_deposit_tile<T, T, 0, false, false>, k_push_deposit_tile<T, T, 0, false, true>,
-                        k_push_deposit_tile<T, T, 0, true, false>, k_push_deposit_tile<T, T, 0, true, true>})
-            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        for (auto* k : {k_push_deposit_tile<T, T, 8, false, false, false>, k_push_deposit_tile<T, T, 8, false, true, false>,
+                        k_push_deposit_tile<T, T, 8, false, true, true>, k_push_deposit_tile<T, T, 0, false, false, false>,
+                        k_push_deposit_tile<T, T, 0, false, true, false>, k_push_deposit_tile<T, T, 0, true, false, false>,
+                        k_push_deposit_tile<T, T, 0, true, true, false>})
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
         attr_set = true;
     }
+    const bool merge = t.tx != o.tx || t.ty != o.ty || t.tz != o.tz;   // (merge_geom: 8^3 work tiles)
     const bool cube8 = t.tx == 8 && t.ty == 8 && t.tz == 8 && g.y3 && g.z3 && sh.fx == 12 && sh.fy == 12 &&
                        sh.fz == 12 && sh.jx == 12 && sh.jy == 12 && sh.jz == 12;
-    const float fx_scale = fixed_scale(g, S);
-    const double inv_dt = 1.0 / g.dt;
     const int grid = std::min(t.ntx * t.nty * t.ntz * parts, kNumSM * 8);
+    PushSet<T> K{};
+    K.fx_scale = fixed_scale(g, S);
+    K.parts = parts;
+    K.dt = T(g.dt);
+    K.idt = T(1.0 / g.dt);
+    const double d[3] = {g.dx, g.dy, g.dz}, id[3] = {g.idx, g.idy, g.idz};
+    for (int a = 0; a < 3; ++a) {
+        K.d[a] = T(d[a]);
+        K.id[a] = T(id[a]);
+        K.hid[a] = T(0.5) * K.id[a];
+    }
+    const T vol = K.d[0] * K.d[1] * K.d[2];
+    for (int q = 0; q < S.ns; ++q) {
+        K.q[q] = S.q[q];
+        K.m[q] = S.m[q];
+        K.beta[q] = S.q[q] * K.dt / (T(2) * S.m[q]);
+        K.fcd[q] = S.q[q] * S.w[q] / vol;
+    }
     // a wall box runs its own instantiation (run-time tile shape)
-    auto* whole = g.wall ? k_push_deposit_tile<T, T, 0, true, false>
-                         : cube8 ? k_push_deposit_tile<T, T, 8, false, false> : k_push_deposit_tile<T, T, 0, false, false>;
-    auto* shared = g.wall ? k_push_deposit_tile<T, T, 0, true, true>
-                          : cube8 ? k_push_deposit_tile<T, T, 8, false, true> : k_push_deposit_tile<T, T, 0, false, true>;
-    auto* kernel = parts > 1 ? shared : whole;
-    kernel<<<grid, kTileThreads, smem, s>>>(g, t, sh, S, (const T*)E, (const T*)B, Jpart, fx_scale, inv_dt, parts);
+    auto* whole = g.wall ? k_push_deposit_tile<T, T, 0, true, false, false>
+                         : cube8 ? k_push_deposit_tile<T, T, 8, false, false, false>
+                                 : k_push_deposit_tile<T, T, 0, false, false, false>;
+    auto* shared = g.wall ? k_push_deposit_tile<T, T, 0, true, true, false>
+                          : cube8 ? k_push_deposit_tile<T, T, 8, false, true, false>
+                                  : k_push_deposit_tile<T, T, 0, false, true, false>;
+    auto* kernel = merge ? k_push_deposit_tile<T, T, 8, false, true, true> : (parts > 1 ? shared : whole);
+    kernel<<<grid, kTileThreads, tile_smem_bytes(sh, merge), s>>>(g, t, o, sh, S, K, (const T*)E, (const T*)B, Jpart);
     // the particles it left over: one thread per mask word
     long long words = 1;
     for (int q = 0; q < S.ns; ++q) words = std::max(words, (S.p[q].n + 31) / 32 + 1);
