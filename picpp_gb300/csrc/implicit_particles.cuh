@@ -259,7 +259,7 @@ __device__ __forceinline__ void implicit_move_particle(const GridP& g, const Par
             wall_reflect_trial<T>(g, ci, u0, mv, vnew, mm, edt, redt, id, pnew);
             p.px[n] = pnew[0]; p.py[n] = pnew[1]; p.pz[n] = pnew[2];
             p.ox[n] = u0[0]; p.oy[n] = u0[1]; p.oz[n] = u0[2];
-            p.cell[n] = (int)lin(g, ci[0], ci[1], ci[2]);
+            p.cell[n] = tristan_escaped<T>(g, ci[0], u0[0]) ? -1 : (int)lin(g, ci[0], ci[1], ci[2]);
             return;
         }
     }
@@ -327,7 +327,7 @@ __device__ __forceinline__ void implicit_move_particle(const GridP& g, const Par
     }
     p.px[n] = pnew[0]; p.py[n] = pnew[1]; p.pz[n] = pnew[2];
     p.ox[n] = u0[0]; p.oy[n] = u0[1]; p.oz[n] = u0[2];
-    p.cell[n] = (int)lin(g, ci[0], ci[1], ci[2]);
+    p.cell[n] = kWall && tristan_escaped<T>(g, ci[0], u0[0]) ? -1 : (int)lin(g, ci[0], ci[1], ci[2]);
 }
 
 // The mover over every particle of one species (periodic or wall box).

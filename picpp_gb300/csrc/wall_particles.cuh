@@ -107,7 +107,9 @@ __device__ __forceinline__ int tristan_wall_x(const GridP& g, int& c, T& u, T di
 }
 
 // True for a particle that left a wall box through the open boundary: its
-// position lies beyond x = (nx - 2) dx (the ghost column).
+// position lies beyond x = (nx - 2) dx (the ghost column).  A mirrored
+// position too may lie there, whole boxes away, when a run that blew up moves
+// a particle that far (the implicit movers' trial velocity is not below c).
 template <typename T>
 __device__ __forceinline__ bool tristan_escaped(const GridP& g, int i, T u) {
     return i > g.nx - 2 || (i == g.nx - 2 && u > T(0));
