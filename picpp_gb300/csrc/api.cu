@@ -362,32 +362,39 @@ pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
 }
 
 // -------------------------------------------------------------- implicit
-// Sub-tiles of the staged deposit: tiles are cut (z first, then y, then x, by
-// the smallest prime factor, so that a sub-tile's keys stay consecutive)
-// until there is one sub-tile per SM and two fit into an SM's shared memory.
-// More cuts do not help: the pairs plane of 32x32x1 (16 tiles, FP64) deposited
-// in 1.73 ms per step uncut, 0.34 ms cut to 256 sub-tiles, 0.5 ms at 1024 (each
-// sub-tile flushes a block of its own).
+// Boxes of cells of the staged deposit: at most 8 per axis, as even as the
+// axis allows (9 cells as 5 + 4), the longest side halved until two boxes fit
+// into an SM's shared memory, every SM has one, and the last round of boxes
+// over the SMs leaves at most a fifth of the time idle.  Boxes of 32 cells (FP64,
+// whose particles take longer: 4) are not cut for that: each flushes a block of
+// its own (the pairs plane of 32x32x1, FP64: 1.73 ms in 16 boxes, 0.20 ms in
+// 256, 0.3 ms in 1024).  They do not follow the sort's tiles, which are single
+// cells along an odd axis: FP32 beams of 39x57x53, 60 per species and cell,
+// deposit in 0.98 ms, tile by tile in 5.03 ms; 112x51x5 shock 0.18 against
+// 0.24 ms (0.29 ms with 182 boxes, uncut); pairs of 61x43x1 0.70 against 1.31 ms.
 template <typename T>
-TileGeom split_tiles(const GridP& g, const TileGeom& t, TileSplit& sp) {
-    TileGeom w = t;
-    int* ext[3] = {&w.tz, &w.ty, &w.tx};
-    int* cnt[3] = {&w.ntz, &w.nty, &w.ntx};
-    int* cut[3] = {&sp.sz, &sp.sy, &sp.sx};
-    auto fits = [&]() {
+TileGeom deposit_boxes(const GridP& g, int ns) {
+    const int n[3] = {g.nx, g.ny, g.nz};
+    int m[3], e[3];
+    auto even = [&](int a, int most) {
+        m[a] = (n[a] + most - 1) / most;
+        e[a] = (n[a] + m[a] - 1) / m[a];
+        m[a] = (n[a] + e[a] - 1) / e[a];
+    };
+    for (int a = 0; a < 3; ++a) even(a, 8);
+    for (;;) {
+        TileGeom w{e[0], e[1], e[2], m[0], m[1], m[2], -1, -1, -1};
         ImpBlock bk = PK<T>::implicit_block(g, w, 0);
         bk.stage = 1;
-        return PK<T>::implicit_tile_smem(bk, w.tx * w.ty * w.tz) <= (size_t)(227 * 1024) / 2 - 1024;
-    };
-    for (int a = 0; a < 3; ++a)
-        while (*ext[a] > 1 && (w.ntx * w.nty * w.ntz < kNumSM || !fits())) {
-            int f = 2;
-            while (*ext[a] % f) ++f;
-            *ext[a] /= f;
-            *cnt[a] *= f;
-            *cut[a] *= f;
-        }
-    return w;
+        const bool fits = PK<T>::implicit_tile_smem(bk, e[0] * e[1] * e[2], ns) <= (size_t)(227 * 1024) / 2 - 1024;
+        int a = 2;
+        for (int b = 1; b >= 0; --b)
+            if (e[b] > e[a]) a = b;
+        const double waves = (double)m[0] * m[1] * m[2] / kNumSM;
+        const bool enough = waves >= 1 && (waves / std::ceil(waves) >= 0.8 || e[0] * e[1] * e[2] <= (sizeof(T) == 4 ? 32 : 4));
+        if ((fits && enough) || e[a] == 1) return w;
+        even(a, (e[a] + 1) / 2);
+    }
 }
 
 template <typename T>
@@ -406,18 +413,17 @@ pic_status implicit_moments(pic_ctx* ctx) {
     // the block fits in shared memory
     // right after a sort every particle is in its tile: no halo, and E, B
     // staged next to the accumulators; otherwise a one-cell halo for drift
-    // (staged: over sub-tiles, split_tiles)
-    TileSplit sp{1, 1, 1};
-    TileGeom wt = split_tiles<T>(g, ctx->tg, sp);
+    // (staged: over boxes of cells, deposit_boxes)
+    const int ns = (int)ctx->sp.size();
+    TileGeom wt = deposit_boxes<T>(g, ns);
     ImpBlock bk = PK<T>::implicit_block(g, wt, 0);
     bk.stage = 1;
-    if (!ctx->fresh_sort || PK<T>::implicit_tile_smem(bk, wt.tx * wt.ty * wt.tz) > 227 * 1024) {
+    if (!ctx->fresh_sort || PK<T>::implicit_tile_smem(bk, wt.tx * wt.ty * wt.tz, ns) > 227 * 1024) {
         wt = ctx->tg;
-        sp = TileSplit{1, 1, 1};
         bk = PK<T>::implicit_block(g, ctx->tg, 1);
-        if (PK<T>::implicit_tile_smem(bk, ctx->T3) > 227 * 1024) bk = PK<T>::implicit_block(g, ctx->tg, 0);
+        if (PK<T>::implicit_tile_smem(bk, ctx->T3, ns) > 227 * 1024) bk = PK<T>::implicit_block(g, ctx->tg, 0);
     }
-    if (!compat && all_sorted(ctx) && PK<T>::implicit_tile_smem(bk, wt.tx * wt.ty * wt.tz) <= 227 * 1024) {
+    if (!compat && all_sorted(ctx) && PK<T>::implicit_tile_smem(bk, wt.tx * wt.ty * wt.tz, ns) <= 227 * 1024) {
         ImpSpecies<T> S{};
         S.ns = (int)ctx->sp.size();
         for (int q = 0; q < S.ns; ++q) {
@@ -435,7 +441,7 @@ pic_status implicit_moments(pic_ctx* ctx) {
             Bf = (const T*)(ctx->fields32 + 3 * N);
         }
         Phase dep(ctx, PIC_PHASE_DEPOSIT, 0);
-        PK<T>::implicit_deposit_tiled(s, g, wt, sp, bk, S, Ef, Bf, ctx->Jh, ctx->mu, ctx->rho, ctx->Pi);
+        PK<T>::implicit_deposit_tiled(s, g, wt, ctx->tg, bk, S, Ef, Bf, ctx->Jh, ctx->mu, ctx->rho, ctx->Pi);
     } else {
         Phase dep(ctx, PIC_PHASE_DEPOSIT, 0);
         for (auto& sp : ctx->sp)

@@ -440,11 +440,12 @@ struct DepositSet {
 // 16-byte load per corner), the keys' offsets too, and each warp copies its
 // next chunk of particles with cp.async while it works on the current one.
 // What bounds it is instruction issue at 16 warps per SM (two CTAs: the run
-// sums' accumulators take 128 registers); tiles are cut so that two fit
-// (split_tiles, api.cu).
-// kSplit: t is the geometry of sub-tiles, cut from the sort's tiles by sp.
-template <typename T, typename A, bool kStaged, bool kSplit>
-__global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(GridP g, TileGeom t, TileSplit sp, ImpBlock bk,
+// sums' accumulators take 128 registers).  t holds boxes of cells then, of
+// which two fit on an SM (deposit_boxes, api.cu), ragged at the grid's ends;
+// they need not follow the sort's tiles o, a cell's particles being found by
+// its key.  Not staged: t holds the sort's tiles.
+template <typename T, typename A, bool kStaged>
+__global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(GridP g, TileGeom t, TileGeom o, ImpBlock bk,
                                                                        ImpSpecies<T> S,
                                                                        const __grid_constant__ DepositSet<T> K,
                                                                        const T* __restrict__ E,
@@ -477,21 +478,17 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
     float* scr = scr0 + warp * (kScrParticles * kScrRow);
     // the lane table of tc_run_sums follows the scratch rows of all warps
     TcLane* s_lane = reinterpret_cast<TcLane*>(scr0 + nwarps * (kScrParticles * kScrRow));
-    // staged: every warp's next chunk, then the keys' offsets of all species
+    // staged: every warp's next chunk, then first particle and end of the
+    // box's cells, of all species
     ChunkBuf<T>* buf = reinterpret_cast<ChunkBuf<T>*>(kTc ? reinterpret_cast<unsigned char*>(s_lane + 32) : after) + warp;
-    int* sOff = reinterpret_cast<int*>(buf - warp + nwarps);
+    int2* sOff = reinterpret_cast<int2*>(buf - warp + nwarps);
     if (kTc && threadIdx.x < 32) s_lane[threadIdx.x] = tc_lane(threadIdx.x);
 
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int ti = tile % t.ntx, tj = (tile / t.ntx) % t.nty, tk = tile / (t.ntx * t.nty);
         const int x0 = ti * t.tx, y0 = tj * t.ty, z0 = tk * t.tz;
-        // first key of the sub-tile: its tile's, plus its place in it
-        const int key0 = kSplit ? ((((tk / sp.sz) * (t.nty / sp.sy) + tj / sp.sy) * (t.ntx / sp.sx) + ti / sp.sx) *
-                                       (sp.sx * sp.sy * sp.sz) +
-                                   ((tk % sp.sz) * sp.sy + tj % sp.sy) * sp.sx + ti % sp.sx) * T3
-                                : tile * T3;
         for (int e = threadIdx.x; e < tot; e += blockDim.x) sN[e] = A(0);
-        if (kStaged) {   // with h = 0 the blocks cover exactly the stencils of the tile's own cells
+        if (kStaged) {   // with h = 0 the blocks cover exactly the stencils of the box's own cells
             for (int e = threadIdx.x; e < bk.NB; e += blockDim.x) {
                 const int lx = e % bk.nbx, ly = (e / bk.nbx) % bk.nby, lz = e / (bk.nbx * bk.nby);
                 const long long id = linw(g, x0 + lx, y0 + ly, z0 + lz);
@@ -512,8 +509,13 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
                     for (int c = 0; c < 3; ++c) sB[c * bk.CB + e] = B[c * g.N + id];
                 }
             }
-            for (int s = 0; s < S.ns; ++s)
-                for (int e = threadIdx.x; e <= T3; e += blockDim.x) sOff[s * (T3 + 1) + e] = S.off[s][key0 + e];
+            for (int e = threadIdx.x; e < T3; e += blockDim.x) {
+                const int i = x0 + e % t.tx, j = y0 + (e / t.tx) % t.ty, k = z0 + e / (t.tx * t.ty);
+                const bool in = i < g.nx && j < g.ny && k < g.nz;
+                const int kk = in ? cell_key(o, i, j, k) : 0;
+                for (int s = 0; s < S.ns; ++s)
+                    sOff[s * T3 + e] = in ? make_int2(S.off[s][kk], S.off[s][kk + 1]) : make_int2(0, 0);
+            }
         }
         __syncthreads();
         for (int s = 0; s < S.ns; ++s) {
@@ -521,15 +523,15 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
             const double cq = K.cq[s], cm = K.cm[s];
             const T beta = K.beta[s], ms = K.m[s];
             if constexpr (kStaged) {
-                const int* __restrict__ of = sOff + s * (T3 + 1);
-                // the warp's chunks: keys warp, warp + nwarps, ... of the tile
+                const int2* __restrict__ of = sOff + s * T3;
+                // the warp's chunks: cells warp, warp + nwarps, ... of the box
                 // (empty ones skipped), each 32 particles at a time
                 auto next_key = [&](int lc) {
-                    while (lc < T3 && of[lc] == of[lc + 1]) lc += nwarps;
+                    while (lc < T3 && of[lc].x == of[lc].y) lc += nwarps;
                     return lc;
                 };
-                int lc = next_key(warp), c0 = lc < T3 ? of[lc] : 0;
-                if (lc < T3 && c0 + lane < of[lc + 1]) stage_particle(buf, p, c0 + lane, lane);
+                int lc = next_key(warp), c0 = lc < T3 ? of[lc].x : 0;
+                if (lc < T3 && c0 + lane < of[lc].y) stage_particle(buf, p, c0 + lane, lane);
                 cp_async_commit();
                 int key = -1, cellK = 0, nbK = 0, cbK = 0;
                 float an[4] = {0.f, 0.f, 0.f, 0.f}, ac[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -541,17 +543,17 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
                         cbK = lk * csz + lj * csy + li;
                         cellK = (int)lin(g, x0 + li, y0 + lj, z0 + lk);
                     }
-                    const bool valid = c0 + lane < of[lc + 1];
+                    const bool valid = c0 + lane < of[lc].y;
                     cp_async_wait_all();   // a lane's own slots
                     const int cell = buf->cell[lane];
                     const T ox = buf->a[0][lane], oy = buf->a[1][lane], oz = buf->a[2][lane];
                     const T mom[3] = {buf->a[3][lane], buf->a[4][lane], buf->a[5][lane]};
                     int nlc = lc, nc0 = c0 + 32;
-                    if (nc0 >= of[lc + 1]) {
+                    if (nc0 >= of[lc].y) {
                         nlc = next_key(lc + nwarps);
-                        nc0 = nlc < T3 ? of[nlc] : 0;
+                        nc0 = nlc < T3 ? of[nlc].x : 0;
                     }
-                    if (nlc < T3 && nc0 + lane < of[nlc + 1]) stage_particle(buf, p, nc0 + lane, lane);
+                    if (nlc < T3 && nc0 + lane < of[nlc].y) stage_particle(buf, p, nc0 + lane, lane);
                     cp_async_commit();
                     // raw quantities: rv (3), alpha (9), node weights x/y/z (2 each), cell weights x/y/z (3 each)
                     T row[kScrRow];
@@ -619,7 +621,7 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
             }
             const int* __restrict__ off = S.off[s];
             for (int lc = warp; lc < T3; lc += nwarps) {
-                const int kk = key0 + lc;
+                const int kk = tile * T3 + lc;
                 const int b0 = off[kk], b1 = off[kk + 1];
                 for (int c0 = b0; c0 < b1; c0 += 32) {
                     const int n = c0 + lane;

@@ -75,8 +75,8 @@ struct PK {
     // tiled deposit (implicit_tile.cuh), periodic pressure placement; needs
     // tile-major sorted particles
     static ImpBlock implicit_block(const GridP& g, const TileGeom& t, int h);
-    static size_t implicit_tile_smem(const ImpBlock& bk, int keys);   // keys per (sub-)tile
-    static void implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileSplit& sp,
+    static size_t implicit_tile_smem(const ImpBlock& bk, int cells, int ns);   // cells per tile or box, species
+    static void implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileGeom& o,
                                        const ImpBlock& bk,
                                        const ImpSpecies<T>& S, const T* E, const T* B, double* J,
                                        double* mu, double* rho, double* Pi);

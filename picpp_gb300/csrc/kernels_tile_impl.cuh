@@ -109,36 +109,33 @@ ImpBlock PK<T>::implicit_block(const GridP& g, const TileGeom& t, int h) {
 }
 
 template <typename T>
-size_t PK<T>::implicit_tile_smem(const ImpBlock& bk, int keys) {
+size_t PK<T>::implicit_tile_smem(const ImpBlock& bk, int cells, int ns) {
     // FP32 accumulators: the per-warp rows of the tensor-core run sums and
     // their 32-entry lane table; staged: every warp's next chunk of particles
-    // and the offsets of the sub-tile's keys for all species
+    // and the particle ranges of the box's cells, of every species
     size_t n = bk.scratch_at();
     if (sizeof(T) == sizeof(float))
         n += (size_t)(imp_threads<T>() / 32) * kScrParticles * kScrRow * sizeof(float) + 32 * sizeof(TcLane);
-    if (bk.stage) n += (size_t)(imp_threads<T>() / 32) * sizeof(ChunkBuf<T>) + (size_t)kMaxSpecies * (keys + 1) * sizeof(int);
+    if (bk.stage) n += (size_t)(imp_threads<T>() / 32) * sizeof(ChunkBuf<T>) + (size_t)ns * cells * sizeof(int2);
     return n;
 }
 
 template <typename T>
-void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileSplit& sp, const ImpBlock& bk,
+void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileGeom& o, const ImpBlock& bk,
                                    const ImpSpecies<T>& S, const T* E, const T* B, double* J, double* mu,
                                    double* rho, double* Pi) {
     static bool attr_set = false;
     if (!attr_set) {
-        for (auto* k : {k_implicit_deposit_tile<T, T, true, false>, k_implicit_deposit_tile<T, T, true, true>,
-                        k_implicit_deposit_tile<T, T, false, false>})
+        for (auto* k : {k_implicit_deposit_tile<T, T, true>, k_implicit_deposit_tile<T, T, false>})
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         attr_set = true;
     }
-    const size_t smem = implicit_tile_smem(bk, t.tx * t.ty * t.tz);
+    const size_t smem = implicit_tile_smem(bk, t.tx * t.ty * t.tz, S.ns);
     const int per_sm = (int)((227 * 1024) / (smem + 1024));
     const int ntiles = t.ntx * t.nty * t.ntz;
     const int grid = ntiles < kNumSM * (per_sm > 0 ? per_sm : 1) ? ntiles : kNumSM * (per_sm > 0 ? per_sm : 1);
     constexpr int nt = imp_threads<T>();
-    const bool split = sp.sx * sp.sy * sp.sz > 1;
-    auto* kernel = !bk.stage ? k_implicit_deposit_tile<T, T, false, false>
-                   : split ? k_implicit_deposit_tile<T, T, true, true> : k_implicit_deposit_tile<T, T, true, false>;
+    auto* kernel = bk.stage ? k_implicit_deposit_tile<T, T, true> : k_implicit_deposit_tile<T, T, false>;
     const double PI_D = 3.14159265358979323846;
     const double ivol = 1.0 / (g.dx * g.dy * g.dz);
     DepositSet<T> K{};
@@ -148,7 +145,7 @@ void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeo
         K.cq[q] = S.q[q] * S.w[q] * ivol;
         K.cm[q] = -(S.w[q] * g.theta * g.dt * g.dt * 2 * PI_D * S.q[q] * S.q[q] / S.m[q]) * ivol;
     }
-    kernel<<<grid, nt, smem, s>>>(g, t, sp, bk, S, K, E, B, J, mu, rho, Pi);
+    kernel<<<grid, nt, smem, s>>>(g, t, o, bk, S, K, E, B, J, mu, rho, Pi);
 }
 
 template <typename T>

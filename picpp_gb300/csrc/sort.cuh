@@ -22,16 +22,7 @@ namespace pic {
 __device__ __forceinline__ int sort_key(const GridP& g, const TileGeom& t, int cell) {
     int i, j, k;
     decode(g, cell, i, j, k);
-    int ti, tj, tk;
-    if (t.lx >= 0) {   // power-of-two tiles (the default): shifts, not divisions
-        ti = i >> t.lx; tj = j >> t.ly; tk = k >> t.lz;
-    } else {
-        ti = i / t.tx; tj = j / t.ty; tk = k / t.tz;
-    }
-    int li = i - ti * t.tx, lj = j - tj * t.ty, lk = k - tk * t.tz;
-    int tile = (tk * t.nty + tj) * t.ntx + ti;
-    int local = (lk * t.ty + lj) * t.tx + li;
-    return tile * (t.tx * t.ty * t.tz) + local;
+    return cell_key(t, i, j, k);
 }
 
 // Runs of equal keys within a warp: the head lane of each run and the run's

@@ -21,12 +21,19 @@ struct TileGeom {
     int lx, ly, lz;      // log2 of the extents when all three are powers of two, else -1
 };
 
-// Sub-tiles of the staged implicit deposit: each tile of the sort key cut into
-// sx, sy, sz pieces per axis whose cells are consecutive keys (y is cut only
-// when z is cut down to single layers, x only when y is).
-struct TileSplit {
-    int sx, sy, sz;
-};
+// Sort key of cell (i, j, k): tile by tile, x fastest in a tile.
+__device__ __forceinline__ int cell_key(const TileGeom& t, int i, int j, int k) {
+    int ti, tj, tk;
+    if (t.lx >= 0) {   // power-of-two tiles (the default): shifts, not divisions
+        ti = i >> t.lx; tj = j >> t.ly; tk = k >> t.lz;
+    } else {
+        ti = i / t.tx; tj = j / t.ty; tk = k / t.tz;
+    }
+    const int li = i - ti * t.tx, lj = j - tj * t.ty, lk = k - tk * t.tz;
+    const int tile = (tk * t.nty + tj) * t.ntx + ti;
+    const int local = (lk * t.ty + lj) * t.tx + li;
+    return tile * (t.tx * t.ty * t.tz) + local;
+}
 
 // Shared-memory blocks of the fused explicit kernel (boris_tile.cuh).
 struct TileShape {
