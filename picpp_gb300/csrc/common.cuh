@@ -59,6 +59,13 @@ __host__ __device__ __forceinline__ long long linw(const GridP& g, int i, int j,
     k = k < 0 ? k + g.nz : (k >= g.nz ? k - g.nz : k);
     return ((long long)k * g.ny + j) * g.nx + i;
 }
+// The same for halos wider than an axis (three cells around two): any offset.
+__host__ __device__ __forceinline__ long long linw_any(const GridP& g, int i, int j, int k) {
+    if (i < -g.nx || i >= 2 * g.nx) i = wrap_any(i, g.nx);
+    if (j < -g.ny || j >= 2 * g.ny) j = wrap_any(j, g.ny);
+    if (k < -g.nz || k >= 2 * g.nz) k = wrap_any(k, g.nz);
+    return linw(g, i, j, k);
+}
 __host__ __device__ __forceinline__ void decode(const GridP& g, int cell, int& i, int& j, int& k) {
 #ifdef __CUDA_ARCH__
     int q = fast_div(cell, g.divx);

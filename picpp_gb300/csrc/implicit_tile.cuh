@@ -808,7 +808,7 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
         __syncthreads();   // previous tile's particles are done with the blocks
         for (int e = threadIdx.x; e < mb.NB; e += blockDim.x) {
             const int lx = e % mb.nbx, ly = (e / mb.nbx) % mb.nby, lz = e / (mb.nbx * mb.nby);
-            const long long gid = linw(g, x0 - hx + lx, y0 - hy + ly, z0 - hz + lz);
+            const long long gid = linw_any(g, x0 - hx + lx, y0 - hy + ly, z0 - hz + lz);
 #pragma unroll
             for (int c = 0; c < 3; ++c) sE[c * mb.NB + e] = T(E[c * g.N + gid]);
             if constexpr (kVec) {
@@ -820,8 +820,8 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
         }
         for (int e = threadIdx.x; e < mb.CB; e += blockDim.x) {
             const int lx = e % mb.cbx, ly = (e / mb.cbx) % mb.cby, lz = e / (mb.cbx * mb.cby);
-            const long long gid = linw(g, x0 - hx - (ax ? 1 : 0) + lx, y0 - hy - (ay ? 1 : 0) + ly,
-                                       z0 - hz - (az ? 1 : 0) + lz);
+            const long long gid = linw_any(g, x0 - hx - (ax ? 1 : 0) + lx, y0 - hy - (ay ? 1 : 0) + ly,
+                                           z0 - hz - (az ? 1 : 0) + lz);
             if constexpr (kVec) {
                 sB4[e] = make_float4(float(B[gid]), float(B[g.N + gid]), float(B[2 * g.N + gid]), 0.f);
             } else {
