@@ -52,6 +52,7 @@ struct pic_ctx {
     TileShape ts{};
     TileGeom wg{};          // work tiles of the fused explicit kernel (merge_geom) and their shape
     TileShape ws{};
+    TileGeom mg{};          // work boxes of the implicit mover (mover_boxes)
     GhostAxes ga{};
     int nkeys = 0, ntiles = 0, T3 = 0;
     int preal = 0;
@@ -296,6 +297,21 @@ void merge_geom(const pic_config& c, const TileGeom& t, TileGeom& w, TileShape& 
     ws.jcells = 12 * 12 * 12;
 }
 
+// Work boxes of the implicit mover: as even as the axes allow, up to 8 cells per
+// axis in whole tiles of the sort, where the caller left the tiles to the
+// library (k_implicit_push_tile has both sides' times).
+TileGeom mover_boxes(const pic_config& c, const TileGeom& t) {
+    const int n[3] = {c.nx, c.ny, c.nz}, tile[3] = {t.tx, t.ty, t.tz};
+    int m[3], e[3];
+    for (int a = 0; a < 3; ++a) {
+        if (c.tile[a] > 0) return t;
+        m[a] = (n[a] + 7) / 8;
+        const int tiles = n[a] / tile[a];
+        e[a] = (tiles + m[a] - 1) / m[a] * tile[a];
+    }
+    return TileGeom{e[0], e[1], e[2], m[0], m[1], m[2], -1, -1, -1};
+}
+
 template <typename T>
 pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
     cudaStream_t s = ctx->s;
@@ -367,8 +383,8 @@ pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
 // into an SM's shared memory, every SM has one, and the last round of boxes
 // over the SMs leaves at most a fifth of the time idle.  Boxes of 32 cells (FP64,
 // whose particles take longer: 4) are not cut for that: each flushes a block of
-// its own (the pairs plane of 32x32x1, FP64: 1.73 ms in 16 boxes, 0.20 ms in
-// 256, 0.3 ms in 1024).  They do not follow the sort's tiles, which are single
+// its own (the pairs plane of 32x32x1, FP64: 1.73 ms in 16 boxes, 0.34 ms in
+// 256, where it is 0.20 ms by now, 0.5 ms in 1024).  They do not follow the sort's tiles, which are single
 // cells along an odd axis: FP32 beams of 39x57x53, 60 per species and cell,
 // deposit in 0.98 ms, tile by tile in 5.03 ms; 112x51x5 shock 0.18 against
 // 0.24 ms (0.29 ms with 182 boxes, uncut); pairs of 61x43x1 0.70 against 1.31 ms.
@@ -379,7 +395,6 @@ TileGeom deposit_boxes(const GridP& g, int ns) {
     auto even = [&](int a, int most) {
         m[a] = (n[a] + most - 1) / most;
         e[a] = (n[a] + m[a] - 1) / m[a];
-        m[a] = (n[a] + e[a] - 1) / e[a];
     };
     for (int a = 0; a < 3; ++a) even(a, 8);
     for (;;) {
@@ -486,7 +501,7 @@ pic_status implicit_move(pic_ctx* ctx) {
             S.off[q] = ctx->sp[q].off;
             S.defer[q] = ctx->sp[q].defer;
         }
-        tiled = PK<T>::implicit_push_tiled(ctx->s, ctx->g, ctx->tg, S, ctx->Ei, ctx->Bi, ctx->Et);
+        tiled = PK<T>::implicit_push_tiled(ctx->s, ctx->g, ctx->mg, ctx->tg, S, ctx->Ei, ctx->Bi, ctx->Et);
     }
     if (!tiled)
         for (auto& sp : ctx->sp)
@@ -612,6 +627,7 @@ pic_status pic_create(const pic_config* cfg, pic_ctx** out) {
     ctx->wg = t;
     ctx->ws = ts;
     merge_geom(c, t, ctx->wg, ctx->ws);
+    ctx->mg = mover_boxes(c, t);
     GhostAxes& ga = ctx->ga;
     ga.cex = c.nx > 1 ? c.nx + 4 : 1; ga.cey = c.ny > 1 ? c.ny + 4 : 1; ga.cez = c.nz > 1 ? c.nz + 4 : 1;
     ga.gx = c.nx > 1 ? 2 : 0; ga.gy = c.ny > 1 ? 2 : 0; ga.gz = c.nz > 1 ? 2 : 0;

@@ -441,12 +441,12 @@ struct DepositSet {
 // next chunk of particles with cp.async while it works on the current one.
 // What bounds it is instruction issue at 16 warps per SM (two CTAs: the run
 // sums' accumulators take 128 registers).  t holds boxes of cells then, of
-// which two fit on an SM (deposit_boxes, api.cu), ragged at the grid's ends;
-// they need not follow the sort's tiles o, a cell's particles being found by
+// which two fit on an SM (deposit_boxes, api.cu), some a cell smaller than
+// others (box_start); they need not follow the sort's tiles o, a cell's particles being found by
 // its key.  Not staged: t holds the sort's tiles.
 template <typename T, typename A, bool kStaged>
 __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(GridP g, TileGeom t, TileGeom o, ImpBlock bk,
-                                                                       ImpSpecies<T> S,
+                                                                       const __grid_constant__ ImpSpecies<T> S,
                                                                        const __grid_constant__ DepositSet<T> K,
                                                                        const T* __restrict__ E,
                                                                        const T* __restrict__ B,
@@ -486,8 +486,9 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
 
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int ti = tile % t.ntx, tj = (tile / t.ntx) % t.nty, tk = tile / (t.ntx * t.nty);
-        const int x0 = ti * t.tx, y0 = tj * t.ty, z0 = tk * t.tz;
+        const int x0 = box_start(g.nx, ti, t.ntx), y0 = box_start(g.ny, tj, t.nty), z0 = box_start(g.nz, tk, t.ntz);
         for (int e = threadIdx.x; e < tot; e += blockDim.x) sN[e] = A(0);
+        const int x1 = box_start(g.nx, ti + 1, t.ntx), y1 = box_start(g.ny, tj + 1, t.nty), z1 = box_start(g.nz, tk + 1, t.ntz);
         if (kStaged) {   // with h = 0 the blocks cover exactly the stencils of the box's own cells
             for (int e = threadIdx.x; e < bk.NB; e += blockDim.x) {
                 const int lx = e % bk.nbx, ly = (e / bk.nbx) % bk.nby, lz = e / (bk.nbx * bk.nby);
@@ -511,180 +512,185 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
             }
             for (int e = threadIdx.x; e < T3; e += blockDim.x) {
                 const int i = x0 + e % t.tx, j = y0 + (e / t.tx) % t.ty, k = z0 + e / (t.tx * t.ty);
-                const bool in = i < g.nx && j < g.ny && k < g.nz;
+                const bool in = i < x1 && j < y1 && k < z1;
                 const int kk = in ? cell_key(o, i, j, k) : 0;
                 for (int s = 0; s < S.ns; ++s)
                     sOff[s * T3 + e] = in ? make_int2(S.off[s][kk], S.off[s][kk + 1]) : make_int2(0, 0);
             }
         }
         __syncthreads();
-        for (int s = 0; s < S.ns; ++s) {
-            const PartView<T> p = S.p[s];
-            const double cq = K.cq[s], cm = K.cm[s];
-            const T beta = K.beta[s], ms = K.m[s];
-            if constexpr (kStaged) {
-                const int2* __restrict__ of = sOff + s * T3;
-                // the warp's chunks: cells warp, warp + nwarps, ... of the box
-                // (empty ones skipped), each 32 particles at a time
-                auto next_key = [&](int lc) {
-                    while (lc < T3 && of[lc].x == of[lc].y) lc += nwarps;
-                    return lc;
-                };
-                int lc = next_key(warp), c0 = lc < T3 ? of[lc].x : 0;
-                if (lc < T3 && c0 + lane < of[lc].y) stage_particle(buf, p, c0 + lane, lane);
-                cp_async_commit();
-                int key = -1, cellK = 0, nbK = 0, cbK = 0;
-                float an[4] = {0.f, 0.f, 0.f, 0.f}, ac[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                while (lc < T3) {
-                    if (lc != key) {
-                        key = lc;
-                        const int li = lc % t.tx, q = lc / t.tx, lj = q % t.ty, lk = q / t.ty;
-                        nbK = lk * nsz + lj * nsy + li;
-                        cbK = lk * csz + lj * csy + li;
-                        cellK = (int)lin(g, x0 + li, y0 + lj, z0 + lk);
-                    }
-                    const bool valid = c0 + lane < of[lc].y;
-                    cp_async_wait_all();   // a lane's own slots
-                    const int cell = buf->cell[lane];
-                    const T ox = buf->a[0][lane], oy = buf->a[1][lane], oz = buf->a[2][lane];
-                    const T mom[3] = {buf->a[3][lane], buf->a[4][lane], buf->a[5][lane]};
-                    int nlc = lc, nc0 = c0 + 32;
-                    if (nc0 >= of[lc].y) {
-                        nlc = next_key(lc + nwarps);
-                        nc0 = nlc < T3 ? of[nlc].x : 0;
-                    }
-                    if (nlc < T3 && nc0 + lane < of[nlc].y) stage_particle(buf, p, nc0 + lane, lane);
-                    cp_async_commit();
-                    // raw quantities: rv (3), alpha (9), node weights x/y/z (2 each), cell weights x/y/z (3 each)
-                    T row[kScrRow];
-                    const bool mine = valid && cell == cellK;   // (always, after a sort)
-                    if (valid) {
-                        T gam, v[3];
-                        gamma_vel<T>(mom, ms, gam, v);
-                        T* nw = row + 12;
-                        T* cw = row + 18;
-                        axis_weights<T>(ox, ax, nw, cw);
-                        axis_weights<T>(oy, ay, nw + 2, cw + 3);
-                        axis_weights<T>(oz, az, nw + 4, cw + 6);
-                        T e[3], bf[3];
-                        if (mine) {
-                            T w[8];
-                            corners<T>(nw[1], nw[3], nw[5], w);
-                            if constexpr (kVec) gather3(sE4, nbK, oxn, oyn, ozn, w, e);
-                            else gather3<T>(sE, bk.NB, nbK, oxn, oyn, ozn, w, e);
-                            // cell pair (c - 1, c) below the centre, (c, c + 1) above
-                            const bool bx = ox < T(0.5), by = oy < T(0.5), bz = oz < T(0.5);
-                            corners<T>(bx ? cw[1] : cw[2], by ? cw[4] : cw[5], bz ? cw[7] : cw[8], w);
-                            const int cbase = cbK + (bx ? 0 : oxc) + (by ? 0 : oyc) + (bz ? 0 : ozc);
-                            if constexpr (kVec) gather3(sB4, cbase, oxc, oyc, ozc, w, bf);
-                            else gather3<T>(sB, bk.CB, cbase, oxc, oyc, ozc, w, bf);
-                        } else {
-                            int i, j, k;
-                            decode(g, cell, i, j, k);
-                            const EB6<T> r = gather_eb_global<T>(g, i, j, k, ox, oy, oz, E, B);
-#pragma unroll
-                            for (int c = 0; c < 3; ++c) { e[c] = r.e[c]; bf[c] = r.b[c]; }
-                        }
-                        T al[9];
-                        alpha_tensor<T>(beta, v, gam, e, bf, al);
-                        const T vg[3] = {v[0] * gam, v[1] * gam, v[2] * gam};
-#pragma unroll
-                        for (int a = 0; a < 3; ++a) row[a] = al[3 * a] * vg[0] + al[3 * a + 1] * vg[1] + al[3 * a + 2] * vg[2];
-#pragma unroll
-                        for (int d = 0; d < 9; ++d) row[3 + d] = al[d];
-                        if (!mine) deposit_row_global<A, T>(g, cell, ox, oy, oz, row, cq, cm, J, mu, rho, Pi);
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < kScrRow; ++q) row[q] = T(0);
-                    }
-                    const unsigned mm = __ballot_sync(0xffffffffu, mine);
-                    if constexpr (kTc) {
-                        if (mm) tc_run_sums(scr, lane, mine, mm, row, an, ac, s_lane[lane]);
-                        if (nlc != lc) {   // the key's sums reach the block once
-                            add_run_sums(sN, sC, bk.NB, bk.CB, nbK, cbK, oxn, oyn, ozn, oxc, oyc, ozc, lane, an, ac, float(cq),
-                                         float(cm));
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) an[q] = 0.f;
-#pragma unroll
-                            for (int q = 0; q < 8; ++q) ac[q] = 0.f;
-                        }
-                    } else if (__popc(mm) >= kXposeMin) {
-                        butterfly_sums<A, T>(row, mine, cq, cm, sN, sC, bk.NB, bk.CB, nbK, cbK, oxn, oyn, ozn, oxc, oyc, ozc,
-                                             lane);
-                    } else if (mine) {
-                        imp_deposit_direct<A, T>(row, cq, cm, sN, sC, bk.NB, bk.CB, nbK, cbK, oxn, oyn, ozn, oxc, oyc, ozc);
-                    }
-                    lc = nlc;
-                    c0 = nc0;
+        if constexpr (kStaged) {
+            // the warp's chunks: keys warp, warp + nwarps, ... (a cell of one
+            // species: all cells of the first, then of the next; empty ones
+            // skipped), each 32 particles at a time
+            const int2* __restrict__ of = sOff;
+            const int keys = S.ns * T3;
+            auto next_key = [&](int lc) {
+                while (lc < keys && of[lc].x == of[lc].y) lc += nwarps;
+                return lc;
+            };
+            int lc = next_key(warp), c0 = lc < keys ? of[lc].x : 0;
+            if (lc < keys && c0 + lane < of[lc].y) stage_particle(buf, S.p[lc / T3], c0 + lane, lane);
+            cp_async_commit();
+            int key = -1, s = 0, cellK = 0, nbK = 0, cbK = 0;
+            float an[4] = {0.f, 0.f, 0.f, 0.f}, ac[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            while (lc < keys) {
+                if (lc != key) {
+                    key = lc;
+                    s = lc / T3;
+                    const int cell = lc - s * T3, li = cell % t.tx, q = cell / t.tx, lj = q % t.ty, lk = q / t.ty;
+                    nbK = lk * nsz + lj * nsy + li;
+                    cbK = lk * csz + lj * csy + li;
+                    cellK = (int)lin(g, x0 + li, y0 + lj, z0 + lk);
                 }
-                continue;
-            }
-            const int* __restrict__ off = S.off[s];
-            for (int lc = warp; lc < T3; lc += nwarps) {
-                const int kk = tile * T3 + lc;
-                const int b0 = off[kk], b1 = off[kk + 1];
-                for (int c0 = b0; c0 < b1; c0 += 32) {
-                    const int n = c0 + lane;
-                    const bool valid = n < b1;
-                    // raw quantities: rv (3), alpha (9), node weights x/y/z (2 each), cell weights x/y/z (3 each)
-                    T row[kScrRow];
-#pragma unroll
-                    for (int f = 0; f < kScrRow; ++f) row[f] = T(0);
-                    int cell = -1, nb = 0, cb = 0;
-                    bool inb = false;
-                    if (valid) {
-                        cell = p.cell[n];
+                const bool valid = c0 + lane < of[lc].y;
+                cp_async_wait_all();   // a lane's own slots
+                const int cell = buf->cell[lane];
+                const T ox = buf->a[0][lane], oy = buf->a[1][lane], oz = buf->a[2][lane];
+                const T mom[3] = {buf->a[3][lane], buf->a[4][lane], buf->a[5][lane]};
+                int nlc = lc, nc0 = c0 + 32;
+                if (nc0 >= of[lc].y) {
+                    nlc = next_key(lc + nwarps);
+                    nc0 = nlc < keys ? of[nlc].x : 0;
+                }
+                if (nlc < keys && nc0 + lane < of[nlc].y) stage_particle(buf, S.p[nlc / T3], nc0 + lane, lane);
+                cp_async_commit();
+                const double cq = K.cq[s], cm = K.cm[s];
+                const T beta = K.beta[s], ms = K.m[s];
+                // raw quantities: rv (3), alpha (9), node weights x/y/z (2 each), cell weights x/y/z (3 each)
+                T row[kScrRow];
+                const bool mine = valid && cell == cellK;   // (always, after a sort)
+                if (valid) {
+                    T gam, v[3];
+                    gamma_vel<T>(mom, ms, gam, v);
+                    T* nw = row + 12;
+                    T* cw = row + 18;
+                    axis_weights<T>(ox, ax, nw, cw);
+                    axis_weights<T>(oy, ay, nw + 2, cw + 3);
+                    axis_weights<T>(oz, az, nw + 4, cw + 6);
+                    T e[3], bf[3];
+                    if (mine) {
+                        T w[8];
+                        corners<T>(nw[1], nw[3], nw[5], w);
+                        if constexpr (kVec) gather3(sE4, nbK, oxn, oyn, ozn, w, e);
+                        else gather3<T>(sE, bk.NB, nbK, oxn, oyn, ozn, w, e);
+                        // cell pair (c - 1, c) below the centre, (c, c + 1) above
+                        const bool bx = ox < T(0.5), by = oy < T(0.5), bz = oz < T(0.5);
+                        corners<T>(bx ? cw[1] : cw[2], by ? cw[4] : cw[5], bz ? cw[7] : cw[8], w);
+                        const int cbase = cbK + (bx ? 0 : oxc) + (by ? 0 : oyc) + (bz ? 0 : ozc);
+                        if constexpr (kVec) gather3(sB4, cbase, oxc, oyc, ozc, w, bf);
+                        else gather3<T>(sB, bk.CB, cbase, oxc, oyc, ozc, w, bf);
+                    } else {
                         int i, j, k;
                         decode(g, cell, i, j, k);
-                        const T ox = p.ox[n], oy = p.oy[n], oz = p.oz[n];
-                        T mom[3] = {p.px[n], p.py[n], p.pz[n]};
-                        T gam, v[3];
-                        gamma_vel<T>(mom, ms, gam, v);
-                        T* nw = row + 12;
-                        T* cw = row + 18;
-                        axis_weights<T>(ox, ax, nw, cw);
-                        axis_weights<T>(oy, ay, nw + 2, cw + 3);
-                        axis_weights<T>(oz, az, nw + 4, cw + 6);
-                        int li = 0, lj = 0, lk = 0;
-                        inb = local_axis(i, x0, t.tx, hx, g.nx, li) && local_axis(j, y0, t.ty, hy, g.ny, lj) &&
-                              local_axis(k, z0, t.tz, hz, g.nz, lk);
-                        if (inb) {
-                            nb = (lk + hz) * nsz + (lj + hy) * nsy + (li + hx);
-                            cb = (lk + hz) * csz + (lj + hy) * csy + (li + hx);
-                        }
-                        T e[3], bf[3];
-                        gather_node<T, T>(g, i, j, k, ox, oy, oz, E, e);
-                        gather_cell<T, T>(g, i, j, k, ox, oy, oz, B, bf);
-                        T al[9];
-                        alpha_tensor<T>(beta, v, gam, e, bf, al);
-                        const T vg[3] = {v[0] * gam, v[1] * gam, v[2] * gam};
+                        const EB6<T> r = gather_eb_global<T>(g, i, j, k, ox, oy, oz, E, B);
 #pragma unroll
-                        for (int a = 0; a < 3; ++a) row[a] = al[3 * a] * vg[0] + al[3 * a + 1] * vg[1] + al[3 * a + 2] * vg[2];
-#pragma unroll
-                        for (int d = 0; d < 9; ++d) row[3 + d] = al[d];
-                        if (!inb) deposit_row_global<A, T>(g, cell, ox, oy, oz, row, cq, cm, J, mu, rho, Pi);
+                        for (int c = 0; c < 3; ++c) { e[c] = r.e[c]; bf[c] = r.b[c]; }
                     }
-                    unsigned pending = __ballot_sync(0xffffffffu, valid && inb);
-                    while (pending) {
-                        const int leader = __ffs(pending) - 1;
-                        const int lcell = __shfl_sync(0xffffffffu, cell, leader);
-                        const bool me = ((pending >> lane) & 1u) && cell == lcell;
-                        const unsigned mem = __ballot_sync(0xffffffffu, me);
-                        pending &= ~mem;
-                        if (__popc(mem) >= (kTc ? kTcMin : kXposeMin)) {
-                            const int nbL = __shfl_sync(0xffffffffu, nb, leader);
-                            const int cbL = __shfl_sync(0xffffffffu, cb, leader);
-                            if constexpr (kTc) {
-                                float dn[4] = {0.f, 0.f, 0.f, 0.f}, dc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                                tc_run_sums(scr, lane, me, mem, row, dn, dc, s_lane[lane]);
-                                add_run_sums(sN, sC, bk.NB, bk.CB, nbL, cbL, oxn, oyn, ozn, oxc, oyc, ozc, lane, dn, dc,
-                                             float(cq), float(cm));
-                            } else {
-                                butterfly_sums<A, T>(row, me, cq, cm, sN, sC, bk.NB, bk.CB, nbL, cbL, oxn, oyn, ozn, oxc, oyc, ozc,
-                                                     lane);
+                    T al[9];
+                    alpha_tensor<T>(beta, v, gam, e, bf, al);
+                    const T vg[3] = {v[0] * gam, v[1] * gam, v[2] * gam};
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) row[a] = al[3 * a] * vg[0] + al[3 * a + 1] * vg[1] + al[3 * a + 2] * vg[2];
+#pragma unroll
+                    for (int d = 0; d < 9; ++d) row[3 + d] = al[d];
+                    if (!mine) deposit_row_global<A, T>(g, cell, ox, oy, oz, row, cq, cm, J, mu, rho, Pi);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < kScrRow; ++q) row[q] = T(0);
+                }
+                const unsigned mm = __ballot_sync(0xffffffffu, mine);
+                if constexpr (kTc) {
+                    if (mm) tc_run_sums(scr, lane, mine, mm, row, an, ac, s_lane[lane]);
+                    if (nlc != lc) {   // the key's sums reach the block once
+                        add_run_sums(sN, sC, bk.NB, bk.CB, nbK, cbK, oxn, oyn, ozn, oxc, oyc, ozc, lane, an, ac, float(cq),
+                                     float(cm));
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) an[q] = 0.f;
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) ac[q] = 0.f;
+                    }
+                } else if (__popc(mm) >= kXposeMin) {
+                    butterfly_sums<A, T>(row, mine, cq, cm, sN, sC, bk.NB, bk.CB, nbK, cbK, oxn, oyn, ozn, oxc, oyc, ozc,
+                                         lane);
+                } else if (mine) {
+                    imp_deposit_direct<A, T>(row, cq, cm, sN, sC, bk.NB, bk.CB, nbK, cbK, oxn, oyn, ozn, oxc, oyc, ozc);
+                }
+                lc = nlc;
+                c0 = nc0;
+            }
+        } else {
+            for (int s = 0; s < S.ns; ++s) {
+                const PartView<T> p = S.p[s];
+                const double cq = K.cq[s], cm = K.cm[s];
+                const T beta = K.beta[s], ms = K.m[s];
+                const int* __restrict__ off = S.off[s];
+                for (int lc = warp; lc < T3; lc += nwarps) {
+                    const int kk = tile * T3 + lc;
+                    const int b0 = off[kk], b1 = off[kk + 1];
+                    for (int c0 = b0; c0 < b1; c0 += 32) {
+                        const int n = c0 + lane;
+                        const bool valid = n < b1;
+                        // raw quantities: rv (3), alpha (9), node weights x/y/z (2 each), cell weights x/y/z (3 each)
+                        T row[kScrRow];
+#pragma unroll
+                        for (int f = 0; f < kScrRow; ++f) row[f] = T(0);
+                        int cell = -1, nb = 0, cb = 0;
+                        bool inb = false;
+                        if (valid) {
+                            cell = p.cell[n];
+                            int i, j, k;
+                            decode(g, cell, i, j, k);
+                            const T ox = p.ox[n], oy = p.oy[n], oz = p.oz[n];
+                            T mom[3] = {p.px[n], p.py[n], p.pz[n]};
+                            T gam, v[3];
+                            gamma_vel<T>(mom, ms, gam, v);
+                            T* nw = row + 12;
+                            T* cw = row + 18;
+                            axis_weights<T>(ox, ax, nw, cw);
+                            axis_weights<T>(oy, ay, nw + 2, cw + 3);
+                            axis_weights<T>(oz, az, nw + 4, cw + 6);
+                            int li = 0, lj = 0, lk = 0;
+                            inb = local_axis(i, x0, t.tx, hx, g.nx, li) && local_axis(j, y0, t.ty, hy, g.ny, lj) &&
+                                  local_axis(k, z0, t.tz, hz, g.nz, lk);
+                            if (inb) {
+                                nb = (lk + hz) * nsz + (lj + hy) * nsy + (li + hx);
+                                cb = (lk + hz) * csz + (lj + hy) * csy + (li + hx);
                             }
-                        } else if (me) {
-                            imp_deposit_direct<A, T>(row, cq, cm, sN, sC, bk.NB, bk.CB, nb, cb, oxn, oyn, ozn, oxc, oyc, ozc);
+                            T e[3], bf[3];
+                            gather_node<T, T>(g, i, j, k, ox, oy, oz, E, e);
+                            gather_cell<T, T>(g, i, j, k, ox, oy, oz, B, bf);
+                            T al[9];
+                            alpha_tensor<T>(beta, v, gam, e, bf, al);
+                            const T vg[3] = {v[0] * gam, v[1] * gam, v[2] * gam};
+#pragma unroll
+                            for (int a = 0; a < 3; ++a) row[a] = al[3 * a] * vg[0] + al[3 * a + 1] * vg[1] + al[3 * a + 2] * vg[2];
+#pragma unroll
+                            for (int d = 0; d < 9; ++d) row[3 + d] = al[d];
+                            if (!inb) deposit_row_global<A, T>(g, cell, ox, oy, oz, row, cq, cm, J, mu, rho, Pi);
+                        }
+                        unsigned pending = __ballot_sync(0xffffffffu, valid && inb);
+                        while (pending) {
+                            const int leader = __ffs(pending) - 1;
+                            const int lcell = __shfl_sync(0xffffffffu, cell, leader);
+                            const bool me = ((pending >> lane) & 1u) && cell == lcell;
+                            const unsigned mem = __ballot_sync(0xffffffffu, me);
+                            pending &= ~mem;
+                            if (__popc(mem) >= (kTc ? kTcMin : kXposeMin)) {
+                                const int nbL = __shfl_sync(0xffffffffu, nb, leader);
+                                const int cbL = __shfl_sync(0xffffffffu, cb, leader);
+                                if constexpr (kTc) {
+                                    float dn[4] = {0.f, 0.f, 0.f, 0.f}, dc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                                    tc_run_sums(scr, lane, me, mem, row, dn, dc, s_lane[lane]);
+                                    add_run_sums(sN, sC, bk.NB, bk.CB, nbL, cbL, oxn, oyn, ozn, oxc, oyc, ozc, lane, dn, dc,
+                                                 float(cq), float(cm));
+                                } else {
+                                    butterfly_sums<A, T>(row, me, cq, cm, sN, sC, bk.NB, bk.CB, nbL, cbL, oxn, oyn, ozn, oxc, oyc, ozc,
+                                                         lane);
+                                }
+                            } else if (me) {
+                                imp_deposit_direct<A, T>(row, cq, cm, sN, sC, bk.NB, bk.CB, nb, cb, oxn, oyn, ozn, oxc, oyc, ozc);
+                            }
                         }
                     }
                 }
@@ -737,6 +743,61 @@ struct MoverBlock {
     int cbx, cby, cbz, CB;
 };
 
+// The rows of tiles along x of a mover's work box (y fastest), species after
+// species: chunks of 32 particles in the rows before each, the row's first
+// particle and its end.  In shared memory, sized by the launch.
+struct RowTable {
+    int *before, *first, *end;   // before[n]: all chunks
+    int n;
+    __device__ RowTable(int* mem, int rows) : before(mem), first(mem + rows + 1), end(mem + 2 * rows + 1), n(rows) {}
+    // The row of chunk c, at or after row `at` (a warp's lanes together; the
+    // last one for a c past the end).
+    __device__ int row_of(int c, int at, int lane) const {
+        unsigned passed;
+        do {
+            const int i = at + 1 + lane;
+            passed = __ballot_sync(0xffffffffu, i < n && before[i < n ? i : 0] <= c);
+            at += __popc(passed);
+        } while (passed == 0xffffffffu);
+        return at;
+    }
+    // Filled by the first warp for the box (ti, tj, tk) of t.
+    template <typename T>
+    __device__ void fill(const ImpSpecies<T>& S, const TileGeom& o, const TileGeom& t, int ti, int tj, int tk) {
+        const int lane = threadIdx.x;
+        if (lane >= 32) return;
+        const int gy = t.ty / o.ty, gz = t.tz / o.tz, T3 = o.tx * o.ty * o.tz;
+        const int a0 = box_start(o.ntx, ti, t.ntx), a1 = box_start(o.ntx, ti + 1, t.ntx);
+        const int b0 = box_start(o.nty, tj, t.nty), b1 = box_start(o.nty, tj + 1, t.nty);
+        const int c0 = box_start(o.ntz, tk, t.ntz), c1 = box_start(o.ntz, tk + 1, t.ntz);
+        int done = 0;
+        for (int h = 0; h < n; h += 32) {
+            const int e = h + lane, s = e / (gy * gz), w = e - s * (gy * gz);
+            const int b = b0 + w % gy, c = c0 + w / gy;
+            int x0 = 0, x1 = 0;
+            if (e < n && b < b1 && c < c1) {
+                const long long row = ((long long)c * o.nty + b) * o.ntx;
+                x0 = S.off[s][(row + a0) * T3];
+                x1 = S.off[s][(row + a1) * T3];
+            }
+            const int mine = (x1 - x0 + 31) / 32;
+            int x = mine;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, d);
+                if (lane >= d) x += y;
+            }
+            if (e < n) {
+                before[e] = done + x - mine;
+                first[e] = x0;
+                end[e] = x1;
+            }
+            done += __shfl_sync(0xffffffffu, x, 31);
+        }
+        if (lane == 0) before[n] = done;
+    }
+};
+
 // The tiled mover's constants in the particle precision.
 template <typename T>
 struct MoverSet {
@@ -753,10 +814,20 @@ struct MoverSet {
 // and its bit set in S.defer: k_implicit_push_deferred moves it from the
 // FP64 grids (the kernel itself calls nothing out of line, which would cost
 // its hot loop register spills).  Same arithmetic as k_implicit_push.
-// kParts: several CTAs per tile (parts > 1); without it the loop keeps no
-// register for the stride.
-template <typename T, bool kWall, bool kParts>
-__global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g, TileGeom t, MoverBlock mb, ImpSpecies<T> S,
+// kRows: t holds work boxes of one or several of the sort's tiles o (some a tile
+// smaller than others, box_start; along an axis that 8 does not divide those tiles are 4, 2 or 1
+// cells wide, and their two-cell halo would be most of what a CTA stages), and
+// `nparts` CTAs share a box.  The particles are the box's rows of tiles along x,
+// one range of indices each and of all species one after the other, which the
+// warps take 32 at a time: in a small box, where a CTA has a few hundred
+// particles, all its warps work at once.  Without it: a CTA per tile, species by
+// species.
+// FP32 beams of 39x57x53 (tiles of one cell), 60 per species and cell: 3,170 ->
+// 802 us; shock of 112x51x5: 192 -> 135 us; FP64 pairs of 61x43x1: 525 -> 413 us;
+// of 32x32x1, 32 per species and cell (whole tiles, 19 CTAs each): 207 -> 108 us.
+template <typename T, bool kWall, bool kRows>
+__global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g, TileGeom t, TileGeom o, MoverBlock mb,
+                                                            const __grid_constant__ ImpSpecies<T> S,
                                                             const __grid_constant__ MoverSet<T> K,
                                                             const double* __restrict__ E, const double* __restrict__ B,
                                                             const double* __restrict__ Et, int nparts) {
@@ -799,12 +870,14 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
     const T dt = K.dt, eta = K.eta, edt = K.edt, redt = K.redt;
     const T id[3] = {K.id[0], K.id[1], K.id[2]};
     const int nn[3] = {g.nx, g.ny, g.nz};
-    const int parts = kParts ? nparts : 1;
-    // `parts` CTAs share a tile: each takes every parts-th run of blockDim particles
+    const int parts = kRows ? nparts : 1;
+    const int nrows = kRows ? S.ns * (t.ty / o.ty) * (t.tz / o.tz) : 0;
+    RowTable rows(sPreCell + blockDim.x, nrows);   // (kRows)
     for (int work = blockIdx.x; work < ntiles * parts; work += gridDim.x) {
         const int tile = work / parts, part = work - tile * parts;
         const int ti = tile % t.ntx, tj = (tile / t.ntx) % t.nty, tk = tile / (t.ntx * t.nty);
-        const int x0 = ti * t.tx, y0 = tj * t.ty, z0 = tk * t.tz;
+        const int x0 = box_start(o.ntx, ti, t.ntx) * o.tx, y0 = box_start(o.nty, tj, t.nty) * o.ty,
+                  z0 = box_start(o.ntz, tk, t.ntz) * o.tz;
         __syncthreads();   // previous tile's particles are done with the blocks
         for (int e = threadIdx.x; e < mb.NB; e += blockDim.x) {
             const int lx = e % mb.nbx, ly = (e / mb.nbx) % mb.nby, lz = e / (mb.nbx * mb.nby);
@@ -829,200 +902,238 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
                 for (int c = 0; c < 3; ++c) sB[c * mb.CB + e] = T(B[c * g.N + gid]);
             }
         }
+        if constexpr (kRows) rows.fill(S, o, t, ti, tj, tk);
         __syncthreads();
-        for (int s = 0; s < S.ns; ++s) {
-            const PartView<T> p = S.p[s];
-            const T beta = K.beta[s], qdt = K.qdt[s], mm = K.m[s];
-            const int b0 = S.off[s][tile * T3] + part * blockDim.x, b1 = S.off[s][(tile + 1) * T3];
-            const int step = kParts ? parts * blockDim.x : blockDim.x;
-            if (b0 + (int)threadIdx.x < b1) stage(p, b0 + threadIdx.x);
+        // moves particle n of species s, staged in this thread's slot, whose copy
+        // of the next one `refill` starts once the slot is read
+        auto move = [&](int s, const PartView<T>& p, T beta, T qdt, T mm, int n, auto refill) {
+            const int bdim = blockDim.x, me = threadIdx.x;
+            const int cell_n = sPreCell[me];
+            const T pu[3] = {sPre[0 * bdim + me], sPre[1 * bdim + me], sPre[2 * bdim + me]};
+            const T pm[3] = {sPre[3 * bdim + me], sPre[4 * bdim + me], sPre[5 * bdim + me]};
+            refill();
             cp_async_commit();
-            for (int n = b0 + threadIdx.x; n < b1; n = b1 - n > step ? n + step : b1) {   // (no int overflow)
-                cp_async_wait_all();   // this thread's particle n (its own slot)
-                const int bdim = blockDim.x, me = threadIdx.x;
-                const int cell_n = sPreCell[me];
-                const T pu[3] = {sPre[0 * bdim + me], sPre[1 * bdim + me], sPre[2 * bdim + me]};
-                const T pm[3] = {sPre[3 * bdim + me], sPre[4 * bdim + me], sPre[5 * bdim + me]};
-                if (b1 - n > step) stage(p, n + step);
-                cp_async_commit();
-                int ci[3];
-                decode(g, cell_n, ci[0], ci[1], ci[2]);
-                // A position (cell c, offset u) is located once: its node and cell
-                // stencils in the staged block (bases, upper weights), shared by the
-                // two or three gathers there; a stencil that leaves the block
-                // gathers from the FP64 grids.
-                struct Loc {
-                    bool inb;
-                    int nbase, cbase;
-                    T wn[3], wc[3];
-                };
-                // from tile-local cells l (the block holds l in [-h, t - 1 + h])
-                auto locate_l = [&](const int l[3], const T u[3], Loc& L) {
-                    L.inb = l[0] >= -hx && l[0] <= t.tx - 1 + hx && l[1] >= -hy && l[1] <= t.ty - 1 + hy &&
-                            l[2] >= -hz && l[2] <= t.tz - 1 + hz;
-                    if (!L.inb) return;
-                    int lo[3];
+            int ci[3];
+            decode(g, cell_n, ci[0], ci[1], ci[2]);
+            // A position (cell c, offset u) is located once: its node and cell
+            // stencils in the staged block (bases, upper weights), shared by the
+            // two or three gathers there; a stencil that leaves the block
+            // gathers from the FP64 grids.
+            struct Loc {
+                bool inb;
+                int nbase, cbase;
+                T wn[3], wc[3];
+            };
+            // from tile-local cells l (the block holds l in [-h, t - 1 + h])
+            auto locate_l = [&](const int l[3], const T u[3], Loc& L) {
+                L.inb = l[0] >= -hx && l[0] <= t.tx - 1 + hx && l[1] >= -hy && l[1] <= t.ty - 1 + hy &&
+                        l[2] >= -hz && l[2] <= t.tz - 1 + hz;
+                if (!L.inb) return;
+                int lo[3];
 #pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        // upper weights: u of the nodes (c, c + 1); of the cell
-                        // pair (c - 1, c) below the centre u + 1/2, (c, c + 1)
-                        // above it u - 1/2
-                        const bool act = nn[a] > 1, below = act && u[a] < T(0.5);
-                        L.wn[a] = act ? u[a] : T(0);
-                        L.wc[a] = act ? u[a] + (below ? T(0.5) : T(-0.5)) : T(0);
-                        lo[a] = below ? l[a] - 1 : l[a];
+                for (int a = 0; a < 3; ++a) {
+                    // upper weights: u of the nodes (c, c + 1); of the cell
+                    // pair (c - 1, c) below the centre u + 1/2, (c, c + 1)
+                    // above it u - 1/2
+                    const bool act = nn[a] > 1, below = act && u[a] < T(0.5);
+                    L.wn[a] = act ? u[a] : T(0);
+                    L.wc[a] = act ? u[a] + (below ? T(0.5) : T(-0.5)) : T(0);
+                    lo[a] = below ? l[a] - 1 : l[a];
+                }
+                L.nbase = (l[2] + hz) * nsz + (l[1] + hy) * nsy + (l[0] + hx) * nsx;
+                const int ex = ax ? 1 : 0, ey = ay ? 1 : 0, ez = az ? 1 : 0;
+                L.cbase = (lo[2] + hz + ez) * csz + (lo[1] + hy + ey) * csy + (lo[0] + hx + ex) * csx;
+            };
+            // from global cells c: the periodic image inside the block, if any
+            auto locate = [&](const int c[3], const T u[3], Loc& L, int l[3]) {
+                if (!(local_axis(c[0], x0, t.tx, hx, g.nx, l[0]) && local_axis(c[1], y0, t.ty, hy, g.ny, l[1]) &&
+                      local_axis(c[2], z0, t.tz, hz, g.nz, l[2]))) {
+                    L.inb = false;
+                    return;
+                }
+                locate_l(l, u, L);
+            };
+            // gathers at a located position inside the block: E^theta
+            // (nodes, corner weights w) and B^n (cells), float4 blocks for FP32
+            auto gatEt = [&](const Loc& L, const T w[8], T out[3]) {
+                if constexpr (kVec) gather3(sEt4, L.nbase, nsx, nsy, nsz, w, out);
+                else gather3<T>(sEt, mb.NB, L.nbase, nsx, nsy, nsz, w, out);
+            };
+            auto gatB = [&](const Loc& L, T out[3]) {
+                T w[8];
+                corners<T>(L.wc[0], L.wc[1], L.wc[2], w);
+                if constexpr (kVec) gather3(sB4, L.cbase, csx, csy, csz, w, out);
+                else gather3<T>(sB, mb.CB, L.cbase, csx, csy, csz, w, out);
+            };
+            auto defer = [&]() { atomicOr(&S.defer[s][n >> 5], 1u << (n & 31)); };
+            T u0[3] = {pu[0], pu[1], pu[2]};
+            T mom0[3] = {pm[0], pm[1], pm[2]};
+            T gam, v[3];
+            gamma_vel<T>(mom0, mm, gam, v);
+            T e[3], e0[3], b[3], al[9];
+            Loc L0;
+            int l0[3];
+            locate(ci, u0, L0, l0);
+            if (!L0.inb) {
+                defer();
+                return;
+            }
+            {
+                T w[8];
+                corners<T>(L0.wn[0], L0.wn[1], L0.wn[2], w);
+                gather3<T>(sE, mb.NB, L0.nbase, nsx, nsy, nsz, w, e0);
+                gatEt(L0, w, e);
+            }
+            gatB(L0, b);
+            alpha_tensor<T>(beta, v, gam, e0, b, al);
+            T vxb[3] = {v[1] * b[2] - v[2] * b[1], -v[0] * b[2] + v[2] * b[0], v[0] * b[1] - v[1] * b[0]};
+            T pnew[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) pnew[d] = mom0[d] + (e[d] + vxb[d]) * qdt;
+            T vnew[3];
+            evaluate_velocity<T>(pnew, mm, vnew);
+            T mv[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) mv[d] = v[d] * (T(1) - eta) + vnew[d] * eta;
+            if constexpr (kWall) {
+                if (wall_left_of<T>(ci[0], u0[0], (mv[0] * edt) * id[0])) {
+                    wall_reflect_trial<T>(g, ci, u0, mv, vnew, mm, edt, redt, id, pnew);
+                    p.px[n] = pnew[0]; p.py[n] = pnew[1]; p.pz[n] = pnew[2];
+                    p.ox[n] = u0[0]; p.oy[n] = u0[1]; p.oz[n] = u0[2];
+                    p.cell[n] = tristan_escaped<T>(g, ci[0], u0[0]) ? -1 : (int)lin(g, ci[0], ci[1], ci[2]);
+                    return;
+                }
+            }
+            T vh[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                vh[a] = (al[3 * a] * gam) * v[0] + (al[3 * a + 1] * gam) * v[1] + (al[3 * a + 2] * gam) * v[2];
+            const T momNorm = (mom0[0] * mom0[0] + mom0[1] * mom0[1] + mom0[2] * mom0[2]);
+            T err = ((mom0[0] - pnew[0]) * (mom0[0] - pnew[0]) + (mom0[1] - pnew[1]) * (mom0[1] - pnew[1]) +
+                             (mom0[2] - pnew[2]) * (mom0[2] - pnew[2]));
+            const T dxN = K.dx2;
+            T cerr = dxN;
+            T newDisp[3] = {mv[0] * edt, mv[1] * edt, mv[2] * edt};
+            T prevDisp[3];
+            int it = 0;
+            bool reflected = false, left = false;
+            while (picard_continue<T>(err, momNorm, cerr, dxN, it)) {
+                ++it;
+                const T prevMom[3] = {pnew[0], pnew[1], pnew[2]};
+#pragma unroll
+                for (int d = 0; d < 3; ++d) prevDisp[d] = newDisp[d];
+                T re[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) re[a] = al[3 * a] * e[0] + al[3 * a + 1] * e[1] + al[3 * a + 2] * e[2];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) mv[d] = vh[d] + re[d] * beta;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) newDisp[d] = mv[d] * edt;
+                if constexpr (kWall) {
+                    if (wall_left_of<T>(ci[0], u0[0], newDisp[0] * id[0])) {
+                        wall_reflect_trial<T>(g, ci, u0, mv, vnew, mm, edt, redt, id, pnew);
+                        reflected = true;
+                        break;
                     }
-                    L.nbase = (l[2] + hz) * nsz + (l[1] + hy) * nsy + (l[0] + hx) * nsx;
-                    const int ex = ax ? 1 : 0, ey = ay ? 1 : 0, ez = az ? 1 : 0;
-                    L.cbase = (lo[2] + hz + ez) * csz + (lo[1] + hy + ey) * csy + (lo[0] + hx + ex) * csx;
-                };
-                // from global cells c: the periodic image inside the block, if any
-                auto locate = [&](const int c[3], const T u[3], Loc& L, int l[3]) {
-                    if (!(local_axis(c[0], x0, t.tx, hx, g.nx, l[0]) && local_axis(c[1], y0, t.ty, hy, g.ny, l[1]) &&
-                          local_axis(c[2], z0, t.tz, hz, g.nz, l[2]))) {
-                        L.inb = false;
-                        return;
-                    }
-                    locate_l(l, u, L);
-                };
-                // gathers at a located position inside the block: E^theta
-                // (nodes, corner weights w) and B^n (cells), float4 blocks for FP32
-                auto gatEt = [&](const Loc& L, const T w[8], T out[3]) {
-                    if constexpr (kVec) gather3(sEt4, L.nbase, nsx, nsy, nsz, w, out);
-                    else gather3<T>(sEt, mb.NB, L.nbase, nsx, nsy, nsz, w, out);
-                };
-                auto gatB = [&](const Loc& L, T out[3]) {
-                    T w[8];
-                    corners<T>(L.wc[0], L.wc[1], L.wc[2], w);
-                    if constexpr (kVec) gather3(sB4, L.cbase, csx, csy, csz, w, out);
-                    else gather3<T>(sB, mb.CB, L.cbase, csx, csy, csz, w, out);
-                };
-                auto defer = [&]() { atomicOr(&S.defer[s][n >> 5], 1u << (n & 31)); };
-                T u0[3] = {pu[0], pu[1], pu[2]};
-                T mom0[3] = {pm[0], pm[1], pm[2]};
-                T gam, v[3];
-                gamma_vel<T>(mom0, mm, gam, v);
-                T e[3], e0[3], b[3], al[9];
-                Loc L0;
-                int l0[3];
-                locate(ci, u0, L0, l0);
-                if (!L0.inb) {
-                    defer();
-                    continue;
+                }
+                // the trial position x^n + newDisp: the offsets as advance_axis
+                // forms them, the cell in tile-local terms (no periodic wrap)
+                T tu[3];
+                int tl[3];
+                Loc L1;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const T sd = u0[d] + newDisp[d] * id[d];
+                    const T fd = dev_floor(sd);
+                    T ud = sd - fd;
+                    int cd = l0[d] + (int)fd;
+                    if (ud >= T(1)) { ud -= T(1); cd += 1; }
+                    tl[d] = nn[d] > 1 ? cd : 0;
+                    tu[d] = ud;
+                }
+                locate_l(tl, tu, L1);
+                if (!L1.inb) {
+                    left = true;
+                    break;
                 }
                 {
                     T w[8];
-                    corners<T>(L0.wn[0], L0.wn[1], L0.wn[2], w);
-                    gather3<T>(sE, mb.NB, L0.nbase, nsx, nsy, nsz, w, e0);
-                    gatEt(L0, w, e);
+                    corners<T>(L1.wn[0], L1.wn[1], L1.wn[2], w);
+                    gatEt(L1, w, e);
                 }
-                gatB(L0, b);
-                alpha_tensor<T>(beta, v, gam, e0, b, al);
-                T vxb[3] = {v[1] * b[2] - v[2] * b[1], -v[0] * b[2] + v[2] * b[0], v[0] * b[1] - v[1] * b[0]};
-                T pnew[3];
+                gatB(L1, b);
+                const T mvxb[3] = {mv[1] * b[2] - mv[2] * b[1], -mv[0] * b[2] + mv[2] * b[0], mv[0] * b[1] - mv[1] * b[0]};
 #pragma unroll
-                for (int d = 0; d < 3; ++d) pnew[d] = mom0[d] + (e[d] + vxb[d]) * qdt;
-                T vnew[3];
-                evaluate_velocity<T>(pnew, mm, vnew);
-                T mv[3];
-#pragma unroll
-                for (int d = 0; d < 3; ++d) mv[d] = v[d] * (T(1) - eta) + vnew[d] * eta;
+                for (int d = 0; d < 3; ++d) pnew[d] = mom0[d] + (e[d] + mvxb[d]) * qdt;
+                err = ((prevMom[0] - pnew[0]) * (prevMom[0] - pnew[0]) +
+                               (prevMom[1] - pnew[1]) * (prevMom[1] - pnew[1]) +
+                               (prevMom[2] - pnew[2]) * (prevMom[2] - pnew[2]));
+                cerr = ((prevDisp[0] - newDisp[0]) * (prevDisp[0] - newDisp[0]) +
+                                (prevDisp[1] - newDisp[1]) * (prevDisp[1] - newDisp[1]) +
+                                (prevDisp[2] - newDisp[2]) * (prevDisp[2] - newDisp[2]));
+            }
+            if (left) {   // nothing written yet: the deferred pass moves it from the start
+                defer();
+                return;
+            }
+            if (!reflected) {
                 if constexpr (kWall) {
-                    if (wall_left_of<T>(ci[0], u0[0], (mv[0] * edt) * id[0])) {
-                        wall_reflect_trial<T>(g, ci, u0, mv, vnew, mm, edt, redt, id, pnew);
-                        p.px[n] = pnew[0]; p.py[n] = pnew[1]; p.pz[n] = pnew[2];
-                        p.ox[n] = u0[0]; p.oy[n] = u0[1]; p.oz[n] = u0[2];
-                        p.cell[n] = tristan_escaped<T>(g, ci[0], u0[0]) ? -1 : (int)lin(g, ci[0], ci[1], ci[2]);
-                        continue;
-                    }
+                    const int o = wall_final_x<T>(g, ci[0], u0[0], (mv[0] * dt) * id[0]);
+                    if (o == 2) { p.cell[n] = -1; return; }   // escaped through the open boundary
+                    if (o == 1) pnew[0] = -pnew[0];
+#pragma unroll
+                    for (int d = 1; d < 3; ++d) advance_axis<T>(u0[d], ci[d], (mv[d] * dt) * id[d], nn[d]);
+                } else {
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) advance_axis<T>(u0[d], ci[d], (mv[d] * dt) * id[d], nn[d]);
                 }
-                T vh[3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-                    vh[a] = (al[3 * a] * gam) * v[0] + (al[3 * a + 1] * gam) * v[1] + (al[3 * a + 2] * gam) * v[2];
-                const T momNorm = (mom0[0] * mom0[0] + mom0[1] * mom0[1] + mom0[2] * mom0[2]);
-                T err = ((mom0[0] - pnew[0]) * (mom0[0] - pnew[0]) + (mom0[1] - pnew[1]) * (mom0[1] - pnew[1]) +
-                                 (mom0[2] - pnew[2]) * (mom0[2] - pnew[2]));
-                const T dxN = K.dx2;
-                T cerr = dxN;
-                T newDisp[3] = {mv[0] * edt, mv[1] * edt, mv[2] * edt};
-                T prevDisp[3];
-                int it = 0;
-                bool reflected = false, left = false;
-                while (picard_continue<T>(err, momNorm, cerr, dxN, it)) {
-                    ++it;
-                    const T prevMom[3] = {pnew[0], pnew[1], pnew[2]};
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) prevDisp[d] = newDisp[d];
-                    T re[3];
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) re[a] = al[3 * a] * e[0] + al[3 * a + 1] * e[1] + al[3 * a + 2] * e[2];
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) mv[d] = vh[d] + re[d] * beta;
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) newDisp[d] = mv[d] * edt;
-                    if constexpr (kWall) {
-                        if (wall_left_of<T>(ci[0], u0[0], newDisp[0] * id[0])) {
-                            wall_reflect_trial<T>(g, ci, u0, mv, vnew, mm, edt, redt, id, pnew);
-                            reflected = true;
-                            break;
-                        }
-                    }
-                    // the trial position x^n + newDisp: the offsets as advance_axis
-                    // forms them, the cell in tile-local terms (no periodic wrap)
-                    T tu[3];
-                    int tl[3];
-                    Loc L1;
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        const T sd = u0[d] + newDisp[d] * id[d];
-                        const T fd = dev_floor(sd);
-                        T ud = sd - fd;
-                        int cd = l0[d] + (int)fd;
-                        if (ud >= T(1)) { ud -= T(1); cd += 1; }
-                        tl[d] = nn[d] > 1 ? cd : 0;
-                        tu[d] = ud;
-                    }
-                    locate_l(tl, tu, L1);
-                    if (!L1.inb) {
-                        left = true;
-                        break;
-                    }
-                    {
-                        T w[8];
-                        corners<T>(L1.wn[0], L1.wn[1], L1.wn[2], w);
-                        gatEt(L1, w, e);
-                    }
-                    gatB(L1, b);
-                    const T mvxb[3] = {mv[1] * b[2] - mv[2] * b[1], -mv[0] * b[2] + mv[2] * b[0], mv[0] * b[1] - mv[1] * b[0]};
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) pnew[d] = mom0[d] + (e[d] + mvxb[d]) * qdt;
-                    err = ((prevMom[0] - pnew[0]) * (prevMom[0] - pnew[0]) +
-                                   (prevMom[1] - pnew[1]) * (prevMom[1] - pnew[1]) +
-                                   (prevMom[2] - pnew[2]) * (prevMom[2] - pnew[2]));
-                    cerr = ((prevDisp[0] - newDisp[0]) * (prevDisp[0] - newDisp[0]) +
-                                    (prevDisp[1] - newDisp[1]) * (prevDisp[1] - newDisp[1]) +
-                                    (prevDisp[2] - newDisp[2]) * (prevDisp[2] - newDisp[2]));
+            }
+            p.px[n] = pnew[0]; p.py[n] = pnew[1]; p.pz[n] = pnew[2];
+            p.ox[n] = u0[0]; p.oy[n] = u0[1]; p.oz[n] = u0[2];
+            p.cell[n] = kWall && tristan_escaped<T>(g, ci[0], u0[0]) ? -1 : (int)lin(g, ci[0], ci[1], ci[2]);
+        };
+        if constexpr (kRows) {
+            const int lane = threadIdx.x & 31, warps = blockDim.x >> 5, per = (t.ty / o.ty) * (t.tz / o.tz);
+            int c = part * warps + (threadIdx.x >> 5), at = 0, n0 = 0, pe = 0, s = 0;   // chunk, row, first particle, row's end, species
+            auto seek = [&]() {
+                at = rows.row_of(c, at, lane);
+                const bool some = c < rows.before[nrows];
+                n0 = some ? rows.first[at] + 32 * (c - rows.before[at]) : 0;
+                pe = some ? rows.end[at] : 0;
+                s = at / per;
+            };
+            seek();
+            if (lane < pe - n0) stage(S.p[s], n0 + lane);
+            cp_async_commit();
+            while (n0 < pe) {
+                cp_async_wait_all();   // this thread's particle (its own slot)
+                const int n = n0 + lane, here = pe - n0, sn = s;
+                c += parts * warps;
+                seek();
+                auto refill = [&]() {
+                    if (lane < pe - n0) stage(S.p[s], n0 + lane);
+                };
+                if (lane < here) {
+                    move(sn, S.p[sn], K.beta[sn], K.qdt[sn], K.m[sn], n, refill);
+                } else {
+                    refill();
+                    cp_async_commit();
                 }
-                if (left) {   // nothing written yet: the deferred pass moves it from the start
-                    defer();
-                    continue;
+                __syncwarp();
+            }
+        } else {
+            for (int s = 0; s < S.ns; ++s) {
+                const PartView<T> p = S.p[s];
+                const T beta = K.beta[s], qdt = K.qdt[s], mm = K.m[s];
+                const int b0 = S.off[s][tile * T3], b1 = S.off[s][(tile + 1) * T3], step = blockDim.x;
+                if (b0 + (int)threadIdx.x < b1) stage(p, b0 + threadIdx.x);
+                cp_async_commit();
+                for (int n = b0 + threadIdx.x; n < b1; n = b1 - n > step ? n + step : b1) {   // (no int overflow)
+                    cp_async_wait_all();   // this thread's particle n (its own slot)
+                    move(s, p, beta, qdt, mm, n, [&]() {
+                        if (b1 - n > step) stage(p, n + step);
+                    });
                 }
-                if (!reflected) {
-                    if constexpr (kWall) {
-                        const int o = wall_final_x<T>(g, ci[0], u0[0], (mv[0] * dt) * id[0]);
-                        if (o == 2) { p.cell[n] = -1; continue; }   // escaped through the open boundary
-                        if (o == 1) pnew[0] = -pnew[0];
-#pragma unroll
-                        for (int d = 1; d < 3; ++d) advance_axis<T>(u0[d], ci[d], (mv[d] * dt) * id[d], nn[d]);
-                    } else {
-#pragma unroll
-                        for (int d = 0; d < 3; ++d) advance_axis<T>(u0[d], ci[d], (mv[d] * dt) * id[d], nn[d]);
-                    }
-                }
-                p.px[n] = pnew[0]; p.py[n] = pnew[1]; p.pz[n] = pnew[2];
-                p.ox[n] = u0[0]; p.oy[n] = u0[1]; p.oz[n] = u0[2];
-                p.cell[n] = kWall && tristan_escaped<T>(g, ci[0], u0[0]) ? -1 : (int)lin(g, ci[0], ci[1], ci[2]);
             }
         }
     }

@@ -30,8 +30,8 @@ inline int red_blocks(long long n) {
     return (int)b;
 }
 
-// CTAs that share one tile's particles in the fused explicit kernel and the
-// tiled mover, of which `slots` run at once.  A box with fewer tiles than that
+// CTAs that share one tile's particles in the fused explicit kernel, of which
+// `slots` run at once.  A box with fewer tiles than that
 // would leave SMs idle: its tiles are cut into as many parts as still run in
 // one wave.  `even`: larger boxes are cut too where that fills the last wave
 // (the FP64 explicit kernel, milliseconds per tile: staging a tile again costs
@@ -80,9 +80,10 @@ struct PK {
                                        const ImpBlock& bk,
                                        const ImpSpecies<T>& S, const T* E, const T* B, double* J,
                                        double* mu, double* rho, double* Pi);
-    // tiled mover (implicit_tile.cuh): fields staged per tile; needs
-    // tile-major sorted particles; false if the blocks do not fit
-    static bool implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const ImpSpecies<T>& S,
+    // tiled mover (implicit_tile.cuh) over work boxes t of the sort's tiles o:
+    // fields staged per box; needs tile-major sorted particles; false if the
+    // blocks do not fit
+    static bool implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileGeom& o, const ImpSpecies<T>& S,
                                     const double* E, const double* B, const double* Et);
     static void implicit_push(cudaStream_t s, const GridP& g, PartView<T> p, double q, double m, const double* E,
                               const double* B, const double* Et);

@@ -13,6 +13,6 @@ template size_t PK<double>::implicit_tile_smem(const ImpBlock&, int, int);
 template void PK<double>::implicit_deposit_tiled(cudaStream_t, const GridP&, const TileGeom&, const TileGeom&,
                                                  const ImpBlock&, const ImpSpecies<double>&, const double*, const double*,
                                                  double*, double*, double*, double*);
-template bool PK<double>::implicit_push_tiled(cudaStream_t, const GridP&, const TileGeom&, const ImpSpecies<double>&,
+template bool PK<double>::implicit_push_tiled(cudaStream_t, const GridP&, const TileGeom&, const TileGeom&, const ImpSpecies<double>&,
                                               const double*, const double*, const double*);
 }  // namespace pic

@@ -149,7 +149,7 @@ void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeo
 }
 
 template <typename T>
-bool PK<T>::implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const ImpSpecies<T>& S,
+bool PK<T>::implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileGeom& o, const ImpSpecies<T>& S,
                                 const double* E, const double* B, const double* Et) {
     MoverBlock mb{};
     const int H = kMoverHalo;
@@ -165,8 +165,28 @@ bool PK<T>::implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& 
     const size_t fld = sizeof(T) == sizeof(float)
                            ? ((size_t)mb.NB + (size_t)mb.CB) * 16 + 3 * (size_t)mb.NB * sizeof(float)
                            : (6 * (size_t)mb.NB + 3 * (size_t)mb.CB) * sizeof(T);
-    // plus every thread's staged next particle (6 values and a cell)
-    const size_t smem = ((fld + 15) & ~size_t(15)) + (size_t)kMoverThreads * (6 * sizeof(T) + sizeof(int));
+    // CTAs per box (p): at least as many as run at once, and so many that the last
+    // wave of them is nearly full, as long as each has enough particles to pay
+    // for staging the box.  FP64 particles, ten times as long in work, are cut as
+    // fine as that allows (pairs of 61x43x1: 6 CTAs per box 511 us, 25 413 us);
+    // FP32 as little (40x56x56: one CTA per box 806 us, five 760 us; 64x64x16: 2
+    // 475 us, 7 435 us).
+    const int n = t.ntx * t.nty * t.ntz, slots = 2 * kNumSM;
+    long long total = 0;
+    for (int q = 0; q < S.ns; ++q) total += S.p[q].n;
+    int parts = n < slots ? slots / n : 1;
+    const long long least = sizeof(T) == 8 ? 192 : 4096;
+    double most = 0;
+    for (int p = parts, limit = 4 * parts + 12; p <= limit && (sizeof(T) == 8 || most < 0.94) && (most == 0 || total / least >= (long long)n * p); ++p) {
+        const double waves = (double)n * p / slots, use = waves / std::ceil(waves);
+        if (use > most + 0.02 || (sizeof(T) == 8 && use >= 0.94)) { most = use; parts = p; }
+    }
+    const bool rows = parts > 1 || t.tx != o.tx || t.ty != o.ty || t.tz != o.tz;
+    // plus every thread's staged next particle (6 values and a cell), and the
+    // rows of a work box
+    const int nrows = S.ns * (t.ty / o.ty) * (t.tz / o.tz);
+    const size_t smem = ((fld + 15) & ~size_t(15)) + (size_t)kMoverThreads * (6 * sizeof(T) + sizeof(int)) +
+                        (rows ? (3 * (size_t)nrows + 1) * sizeof(int) : 0);
     if (smem > 227 * 1024) return false;
     static bool attr_set = false;
     if (!attr_set) {
@@ -177,15 +197,14 @@ bool PK<T>::implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& 
     }
     const int per_sm = (int)((228 * 1024) / (smem + 1024));
     const int cap = kNumSM * (per_sm > 0 ? per_sm : 1);
-    const int parts = tile_parts(t, 2 * kNumSM, false);
-    const int nwork = t.ntx * t.nty * t.ntz * parts;
-    // the wall rules are a separate instantiation: the periodic mover keeps
-    // none of their code in its loop
+    const int nwork = n * parts;
     // the particles it left over: one thread per mask word
     long long words = 1;
     for (int q = 0; q < S.ns; ++q) words = std::max(words, (S.p[q].n + 31) / 32);
-    auto* kernel = g.wall ? (parts > 1 ? k_implicit_push_tile<T, true, true> : k_implicit_push_tile<T, true, false>)
-                          : (parts > 1 ? k_implicit_push_tile<T, false, true> : k_implicit_push_tile<T, false, false>);
+    // the wall rules are a separate instantiation: the periodic mover keeps
+    // none of their code in its loop
+    auto* kernel = g.wall ? (rows ? k_implicit_push_tile<T, true, true> : k_implicit_push_tile<T, true, false>)
+                          : (rows ? k_implicit_push_tile<T, false, true> : k_implicit_push_tile<T, false, false>);
     MoverSet<T> K{};
     K.dt = T(g.dt); K.eta = T(g.eta); K.edt = T(g.eta * g.dt); K.redt = T((1.0 - g.eta) * g.dt);
     K.dx2 = T(g.dx) * T(g.dx);
@@ -195,7 +214,7 @@ bool PK<T>::implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& 
         K.qdt[q] = T(S.q[q] * g.dt);
         K.m[q] = T(S.m[q]);
     }
-    kernel<<<nwork < cap ? nwork : cap, kMoverThreads, smem, s>>>(g, t, mb, S, K, E, B, Et, parts);
+    kernel<<<nwork < cap || rows ? nwork : cap, kMoverThreads, smem, s>>>(g, t, o, mb, S, K, E, B, Et, parts);
     if (g.wall) k_implicit_push_deferred<T, true><<<grid_for(words, 128), 128, 0, s>>>(g, S, E, B, Et);
     else k_implicit_push_deferred<T, false><<<grid_for(words, 128), 128, 0, s>>>(g, S, E, B, Et);
     return true;

@@ -21,6 +21,13 @@ struct TileGeom {
     int lx, ly, lz;      // log2 of the extents when all three are powers of two, else -1
 };
 
+// Boxes that need not divide an axis: the first of n cells (or tiles) of box b
+// of m (the first n % m boxes have one more than the others).
+__host__ __device__ __forceinline__ int box_start(int n, int b, int m) {
+    const int q = n / m, r = n - q * m;
+    return b * q + (b < r ? b : r);
+}
+
 // Sort key of cell (i, j, k): tile by tile, x fastest in a tile.
 __device__ __forceinline__ int cell_key(const TileGeom& t, int i, int j, int k) {
     int ti, tj, tk;

@@ -1,5 +1,7 @@
-"""The implicit mover on a two-cell periodic axis, whose halo wraps around it
-more than once, against the oracle.  Needs a GB300."""
+"""The implicit mover's work boxes (csrc/implicit_tile.cuh) on grids whose axes 8
+does not divide, against one CTA per tile of the sort (the same tiles asked for
+by name); and a two-cell periodic axis, whose halo wraps around it more than
+once, against the oracle.  Needs a GB300."""
 import numpy as np
 import pytest
 
@@ -39,6 +41,33 @@ def by_id(d):
 def distances(box, a, b):
     for x, y, l, d in zip(I.positions(box, a), I.positions(box, b), (box.nx, box.ny, box.nz), (box.dx, box.dy, box.dz)):
         yield periodic_dist(x, y, l * d).max() / d
+
+
+def divisor(n):
+    return next(t for t in (8, 4, 2, 1) if n % t == 0)
+
+
+@pytest.mark.parametrize("n,ppc", [((9, 9, 9), 3), ((20, 7, 3), 9), ((36, 12, 10), 2), ((33, 15, 1), 40), ((3, 5, 17), 33)])
+@pytest.mark.parametrize("real", [0, 1])
+@pytest.mark.parametrize("every", [1, 3])
+def test_work_boxes_match_one_cta_per_tile(pg, n, ppc, real, every):
+    st = state(n, ppc)
+    out = []
+    for tile in ((0, 0, 0), tuple(divisor(a) for a in n)):
+        sim = pg.GpuSimulation(st.box, pg.IMPLICIT, particle_real=real, pressure_compat=0, sort_every=every, tile=tile)
+        sim.upload_state(st)
+        for _ in range(3):
+            sim.implicit_step(pg.solve_opts(pg.GMRES_RESTARTED, tol=1e-13))
+        out.append([by_id(sim.download_particles(s)) for s in range(2)])
+        sim.close()
+    # the movers do the same arithmetic; the moments' sums come in another order
+    # (FP64 1e-16 a term, FP32 6e-8), which the solve passes on at its condition
+    # number (about 10) in each of three steps
+    tol = 1e-11 if real else 1e-5
+    for a, b in zip(*out):
+        assert max(distances(st.box, a, b)) <= tol
+        for k in ("px", "py", "pz"):
+            assert rel_err(a[k], b[k]) <= tol
 
 
 @pytest.mark.parametrize("n", [(9, 2, 2), (2, 9, 1), (8, 2, 3)])
