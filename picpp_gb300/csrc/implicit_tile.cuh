@@ -39,28 +39,6 @@ constexpr int kXposeMin = 4;   // fewest lanes of one cell that take the transpo
 constexpr int kTcMin = 1;      // fewest lanes of one cell that take the tensor-core run sums (FP32)
 
 
-// Symmetric pressure components kept in shared memory, q = 0..5:
-// (a, b) = (0,0) (0,1) (0,2) (1,1) (1,2) (2,2).
-__host__ __device__ constexpr int sym_a(int q) { return q < 3 ? 0 : (q < 5 ? 1 : 2); }
-__host__ __device__ constexpr int sym_b(int q) { return q < 3 ? q : (q < 5 ? q - 2 : 2); }
-
-// Butterfly transpose-reduction of one 32-product pass: returns, in lane L,
-// the sum over the warp of v[L].
-template <typename A>
-__device__ __forceinline__ A xpose_sum(A v[32], int lane) {
-#pragma unroll
-    for (int w = 16; w >= 1; w >>= 1) {
-        const bool up = (lane & w) != 0;
-#pragma unroll
-        for (int i = 0; i < w; ++i) {
-            const A send = up ? v[i] : v[i + w];
-            const A keep = up ? v[i + w] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
-        }
-    }
-    return v[0];
-}
-
 // Node weights (c, c + 1) and cell weights (c - 1, c, c + 1) of one axis
 // (node_w and cell_w of common.cuh without branches).
 template <typename T>
@@ -734,7 +712,6 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
 
 namespace pic {
 
-constexpr int kMoverHalo = 2;   // cells of field halo staged around a mover tile
 
 // Field blocks of the tiled mover: nodes (E^n, E^theta) over tile + 2H + 1,
 // cells (B^n) over tile + 2H + 2 on active axes.

@@ -180,7 +180,8 @@ void PK<T>::implicit_deposit(cudaStream_t s, const GridP& g, PartView<T> p, doub
                              const double* E, const double* B, double* J, double* mu, double* rho, double* Pi,
                              int compat, const GhostAxes& ga) {
     if (p.n == 0) return;
-    k_implicit_deposit<T><<<grid_for(p.n, 128, 32), 128, 0, s>>>(g, p, q, m, w, E, B, J, mu, rho, Pi, compat, ga);
+    auto* kernel = compat ? k_implicit_deposit<T, true> : k_implicit_deposit<T, false>;
+    kernel<<<grid_for(p.n, 128, 32), 128, 0, s>>>(g, p, q, m, w, E, B, J, mu, rho, Pi, ga);
 }
 
 template <typename T>

@@ -165,13 +165,19 @@ bool PK<T>::implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& 
     const size_t fld = sizeof(T) == sizeof(float)
                            ? ((size_t)mb.NB + (size_t)mb.CB) * 16 + 3 * (size_t)mb.NB * sizeof(float)
                            : (6 * (size_t)mb.NB + 3 * (size_t)mb.CB) * sizeof(T);
+    // after the fields every thread's staged next particle (6 values and a cell),
+    // and the rows of a work box
+    const int nrows = S.ns * (t.ty / o.ty) * (t.tz / o.tz);
+    const size_t whole = ((fld + 15) & ~size_t(15)) + (size_t)kMoverThreads * (6 * sizeof(T) + sizeof(int));
+    const size_t most_smem = whole + (3 * (size_t)nrows + 1) * sizeof(int);
+    if (most_smem > 227 * 1024) return false;
     // CTAs per box (p): at least as many as run at once, and so many that the last
     // wave of them is nearly full, as long as each has enough particles to pay
     // for staging the box.  FP64 particles, ten times as long in work, are cut as
     // fine as that allows (pairs of 61x43x1: 6 CTAs per box 511 us, 25 413 us);
     // FP32 as little (40x56x56: one CTA per box 806 us, five 760 us; 64x64x16: 2
     // 475 us, 7 435 us).
-    const int n = t.ntx * t.nty * t.ntz, slots = 2 * kNumSM;
+    const int n = t.ntx * t.nty * t.ntz, slots = (int)std::min<size_t>(2, 228 * 1024 / (most_smem + 1024)) * kNumSM;
     long long total = 0;
     for (int q = 0; q < S.ns; ++q) total += S.p[q].n;
     int parts = n < slots ? slots / n : 1;
@@ -182,12 +188,7 @@ bool PK<T>::implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& 
         if (use > most + 0.02 || (sizeof(T) == 8 && use >= 0.94)) { most = use; parts = p; }
     }
     const bool rows = parts > 1 || t.tx != o.tx || t.ty != o.ty || t.tz != o.tz;
-    // plus every thread's staged next particle (6 values and a cell), and the
-    // rows of a work box
-    const int nrows = S.ns * (t.ty / o.ty) * (t.tz / o.tz);
-    const size_t smem = ((fld + 15) & ~size_t(15)) + (size_t)kMoverThreads * (6 * sizeof(T) + sizeof(int)) +
-                        (rows ? (3 * (size_t)nrows + 1) * sizeof(int) : 0);
-    if (smem > 227 * 1024) return false;
+    const size_t smem = rows ? most_smem : whole;
     static bool attr_set = false;
     if (!attr_set) {
         for (auto* k : {k_implicit_push_tile<T, false, false>, k_implicit_push_tile<T, false, true>,

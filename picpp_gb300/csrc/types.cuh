@@ -91,6 +91,8 @@ struct ImpBlock {
     }
 };
 
+constexpr int kMoverHalo = 2;   // cells of field halo staged around a tile of the implicit mover
+
 // Coefficients of the matrix-free Maxwell operator (implicit_grid.cuh).
 struct OpCoef {
     double K;
