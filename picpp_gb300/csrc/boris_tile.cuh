@@ -672,13 +672,21 @@ __global__ void __launch_bounds__(256) k_push_deposit_deferred(GridP g, SpeciesS
 // periodic images visited in a fixed order (deterministic).  FP32 particles:
 // the partials are 64-bit fixed-point integers, summed exactly and scaled by
 // inv_scale (a power of two) once; FP64 particles: FP64 partials.
-template <typename TP, bool kParts>
+// kWhole: tiles of four or more cells that divide their axis, of which at most
+// two cover a cell.  Finding them is cheap, so a thread takes one component of a
+// cell: on a small box the loads' latency is the time (32^3, 4 partials per tile:
+// 14.8 us with one thread for the three, 8.3 us so; 128^3, bound by the partials'
+// traffic: 82 us, 15 less).  Else every tile is tried that may, once for the
+// three components (100x60x54 in work tiles: 21 us, 40 us one by one).
+template <typename TP, bool kParts, bool kWhole>
 __global__ void __launch_bounds__(256) k_assemble_j(GridP g, TileGeom t, TileShape s, const double* __restrict__ Jpart,
                                                     const double* __restrict__ Jfix, double* __restrict__ J,
                                                     double inv_scale, int nparts) {
     constexpr bool kFixed = sizeof(TP) == sizeof(float);
+    constexpr int kCand = kWhole ? 2 : 16;
     const int parts = kParts ? nparts : 1;
     const long long JC = s.jcells;
+    const int first = kWhole ? blockIdx.y : 0, last = kWhole ? first : 2;   // components
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.N;
          c += (long long)gridDim.x * blockDim.x) {
         int p[3];
@@ -689,53 +697,66 @@ __global__ void __launch_bounds__(256) k_assemble_j(GridP g, TileGeom t, TileSha
         const int je[3] = {s.jx, s.jy, s.jz};
         const int hg[3] = {s.gx, s.gy, s.gz};
         // per axis: every (tile, local index) whose current block holds this
-        // cell or one of its periodic images, in increasing image order
-        constexpr int kCand = 16;
+        // cell or one of its periodic images
         int cand_t[3][kCand], cand_l[3][kCand], cnt[3];
+#pragma unroll
         for (int ax = 0; ax < 3; ++ax) {
-            cnt[ax] = 0;
-            for (int sh = -1; sh <= 1; ++sh) {
-                const int q = p[ax] + sh * n[ax];
-                // block of tile T spans [T*te - hg, T*te - hg + je)
-                int tlo = q + hg[ax] - je[ax] + 1;
-                tlo = tlo >= 0 ? (tlo + te[ax] - 1) / te[ax] : -((-tlo) / te[ax]);
-                int thi = q + hg[ax];
-                thi = thi >= 0 ? thi / te[ax] : -((-thi + te[ax] - 1) / te[ax]);
-                if (tlo < 0) tlo = 0;
-                if (thi > nt[ax] - 1) thi = nt[ax] - 1;
-                for (int T = tlo; T <= thi && cnt[ax] < kCand; ++T) {
-                    cand_t[ax][cnt[ax]] = T;
-                    cand_l[ax][cnt[ax]] = q - (T * te[ax] - hg[ax]);
-                    cnt[ax]++;
+            if constexpr (kWhole) {
+                const int T = p[ax] / te[ax], l = p[ax] - T * te[ax];
+                cand_t[ax][0] = T;
+                cand_l[ax][0] = l + hg[ax];
+                const bool low = l < hg[ax], up = l >= te[ax] - hg[ax];
+                cnt[ax] = low || up ? 2 : 1;
+                cand_t[ax][1] = low ? (T > 0 ? T - 1 : nt[ax] - 1) : (T + 1 < nt[ax] ? T + 1 : 0);
+                cand_l[ax][1] = l + hg[ax] + (low ? te[ax] : -te[ax]);
+            } else {
+                cnt[ax] = 0;
+                for (int sh = -1; sh <= 1; ++sh) {
+                    const int q = p[ax] + sh * n[ax];
+                    // block of tile T spans [T*te - hg, T*te - hg + je)
+                    int tlo = q + hg[ax] - je[ax] + 1;
+                    tlo = tlo >= 0 ? (tlo + te[ax] - 1) / te[ax] : -((-tlo) / te[ax]);
+                    int thi = q + hg[ax];
+                    thi = thi >= 0 ? thi / te[ax] : -((-thi + te[ax] - 1) / te[ax]);
+                    if (tlo < 0) tlo = 0;
+                    if (thi > nt[ax] - 1) thi = nt[ax] - 1;
+                    for (int T = tlo; T <= thi && cnt[ax] < kCand; ++T) {
+                        cand_t[ax][cnt[ax]] = T;
+                        cand_l[ax][cnt[ax]] = q - (T * te[ax] - hg[ax]);
+                        cnt[ax]++;
+                    }
                 }
             }
         }
-        double acc[3] = {Jfix[c], Jfix[g.N + c], Jfix[2 * g.N + c]};
-        long long iacc[3] = {0, 0, 0};
-        for (int a = 0; a < cnt[0]; ++a)
-            for (int b = 0; b < cnt[1]; ++b)
-                for (int d = 0; d < cnt[2]; ++d) {
-                    long long tile = ((long long)cand_t[2][d] * t.nty + cand_t[1][b]) * t.ntx + cand_t[0][a];
-                    long long e = ((long long)cand_l[2][d] * s.jy + cand_l[1][b]) * s.jx + cand_l[0][a];
-                    for (int r = 0; r < parts; ++r) {
-                        const double* src = Jpart + (tile * parts + r) * 3 * JC;
-                        if constexpr (kFixed) {
-                            const long long* srci = reinterpret_cast<const long long*>(src);
-                            iacc[0] += srci[e];
-                            iacc[1] += srci[JC + e];
-                            iacc[2] += srci[2 * JC + e];
-                        } else {
-                            acc[0] += src[e];
-                            acc[1] += src[JC + e];
-                            acc[2] += src[2 * JC + e];
-                        }
-                    }
+        for (int comp = first; comp <= last; ++comp) {
+            double acc = Jfix[comp * g.N + c];
+            long long iacc = 0;
+            auto add = [&](int a, int b, int d) {
+                const long long tile = ((long long)cand_t[2][d] * t.nty + cand_t[1][b]) * t.ntx + cand_t[0][a];
+                const long long e = ((long long)cand_l[2][d] * s.jy + cand_l[1][b]) * s.jx + cand_l[0][a] + comp * JC;
+#pragma unroll 4
+                for (int r = 0; r < parts; ++r) {
+                    const double* src = Jpart + (tile * parts + r) * 3 * JC + e;
+                    if constexpr (kFixed) iacc += *reinterpret_cast<const long long*>(src);
+                    else acc += *src;
                 }
-        if constexpr (kFixed) {
+            };
+            if constexpr (kWhole) {
 #pragma unroll
-            for (int q = 0; q < 3; ++q) acc[q] += (double)iacc[q] * inv_scale;
+                for (int a = 0; a < kCand; ++a)
+#pragma unroll
+                    for (int b = 0; b < kCand; ++b)
+#pragma unroll
+                        for (int d = 0; d < kCand; ++d)
+                            if (a < cnt[0] && b < cnt[1] && d < cnt[2]) add(a, b, d);
+            } else {
+                for (int a = 0; a < cnt[0]; ++a)
+                    for (int b = 0; b < cnt[1]; ++b)
+                        for (int d = 0; d < cnt[2]; ++d) add(a, b, d);
+            }
+            if constexpr (kFixed) acc += (double)iacc * inv_scale;
+            J[comp * g.N + c] = acc;
         }
-        J[c] = acc[0]; J[g.N + c] = acc[1]; J[2 * g.N + c] = acc[2];
     }
 }
 

@@ -88,8 +88,12 @@ float PK<T>::fixed_scale(const GridP& g, const SpeciesSet<T>& S) {
 template <typename T>
 void PK<T>::assemble_j(cudaStream_t s, const GridP& g, const TileGeom& t, const TileShape& sh, const double* Jpart,
                        const double* Jfix, double* J, double inv_scale, int parts) {
-    auto* kernel = parts > 1 ? k_assemble_j<T, true> : k_assemble_j<T, false>;
-    kernel<<<grid_for(g.N, 256), 256, 0, s>>>(g, t, sh, Jpart, Jfix, J, inv_scale, parts);
+    // (an axis of one cell: one tile, no halo)
+    auto whole_axis = [](int n, int te, int nt) { return n == 1 || (te >= 4 && te * nt == n); };
+    const bool whole = whole_axis(g.nx, t.tx, t.ntx) && whole_axis(g.ny, t.ty, t.nty) && whole_axis(g.nz, t.tz, t.ntz);
+    auto* kernel = parts > 1 ? (whole ? k_assemble_j<T, true, true> : k_assemble_j<T, true, false>)
+                             : (whole ? k_assemble_j<T, false, true> : k_assemble_j<T, false, false>);
+    kernel<<<dim3(grid_for(g.N, 256), whole ? 3 : 1), 256, 0, s>>>(g, t, sh, Jpart, Jfix, J, inv_scale, parts);
 }
 
 template <typename T>
