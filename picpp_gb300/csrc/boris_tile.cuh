@@ -686,7 +686,8 @@ __global__ void __launch_bounds__(256) k_assemble_j(GridP g, TileGeom t, TileSha
     constexpr int kCand = kWhole ? 2 : 16;
     const int parts = kParts ? nparts : 1;
     const long long JC = s.jcells;
-    const int first = kWhole ? blockIdx.y : 0, last = kWhole ? first : 2;   // components
+    constexpr int kComp = kWhole ? 1 : 3;        // components of a thread, from the first
+    const int first = kWhole ? blockIdx.y : 0;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.N;
          c += (long long)gridDim.x * blockDim.x) {
         int p[3];
@@ -728,34 +729,40 @@ __global__ void __launch_bounds__(256) k_assemble_j(GridP g, TileGeom t, TileSha
                 }
             }
         }
-        for (int comp = first; comp <= last; ++comp) {
-            double acc = Jfix[comp * g.N + c];
-            long long iacc = 0;
-            auto add = [&](int a, int b, int d) {
-                const long long tile = ((long long)cand_t[2][d] * t.nty + cand_t[1][b]) * t.ntx + cand_t[0][a];
-                const long long e = ((long long)cand_l[2][d] * s.jy + cand_l[1][b]) * s.jx + cand_l[0][a] + comp * JC;
-#pragma unroll 4
-                for (int r = 0; r < parts; ++r) {
-                    const double* src = Jpart + (tile * parts + r) * 3 * JC + e;
-                    if constexpr (kFixed) iacc += *reinterpret_cast<const long long*>(src);
-                    else acc += *src;
+        double acc[kComp];
+        long long iacc[kComp] = {};
+#pragma unroll
+        for (int q = 0; q < kComp; ++q) acc[q] = Jfix[(first + q) * g.N + c];
+        auto add = [&](int a, int b, int d) {
+            const long long tile = ((long long)cand_t[2][d] * t.nty + cand_t[1][b]) * t.ntx + cand_t[0][a];
+            const long long e = ((long long)cand_l[2][d] * s.jy + cand_l[1][b]) * s.jx + cand_l[0][a] + first * JC;
+#pragma unroll(kWhole ? 4 : 1)
+            for (int r = 0; r < parts; ++r) {
+                const double* src = Jpart + (tile * parts + r) * 3 * JC + e;
+#pragma unroll
+                for (int q = 0; q < kComp; ++q) {
+                    if constexpr (kFixed) iacc[q] += *reinterpret_cast<const long long*>(src + q * JC);
+                    else acc[q] += src[q * JC];
                 }
-            };
-            if constexpr (kWhole) {
-#pragma unroll
-                for (int a = 0; a < kCand; ++a)
-#pragma unroll
-                    for (int b = 0; b < kCand; ++b)
-#pragma unroll
-                        for (int d = 0; d < kCand; ++d)
-                            if (a < cnt[0] && b < cnt[1] && d < cnt[2]) add(a, b, d);
-            } else {
-                for (int a = 0; a < cnt[0]; ++a)
-                    for (int b = 0; b < cnt[1]; ++b)
-                        for (int d = 0; d < cnt[2]; ++d) add(a, b, d);
             }
-            if constexpr (kFixed) acc += (double)iacc * inv_scale;
-            J[comp * g.N + c] = acc;
+        };
+        if constexpr (kWhole) {
+#pragma unroll
+            for (int a = 0; a < kCand; ++a)
+#pragma unroll
+                for (int b = 0; b < kCand; ++b)
+#pragma unroll
+                    for (int d = 0; d < kCand; ++d)
+                        if (a < cnt[0] && b < cnt[1] && d < cnt[2]) add(a, b, d);
+        } else {
+            for (int a = 0; a < cnt[0]; ++a)
+                for (int b = 0; b < cnt[1]; ++b)
+                    for (int d = 0; d < cnt[2]; ++d) add(a, b, d);
+        }
+#pragma unroll
+        for (int q = 0; q < kComp; ++q) {
+            if constexpr (kFixed) acc[q] += (double)iacc[q] * inv_scale;
+            J[(first + q) * g.N + c] = acc[q];
         }
     }
 }
