@@ -184,14 +184,11 @@ bool is_buneman(const pic_ctx* c) { return c->cfg.solver == PIC_SOLVER_BUNEMAN; 
 // -------------------------------------------------------------- sort
 template <typename T>
 pic_status sort_species(pic_ctx* ctx, Species& sp) {
-    Phase ph(ctx, PIC_PHASE_SORT, 8);
+    Phase ph(ctx, PIC_PHASE_SORT, 7);
     cudaStream_t s = ctx->s;
     const long long n = sp.n;
-    CK(cudaMemsetAsync(ctx->counts, 0, sizeof(int) * ((size_t)ctx->nkeys + 1), s));
     launch_keys_hist(s, ctx->g, ctx->tg, sp.cell, n, ctx->key, ctx->counts);
-    launch_excl_scan(s, ctx->counts, (long long)ctx->nkeys + 1, ctx->block_sums, nullptr);
-    CK(cudaMemcpyAsync(sp.off, ctx->counts, sizeof(int) * ((size_t)ctx->nkeys + 1), cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(ctx->cursor, ctx->counts, sizeof(int) * (size_t)ctx->nkeys, cudaMemcpyDeviceToDevice, s));
+    launch_offsets(s, ctx->counts, ctx->nkeys, ctx->block_sums, sp.off, ctx->cursor, ctx->long_count);
     launch_scatter_atomic(s, ctx->key, n, ctx->cursor, ctx->tmp);
     launch_segsort(s, sp.off, ctx->nkeys, ctx->tmp, sp.perm, ctx->long_count, ctx->long_list);
     long long kept = n;

@@ -19,12 +19,11 @@ void launch_keys_hist(cudaStream_t s, const GridP& g, const TileGeom& t, const i
     k_keys_hist<<<grid_for(n, 256, 32), 256, 0, s>>>(g, t, cell, n, key, counts);
 }
 
-void launch_excl_scan(cudaStream_t s, int* a, long long n, int* block_sums, int* grand_total) {
-    const long long per = (long long)kScanThreads * kScanItems;
+void launch_offsets(cudaStream_t s, int* counts, int nkeys, int* block_sums, int* off, int* cursor, int* long_count) {
+    const long long n = (long long)nkeys + 1, per = (long long)kScanThreads * kScanItems;
     const int nb = (int)((n + per - 1) / per);
-    k_scan_blocks<<<nb, kScanThreads, 0, s>>>(a, n, block_sums);
-    k_scan_top<<<1, kScanThreads, 0, s>>>(block_sums, nb, grand_total);
-    k_scan_add<<<nb, kScanThreads, 0, s>>>(a, n, block_sums);
+    k_scan_totals<<<nb, kScanThreads, 0, s>>>(counts, n, block_sums);
+    k_scan_offsets<<<nb, kScanThreads, 0, s>>>(counts, n, block_sums, off, cursor, long_count);
 }
 
 void launch_scatter_atomic(cudaStream_t s, const int* key, long long n, int* cursor, int* tmp) {
@@ -34,8 +33,7 @@ void launch_scatter_atomic(cudaStream_t s, const int* key, long long n, int* cur
 
 void launch_segsort(cudaStream_t s, const int* off, int nkeys, const int* tmp, int* perm, int* long_count,
                     int* long_list) {
-    cudaMemsetAsync(long_count, 0, sizeof(int), s);
-    long long warps = nkeys;
+    long long warps = ((long long)nkeys + 1) / 2;
     int blocks = (int)std::min<long long>((warps * 32 + 255) / 256, (long long)kNumSM * 32);
     k_segsort_warp<<<blocks, 256, 0, s>>>(off, nkeys, tmp, perm, long_count, long_list);
     k_segsort_block<<<kNumSM, 1024, 0, s>>>(off, long_list, long_count, tmp, perm);

@@ -109,7 +109,9 @@ void launch_fill(cudaStream_t s, PartView<T> p, long long ppc, unsigned long lon
 // grid.cu
 void launch_keys_hist(cudaStream_t s, const GridP& g, const TileGeom& t, const int* cell, long long n, int* key,
                       int* counts);
-void launch_excl_scan(cudaStream_t s, int* a, long long n, int* block_sums, int* grand_total);
+// offsets of the keys from their counts, to off (nkeys + 1) and cursor; leaves the
+// counts and *long_count (launch_segsort's) at 0
+void launch_offsets(cudaStream_t s, int* counts, int nkeys, int* block_sums, int* off, int* cursor, int* long_count);
 void launch_scatter_atomic(cudaStream_t s, const int* key, long long n, int* cursor, int* tmp);
 void launch_segsort(cudaStream_t s, const int* off, int nkeys, const int* tmp, int* perm, int* long_count,
                     int* long_list);

@@ -6,7 +6,7 @@
 // oracle's stable counting sort:
 //   1. key per particle, histogram (integer atomics per run of equal keys
 //      in a warp: exact counts)
-//   2. exclusive scan of the counts (3-phase block scan)
+//   2. exclusive scan of the counts (block totals, then offsets)
 //   3. scatter of source indices with one atomic cursor per key and run
 //      (arbitrary order inside a key), then
 //   4. per-key segment sort of the source indices by rank counting, which
@@ -84,10 +84,27 @@ __device__ __forceinline__ int block_excl_scan(int v, int* sh, int& total) {
     return warp_off + x - v;
 }
 
-// in-place exclusive scan, phase 1: per-block scan, block totals out.
-__global__ void __launch_bounds__(kScanThreads) k_scan_blocks(int* __restrict__ a, long long n, int* __restrict__ block_sums) {
+// Exclusive scan of the counts, phase 1: the blocks' totals.
+__global__ void __launch_bounds__(kScanThreads) k_scan_totals(const int* __restrict__ a, long long n, int* __restrict__ block_sums) {
     __shared__ int sh[32];
-    long long base = (long long)blockIdx.x * kScanThreads * kScanItems + (long long)threadIdx.x * kScanItems;
+    const long long base = (long long)blockIdx.x * kScanThreads * kScanItems + threadIdx.x;
+    int s = 0;
+#pragma unroll
+    for (int q = 0; q < kScanItems; ++q)
+        if (base + q * kScanThreads < n) s += a[base + q * kScanThreads];
+    int total;
+    block_excl_scan(s, sh, total);
+    if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
+}
+
+// Phase 2: every block adds up the totals before it and scans its own part: the
+// offsets to off, and to cursor but for the last (n entries, n - 1 keys).  Leaves
+// the counts and *zero at 0 for the next sort: that, the copies and a third
+// phase were five more operations of 2 to 6 us each on the stream.
+__global__ void __launch_bounds__(kScanThreads) k_scan_offsets(int* __restrict__ a, long long n, const int* __restrict__ block_sums,
+                                                               int* __restrict__ off, int* __restrict__ cursor, int* __restrict__ zero) {
+    __shared__ int sh[32];
+    const long long base = (long long)blockIdx.x * kScanThreads * kScanItems + (long long)threadIdx.x * kScanItems;
     int v[kScanItems];
     int s = 0;
 #pragma unroll
@@ -95,37 +112,21 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_blocks(int* __restrict__ 
         v[q] = (base + q < n) ? a[base + q] : 0;
         s += v[q];
     }
-    int total;
-    int off = block_excl_scan(s, sh, total);
+    int before = 0, total;
+    for (int b = threadIdx.x; b < (int)blockIdx.x; b += kScanThreads) before += block_sums[b];
+    block_excl_scan(before, sh, total);
+    before = total;
+    int at = before + block_excl_scan(s, sh, total);
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) {
-        if (base + q < n) a[base + q] = off;
-        off += v[q];
+        if (base + q < n) {
+            off[base + q] = at;
+            if (base + q + 1 < n) cursor[base + q] = at;
+            a[base + q] = 0;
+        }
+        at += v[q];
     }
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
-}
-
-// phase 2: exclusive scan of the block totals by one block (any count).
-__global__ void __launch_bounds__(kScanThreads) k_scan_top(int* __restrict__ s, int nb, int* __restrict__ grand_total) {
-    __shared__ int sh[32];
-    int carry = 0;
-    for (int base = 0; base < nb; base += kScanThreads) {
-        int idx = base + threadIdx.x;
-        int v = idx < nb ? s[idx] : 0;
-        int total;
-        int off = block_excl_scan(v, sh, total);
-        if (idx < nb) s[idx] = carry + off;
-        carry += total;
-    }
-    if (threadIdx.x == 0 && grand_total) *grand_total = carry;
-}
-
-// phase 3: add block offsets.
-__global__ void __launch_bounds__(kScanThreads) k_scan_add(int* __restrict__ a, long long n, const int* __restrict__ block_sums) {
-    long long base = (long long)blockIdx.x * kScanThreads * kScanItems;
-    int add = block_sums[blockIdx.x];
-    for (int q = threadIdx.x; q < kScanThreads * kScanItems; q += kScanThreads)
-        if (base + q < n) a[base + q] += add;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *zero = 0;
 }
 
 // Source index a to tmp[cursor[key[a]]++], one atomic per run of equal keys
@@ -204,8 +205,30 @@ __device__ __forceinline__ void warp_sort_segment(const int* __restrict__ tmp, i
         if (32 * r + lane < len) perm[b + 32 * r + lane] = v[r];
 }
 
+// Two segments of at most 16 elements, one per half warp: this lane's segment
+// [b, b + len).
+__device__ __forceinline__ void half_sort_segments(const int* __restrict__ tmp, int* __restrict__ perm, int b, int len,
+                                                   int lane) {
+    const int l = lane & 15;
+    int v = l < len ? tmp[b + l] : INT_MAX;
+    const int next = __shfl_down_sync(0xffffffffu, v, 1, 16);
+    if (!__all_sync(0xffffffffu, l + 1 >= len || v <= next)) {
+#pragma unroll
+        for (int k = 2; k <= 16; k <<= 1)
+#pragma unroll
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                const int y = __shfl_xor_sync(0xffffffffu, v, j);
+                const bool up = (l & k) == 0, lower = (l & j) == 0;
+                v = lower == up ? min(v, y) : max(v, y);
+            }
+    }
+    if (l < len) perm[b + l] = v;
+}
+
 // Stable order of each key segment [off[k], off[k+1]) of tmp into perm
-// (ascending source index).  Segments up to kWarpSeg elements use one warp;
+// (ascending source index).  Segments up to kWarpSeg elements use one warp,
+// two neighbours of up to 16 elements a half each (128^3, 16 per species and
+// cell, bound by the latency of each warp's few loads: 339 -> 192 us per species);
 // longer ones are left to k_segsort_block.
 constexpr int kWarpSeg = 256;
 __global__ void k_segsort_warp(const int* __restrict__ off, int nkeys, const int* __restrict__ tmp, int* __restrict__ perm,
@@ -213,19 +236,29 @@ __global__ void k_segsort_warp(const int* __restrict__ off, int nkeys, const int
     const int lane = threadIdx.x & 31;
     const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long kk = warp; kk < nkeys; kk += nwarps) {
-        int b = off[kk], e = off[kk + 1];
-        int len = e - b;
-        if (len <= 0) continue;
-        if (len == 1) { if (lane == 0) perm[b] = tmp[b]; continue; }
-        if (len > kWarpSeg) {
-            if (lane == 0) { int slot = atomicAdd(long_count, 1); long_list[slot] = (int)kk; }
+    for (long long k0 = 2 * warp; k0 < nkeys; k0 += 2 * nwarps) {
+        const bool two = k0 + 1 < nkeys;
+        const int o0 = off[k0], o1 = off[k0 + 1], o2 = two ? off[k0 + 2] : o1;
+        if (o1 - o0 <= 16 && o2 - o1 <= 16) {
+            if (o2 > o0) half_sort_segments(tmp, perm, lane < 16 ? o0 : o1, lane < 16 ? o1 - o0 : o2 - o1, lane);
             continue;
         }
-        if (len <= 32) warp_sort_segment<1>(tmp, perm, b, len, lane);
-        else if (len <= 64) warp_sort_segment<2>(tmp, perm, b, len, lane);
-        else if (len <= 128) warp_sort_segment<4>(tmp, perm, b, len, lane);
-        else warp_sort_segment<8>(tmp, perm, b, len, lane);
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+            const int b = h ? o1 : o0, len = (h ? o2 : o1) - b;
+            if (len <= 0) continue;
+            if (len > kWarpSeg) {
+                if (lane == 0) { int slot = atomicAdd(long_count, 1); long_list[slot] = (int)k0 + h; }
+            } else if (len <= 32) {
+                warp_sort_segment<1>(tmp, perm, b, len, lane);
+            } else if (len <= 64) {
+                warp_sort_segment<2>(tmp, perm, b, len, lane);
+            } else if (len <= 128) {
+                warp_sort_segment<4>(tmp, perm, b, len, lane);
+            } else {
+                warp_sort_segment<8>(tmp, perm, b, len, lane);
+            }
+        }
     }
 }
 
