@@ -63,10 +63,15 @@ __device__ __forceinline__ bool local_axis(int c, int x0, int t, int h, int n, i
     return false;
 }
 
-// Weights of the eight corners (x fastest) from the upper weight of each axis.
-template <typename T>
+// Weights of the eight corners (x fastest) from the upper weight of each axis;
+// kFlat: the four of a box of one cell along z (wz is 0).
+template <typename T, bool kFlat = false>
 __device__ __forceinline__ void corners(T wx, T wy, T wz, T w[8]) {
     const T ux = T(1) - wx, uy = T(1) - wy, uz = T(1) - wz;
+    if constexpr (kFlat) {
+        w[0] = ux * uy; w[1] = wx * uy; w[2] = ux * wy; w[3] = wx * wy;
+        return;
+    }
     const T yz[4] = {uy * uz, wy * uz, uy * wz, wy * wz};
 #pragma unroll
     for (int q = 0; q < 4; ++q) { w[2 * q] = ux * yz[q]; w[2 * q + 1] = wx * yz[q]; }
@@ -75,7 +80,7 @@ __device__ __forceinline__ void corners(T wx, T wy, T wz, T w[8]) {
 // and 24 multiply-adds; nested interpolations are 14 operations per component): from three planes of a staged block, `plane`
 // entries apart, or from a block of float4 nodes or cells (x, y, z, unused),
 // one 16-byte load per corner.
-template <typename T>
+template <typename T, bool kFlat = false>
 __device__ __forceinline__ void gather3(const T* __restrict__ F, int plane, int base, int sx, int sy, int sz,
                                         const T w[8], T out[3]) {
 #pragma unroll
@@ -85,6 +90,10 @@ __device__ __forceinline__ void gather3(const T* __restrict__ F, int plane, int 
         v = fma(w[1], f[sx], v);
         v = fma(w[2], f[sy], v);
         v = fma(w[3], f[sy + sx], v);
+        if constexpr (kFlat) {
+            out[q] = v;
+            continue;
+        }
         v = fma(w[4], f[sz], v);
         v = fma(w[5], f[sz + sx], v);
         v = fma(w[6], f[sz + sy], v);
@@ -350,35 +359,40 @@ __device__ __noinline__ EB6<T> gather_eb_global(const GridP g, int i, int j, int
 
 // The run sums of the lanes `me` (one stencil base) with FP64 accumulators: a
 // butterfly per 32 products, one shared atomic per lane and pass.
-template <typename A, typename T>
+// kFlat (one cell along z): 4 corners and 9 slots, 4 passes instead of 9.
+template <typename A, typename T, bool kFlat = false>
 __device__ __forceinline__ void butterfly_sums(const T row[kScrRow], bool me, double cq, double cm, A* __restrict__ sN,
                                                A* __restrict__ sC, int NB, int CB, int nb, int cb, int oxn, int oyn,
                                                int ozn, int oxc, int oyc, int ozc, int lane) {
     A QN[12], QC[7], wn[8], wc[27];
     run_quantities<A, T>(row, cq, cm, QN, QC);
     run_weights<A, T>(row, wn, wc);
+    constexpr int NC = kFlat ? 4 : 8, NS = kFlat ? 9 : 27, Z = kFlat ? 9 : 0;   // corners, slots (of z slot 1), first slot
     A vv[32];
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
+    for (int r = 0; r < (12 * NC + 31) / 32; ++r) {
 #pragma unroll
-        for (int x = 0; x < 32; ++x) vv[x] = me ? QN[4 * r + x / 8] * wn[x % 8] : A(0);
+        for (int x = 0; x < 32; ++x) {
+            const int idx = 32 * r + x;
+            vv[x] = (idx < 12 * NC && me) ? QN[idx / NC] * wn[idx % NC] : A(0);
+        }
         const A sum = xpose_sum<A>(vv, lane);
-        const int q = 4 * r + lane / 8, c = lane % 8;
-        if (sum != A(0))
+        const int idx = 32 * r + lane, q = idx / NC, c = idx % NC;
+        if (idx < 12 * NC && sum != A(0))
             atomicAdd(&sN[q * NB + nb + (c & 1) * oxn + ((c >> 1) & 1) * oyn + (c >> 2) * ozn],
                       sum);
     }
 #pragma unroll
-    for (int r = 0; r < 6; ++r) {
+    for (int r = 0; r < (7 * NS + 31) / 32; ++r) {
 #pragma unroll
         for (int x = 0; x < 32; ++x) {
             const int idx = 32 * r + x;
-            vv[x] = (idx < 189 && me) ? QC[idx / 27] * wc[idx % 27] : A(0);
+            vv[x] = (idx < 7 * NS && me) ? QC[idx / NS] * wc[Z + idx % NS] : A(0);
         }
         const A sum = xpose_sum<A>(vv, lane);
         const int idx = 32 * r + lane;
-        if (idx < 189 && sum != A(0)) {
-            const int q = idx / 27, sl = idx % 27;
+        if (idx < 7 * NS && sum != A(0)) {
+            const int q = idx / NS, sl = idx % NS;
             atomicAdd(&sC[q * CB + cb + (sl % 3) * oxc + ((sl / 3) % 3) * oyc + (sl / 9) * ozc],
                       sum);
         }
@@ -422,7 +436,9 @@ struct DepositSet {
 // which two fit on an SM (deposit_boxes, api.cu), some a cell smaller than
 // others (box_start); they need not follow the sort's tiles o, a cell's particles being found by
 // its key.  Not staged: t holds the sort's tiles.
-template <typename T, typename A, bool kStaged>
+// kFlat (FP64, one cell along z): without the corners and slots that weigh 0;
+// the FP64 pipe is what bounds it (pairs of 32x32x1: 192 -> 117 us).
+template <typename T, typename A, bool kStaged, bool kFlat>
 __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(GridP g, TileGeom t, TileGeom o, ImpBlock bk,
                                                                        const __grid_constant__ ImpSpecies<T> S,
                                                                        const __grid_constant__ DepositSet<T> K,
@@ -549,15 +565,15 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
                     T e[3], bf[3];
                     if (mine) {
                         T w[8];
-                        corners<T>(nw[1], nw[3], nw[5], w);
+                        corners<T, kFlat>(nw[1], nw[3], nw[5], w);
                         if constexpr (kVec) gather3(sE4, nbK, oxn, oyn, ozn, w, e);
-                        else gather3<T>(sE, bk.NB, nbK, oxn, oyn, ozn, w, e);
+                        else gather3<T, kFlat>(sE, bk.NB, nbK, oxn, oyn, ozn, w, e);
                         // cell pair (c - 1, c) below the centre, (c, c + 1) above
                         const bool bx = ox < T(0.5), by = oy < T(0.5), bz = oz < T(0.5);
-                        corners<T>(bx ? cw[1] : cw[2], by ? cw[4] : cw[5], bz ? cw[7] : cw[8], w);
+                        corners<T, kFlat>(bx ? cw[1] : cw[2], by ? cw[4] : cw[5], bz ? cw[7] : cw[8], w);
                         const int cbase = cbK + (bx ? 0 : oxc) + (by ? 0 : oyc) + (bz ? 0 : ozc);
                         if constexpr (kVec) gather3(sB4, cbase, oxc, oyc, ozc, w, bf);
-                        else gather3<T>(sB, bk.CB, cbase, oxc, oyc, ozc, w, bf);
+                        else gather3<T, kFlat>(sB, bk.CB, cbase, oxc, oyc, ozc, w, bf);
                     } else {
                         int i, j, k;
                         decode(g, cell, i, j, k);
@@ -589,7 +605,7 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
                         for (int q = 0; q < 8; ++q) ac[q] = 0.f;
                     }
                 } else if (__popc(mm) >= kXposeMin) {
-                    butterfly_sums<A, T>(row, mine, cq, cm, sN, sC, bk.NB, bk.CB, nbK, cbK, oxn, oyn, ozn, oxc, oyc, ozc,
+                    butterfly_sums<A, T, kFlat>(row, mine, cq, cm, sN, sC, bk.NB, bk.CB, nbK, cbK, oxn, oyn, ozn, oxc, oyc, ozc,
                                          lane);
                 } else if (mine) {
                     imp_deposit_direct<A, T>(row, cq, cm, sN, sC, bk.NB, bk.CB, nbK, cbK, oxn, oyn, ozn, oxc, oyc, ozc);
@@ -802,7 +818,9 @@ struct MoverSet {
 // FP32 beams of 39x57x53 (tiles of one cell), 60 per species and cell: 3,170 ->
 // 802 us; shock of 112x51x5: 192 -> 135 us; FP64 pairs of 61x43x1: 525 -> 413 us;
 // of 32x32x1, 32 per species and cell (whole tiles, 19 CTAs each): 207 -> 108 us.
-template <typename T, bool kWall, bool kRows>
+// kFlat (FP64, one cell along z): gathers from four corners, where eight keep the
+// FP64 pipe busy with weights of 0 (32x32x1: 108 -> 82 us).
+template <typename T, bool kWall, bool kRows, bool kFlat>
 __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g, TileGeom t, TileGeom o, MoverBlock mb,
                                                             const __grid_constant__ ImpSpecies<T> S,
                                                             const __grid_constant__ MoverSet<T> K,
@@ -934,13 +952,13 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
             // (nodes, corner weights w) and B^n (cells), float4 blocks for FP32
             auto gatEt = [&](const Loc& L, const T w[8], T out[3]) {
                 if constexpr (kVec) gather3(sEt4, L.nbase, nsx, nsy, nsz, w, out);
-                else gather3<T>(sEt, mb.NB, L.nbase, nsx, nsy, nsz, w, out);
+                else gather3<T, kFlat>(sEt, mb.NB, L.nbase, nsx, nsy, nsz, w, out);
             };
             auto gatB = [&](const Loc& L, T out[3]) {
                 T w[8];
-                corners<T>(L.wc[0], L.wc[1], L.wc[2], w);
+                corners<T, kFlat>(L.wc[0], L.wc[1], L.wc[2], w);
                 if constexpr (kVec) gather3(sB4, L.cbase, csx, csy, csz, w, out);
-                else gather3<T>(sB, mb.CB, L.cbase, csx, csy, csz, w, out);
+                else gather3<T, kFlat>(sB, mb.CB, L.cbase, csx, csy, csz, w, out);
             };
             auto defer = [&]() { atomicOr(&S.defer[s][n >> 5], 1u << (n & 31)); };
             T u0[3] = {pu[0], pu[1], pu[2]};
@@ -957,8 +975,8 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
             }
             {
                 T w[8];
-                corners<T>(L0.wn[0], L0.wn[1], L0.wn[2], w);
-                gather3<T>(sE, mb.NB, L0.nbase, nsx, nsy, nsz, w, e0);
+                corners<T, kFlat>(L0.wn[0], L0.wn[1], L0.wn[2], w);
+                gather3<T, kFlat>(sE, mb.NB, L0.nbase, nsx, nsy, nsz, w, e0);
                 gatEt(L0, w, e);
             }
             gatB(L0, b);
@@ -1035,7 +1053,7 @@ __global__ void __launch_bounds__(kMoverThreads, 2) k_implicit_push_tile(GridP g
                 }
                 {
                     T w[8];
-                    corners<T>(L1.wn[0], L1.wn[1], L1.wn[2], w);
+                    corners<T, kFlat>(L1.wn[0], L1.wn[1], L1.wn[2], w);
                     gatEt(L1, w, e);
                 }
                 gatB(L1, b);

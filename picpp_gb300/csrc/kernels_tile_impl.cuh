@@ -130,9 +130,11 @@ template <typename T>
 void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileGeom& o, const ImpBlock& bk,
                                    const ImpSpecies<T>& S, const T* E, const T* B, double* J, double* mu,
                                    double* rho, double* Pi) {
+    constexpr bool kF64 = sizeof(T) == sizeof(double);   // its kernels for boxes of one cell along z
     static bool attr_set = false;
     if (!attr_set) {
-        for (auto* k : {k_implicit_deposit_tile<T, T, true>, k_implicit_deposit_tile<T, T, false>})
+        for (auto* k : {k_implicit_deposit_tile<T, T, true, false>, k_implicit_deposit_tile<T, T, true, kF64>,
+                        k_implicit_deposit_tile<T, T, false, false>})
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         attr_set = true;
     }
@@ -141,7 +143,8 @@ void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeo
     const int ntiles = t.ntx * t.nty * t.ntz;
     const int grid = ntiles < kNumSM * (per_sm > 0 ? per_sm : 1) ? ntiles : kNumSM * (per_sm > 0 ? per_sm : 1);
     constexpr int nt = imp_threads<T>();
-    auto* kernel = bk.stage ? k_implicit_deposit_tile<T, T, true> : k_implicit_deposit_tile<T, T, false>;
+    auto* kernel = !bk.stage ? k_implicit_deposit_tile<T, T, false, false>
+                   : g.z3    ? k_implicit_deposit_tile<T, T, true, false> : k_implicit_deposit_tile<T, T, true, kF64>;
     const double PI_D = 3.14159265358979323846;
     const double ivol = 1.0 / (g.dx * g.dy * g.dz);
     DepositSet<T> K{};
@@ -157,6 +160,7 @@ void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeo
 template <typename T>
 bool PK<T>::implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileGeom& o, const ImpSpecies<T>& S,
                                 const double* E, const double* B, const double* Et) {
+    constexpr bool kF64 = sizeof(T) == sizeof(double);   // its kernels for boxes of one cell along z
     MoverBlock mb{};
     const int H = kMoverHalo;
     mb.nbx = g.nx > 1 ? t.tx + 2 * H + 1 : 1;
@@ -197,8 +201,9 @@ bool PK<T>::implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& 
     const size_t smem = rows ? most_smem : whole;
     static bool attr_set = false;
     if (!attr_set) {
-        for (auto* k : {k_implicit_push_tile<T, false, false>, k_implicit_push_tile<T, false, true>,
-                        k_implicit_push_tile<T, true, false>, k_implicit_push_tile<T, true, true>})
+        for (auto* k : {k_implicit_push_tile<T, false, false, false>, k_implicit_push_tile<T, false, true, false>,
+                        k_implicit_push_tile<T, false, false, kF64>, k_implicit_push_tile<T, false, true, kF64>,
+                        k_implicit_push_tile<T, true, false, false>, k_implicit_push_tile<T, true, true, false>})
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         attr_set = true;
     }
@@ -210,8 +215,9 @@ bool PK<T>::implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& 
     for (int q = 0; q < S.ns; ++q) words = std::max(words, (S.p[q].n + 31) / 32);
     // the wall rules are a separate instantiation: the periodic mover keeps
     // none of their code in its loop
-    auto* kernel = g.wall ? (rows ? k_implicit_push_tile<T, true, true> : k_implicit_push_tile<T, true, false>)
-                          : (rows ? k_implicit_push_tile<T, false, true> : k_implicit_push_tile<T, false, false>);
+    auto* kernel = g.wall ? (rows ? k_implicit_push_tile<T, true, true, false> : k_implicit_push_tile<T, true, false, false>)
+                   : g.z3 ? (rows ? k_implicit_push_tile<T, false, true, false> : k_implicit_push_tile<T, false, false, false>)
+                          : (rows ? k_implicit_push_tile<T, false, true, kF64> : k_implicit_push_tile<T, false, false, kF64>);
     MoverSet<T> K{};
     K.dt = T(g.dt); K.eta = T(g.eta); K.edt = T(g.eta * g.dt); K.redt = T((1.0 - g.eta) * g.dt);
     K.dx2 = T(g.dx) * T(g.dx);
