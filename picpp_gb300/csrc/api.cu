@@ -400,12 +400,16 @@ pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
 // over the SMs leaves at most a fifth of the time idle.  Boxes of 32 cells (FP64,
 // whose particles take longer: 4) are not cut for that: each flushes a block of
 // its own (the pairs plane of 32x32x1, FP64: 1.73 ms in 16 boxes, 0.34 ms in
-// 256, where it is 0.20 ms by now, 0.5 ms in 1024).  They do not follow the sort's tiles, which are single
-// cells along an odd axis: FP32 beams of 39x57x53, 60 per species and cell,
-// deposit in 0.98 ms, tile by tile in 5.03 ms; 112x51x5 shock 0.18 against
-// 0.24 ms (0.29 ms with 182 boxes, uncut); pairs of 61x43x1 0.70 against 1.31 ms.
+// 256, where it is 0.12 ms by now, 0.5 ms in 1024).  They do not follow the
+// sort's tiles, which are single cells along an odd axis: FP32 beams of 39x57x53, 60 per species and cell,
+// deposit in 0.98 ms, tile by tile in 5.03 ms; FP64 pairs of 61x43x1 in 0.33
+// against 1.31 ms.  FP32 particles take boxes of several tiles only where a tile
+// has fewer cells than a CTA has warps: across tiles their sums have to meet in
+// FP64 accumulators, whose adds cost more than small tiles that keep every warp
+// busy (50x53x8, tiles of 2x1x8, 13 per species: 92 us, 135 us in boxes; shock of
+// 112x51x5, tiles of 8x1x1: 235 and 240 us).
 template <typename T>
-TileGeom deposit_boxes(const GridP& g, int ns) {
+TileGeom deposit_boxes(const GridP& g, const TileGeom& t, int ns, ImpBlock& bk) {
     const int n[3] = {g.nx, g.ny, g.nz};
     int m[3], e[3];
     auto even = [&](int a, int most) {
@@ -413,9 +417,14 @@ TileGeom deposit_boxes(const GridP& g, int ns) {
         e[a] = (n[a] + m[a] - 1) / m[a];
     };
     for (int a = 0; a < 3; ++a) even(a, 8);
+    const int tile[3] = {t.tx, t.ty, t.tz}, cells = t.tx * t.ty * t.tz;
+    if (sizeof(T) == 4 && cells >= 8 && cells <= 512)
+        for (int a = 0; a < 3; ++a) { e[a] = tile[a]; m[a] = n[a] / tile[a]; }
     for (;;) {
         TileGeom w{e[0], e[1], e[2], m[0], m[1], m[2], -1, -1, -1};
-        ImpBlock bk = PK<T>::implicit_block(g, w, 0);
+        // FP32 sums of several of the sort's tiles meet in FP64, as in the grids
+        const bool wide = sizeof(T) == 4 && (e[0] > t.tx || e[1] > t.ty || e[2] > t.tz);
+        bk = PK<T>::implicit_block(g, w, 0, wide);
         bk.stage = 1;
         const bool fits = PK<T>::implicit_tile_smem(bk, e[0] * e[1] * e[2], ns) <= (size_t)(227 * 1024) / 2 - 1024;
         int a = 2;
@@ -446,9 +455,8 @@ pic_status implicit_moments(pic_ctx* ctx) {
     // staged next to the accumulators; otherwise a one-cell halo for drift
     // (staged: over boxes of cells, deposit_boxes)
     const int ns = (int)ctx->sp.size();
-    TileGeom wt = deposit_boxes<T>(g, ns);
-    ImpBlock bk = PK<T>::implicit_block(g, wt, 0);
-    bk.stage = 1;
+    ImpBlock bk;
+    TileGeom wt = deposit_boxes<T>(g, ctx->tg, ns, bk);
     if (!ctx->fresh_sort || PK<T>::implicit_tile_smem(bk, wt.tx * wt.ty * wt.tz, ns) > 227 * 1024) {
         wt = ctx->tg;
         bk = PK<T>::implicit_block(g, ctx->tg, 1);

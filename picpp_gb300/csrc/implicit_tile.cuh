@@ -233,7 +233,8 @@ __device__ __forceinline__ void tc_run_sums(float* __restrict__ scr, int lane, b
 
 // Adds the run sums of tc_run_sums (lane layout as there) to the shared
 // blocks at node base nb and cell base cb, times the species factors.
-__device__ __forceinline__ void add_run_sums(float* __restrict__ sN, float* __restrict__ sC, int NB, int CB, int nb,
+template <typename A>
+__device__ __forceinline__ void add_run_sums(A* __restrict__ sN, A* __restrict__ sC, int NB, int CB, int nb,
                                              int cb, int oxn, int oyn, int ozn, int oxc, int oyc, int ozc, int lane,
                                              const float dn[4], const float dc[8], float cq, float cm) {
     const int gq = lane >> 2, tq = lane & 3;
@@ -241,13 +242,13 @@ __device__ __forceinline__ void add_run_sums(float* __restrict__ sN, float* __re
     for (int i = 0; i < 4; ++i) {
         const int q = gq + 8 * (i >> 1), c = 2 * tq + (i & 1);
         if (q < 12 && dn[i] != 0.f)
-            atomicAdd(&sN[q * NB + nb + (c & 1) * oxn + ((c >> 1) & 1) * oyn + (c >> 2) * ozn], dn[i] * (q < 3 ? cq : cm));
+            atomicAdd(&sN[q * NB + nb + (c & 1) * oxn + ((c >> 1) & 1) * oyn + (c >> 2) * ozn], A(dn[i] * (q < 3 ? cq : cm)));
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int sl = 16 * (i >> 2) + gq + 8 * ((i >> 1) & 1), q = 2 * tq + (i & 1);
         if (sl < 27 && q < 7 && dc[i] != 0.f)
-            atomicAdd(&sC[q * CB + cb + (sl % 3) * oxc + ((sl / 3) % 3) * oyc + (sl / 9) * ozc], dc[i] * cq);
+            atomicAdd(&sC[q * CB + cb + (sl % 3) * oxc + ((sl / 3) % 3) * oyc + (sl / 9) * ozc], A(dc[i] * cq));
     }
 }
 
@@ -436,6 +437,10 @@ struct DepositSet {
 // which two fit on an SM (deposit_boxes, api.cu), some a cell smaller than
 // others (box_start); they need not follow the sort's tiles o, a cell's particles being found by
 // its key.  Not staged: t holds the sort's tiles.
+// A: FP64 too for FP32 particles in a box of several of the sort's tiles: the
+// tiles' sums met in the FP64 grids before, and so they still do (39x27x23, 60
+// per species and cell: E after a step 8.5e-7 from 64 bits, with FP32
+// accumulators 1.1e-6; 39x57x53: 985 us, with FP32 ones 846 us).
 // kFlat (FP64, one cell along z): without the corners and slots that weigh 0;
 // the FP64 pipe is what bounds it (pairs of 32x32x1: 192 -> 117 us).
 template <typename T, typename A, bool kStaged, bool kFlat>
@@ -466,7 +471,7 @@ __global__ void __launch_bounds__(imp_threads<T>(), 2) k_implicit_deposit_tile(G
     const int oxn = ax ? 1 : 0, oyn = ay ? nsy : 0, ozn = az ? nsz : 0;   // corner strides
     const int oxc = ax ? 1 : 0, oyc = ay ? csy : 0, ozc = az ? csz : 0;   // slot strides
     const int tot = 12 * bk.NB + 7 * bk.CB;
-    constexpr bool kTc = sizeof(A) == sizeof(float);   // FP32 accumulators: tensor-core run sums
+    constexpr bool kTc = sizeof(T) == sizeof(float);   // FP32 particles: tensor-core run sums
     unsigned char* after = imp_smem + bk.scratch_at();
     float* scr0 = reinterpret_cast<float*>(after);
     float* scr = scr0 + warp * (kScrParticles * kScrRow);

@@ -74,7 +74,7 @@ struct PK {
                                  int compat, const GhostAxes& ga);
     // tiled deposit (implicit_tile.cuh), periodic pressure placement; needs
     // tile-major sorted particles
-    static ImpBlock implicit_block(const GridP& g, const TileGeom& t, int h);
+    static ImpBlock implicit_block(const GridP& g, const TileGeom& t, int h, bool wide = false);   // wide: FP64 accumulators
     static size_t implicit_tile_smem(const ImpBlock& bk, int cells, int ns);   // cells per tile or box, species
     static void implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileGeom& o,
                                        const ImpBlock& bk,

@@ -8,7 +8,7 @@ template void PK<double>::push_deposit_tiled(cudaStream_t, const GridP&, const T
 template float PK<double>::fixed_scale(const GridP&, const SpeciesSet<double>&);
 template void PK<double>::assemble_j(cudaStream_t, const GridP&, const TileGeom&, const TileShape&, const double*,
                                      const double*, double*, double, int);
-template ImpBlock PK<double>::implicit_block(const GridP&, const TileGeom&, int);
+template ImpBlock PK<double>::implicit_block(const GridP&, const TileGeom&, int, bool);
 template size_t PK<double>::implicit_tile_smem(const ImpBlock&, int, int);
 template void PK<double>::implicit_deposit_tiled(cudaStream_t, const GridP&, const TileGeom&, const TileGeom&,
                                                  const ImpBlock&, const ImpSpecies<double>&, const double*, const double*,

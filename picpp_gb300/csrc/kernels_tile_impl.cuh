@@ -99,10 +99,11 @@ void PK<T>::assemble_j(cudaStream_t s, const GridP& g, const TileGeom& t, const 
 }
 
 template <typename T>
-ImpBlock PK<T>::implicit_block(const GridP& g, const TileGeom& t, int h) {
+ImpBlock PK<T>::implicit_block(const GridP& g, const TileGeom& t, int h, bool wide) {
     ImpBlock b{};
     b.h = h;
-    b.areal = sizeof(T);
+    b.areal = wide ? sizeof(double) : sizeof(T);
+    b.field = sizeof(T) == sizeof(float) ? sizeof(float4) : 3 * sizeof(double);
     b.nbx = g.nx > 1 ? t.tx + 2 * h + 1 : 1;
     b.nby = g.y3 ? t.ty + 2 * h + 1 : 1;
     b.nbz = g.z3 ? t.tz + 2 * h + 1 : 1;
@@ -133,8 +134,8 @@ void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeo
     constexpr bool kF64 = sizeof(T) == sizeof(double);   // its kernels for boxes of one cell along z
     static bool attr_set = false;
     if (!attr_set) {
-        for (auto* k : {k_implicit_deposit_tile<T, T, true, false>, k_implicit_deposit_tile<T, T, true, kF64>,
-                        k_implicit_deposit_tile<T, T, false, false>})
+        for (auto* k : {k_implicit_deposit_tile<T, T, true, false>, k_implicit_deposit_tile<T, double, true, false>,
+                        k_implicit_deposit_tile<T, T, true, kF64>, k_implicit_deposit_tile<T, T, false, false>})
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         attr_set = true;
     }
@@ -143,8 +144,10 @@ void PK<T>::implicit_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeo
     const int ntiles = t.ntx * t.nty * t.ntz;
     const int grid = ntiles < kNumSM * (per_sm > 0 ? per_sm : 1) ? ntiles : kNumSM * (per_sm > 0 ? per_sm : 1);
     constexpr int nt = imp_threads<T>();
-    auto* kernel = !bk.stage ? k_implicit_deposit_tile<T, T, false, false>
-                   : g.z3    ? k_implicit_deposit_tile<T, T, true, false> : k_implicit_deposit_tile<T, T, true, kF64>;
+    const bool wide = bk.areal > (int)sizeof(T);
+    auto* kernel = !bk.stage      ? k_implicit_deposit_tile<T, T, false, false>
+                   : wide         ? k_implicit_deposit_tile<T, double, true, false>
+                   : g.z3         ? k_implicit_deposit_tile<T, T, true, false> : k_implicit_deposit_tile<T, T, true, kF64>;
     const double PI_D = 3.14159265358979323846;
     const double ivol = 1.0 / (g.dx * g.dy * g.dz);
     DepositSet<T> K{};

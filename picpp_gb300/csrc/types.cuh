@@ -82,12 +82,12 @@ struct ImpBlock {
     int nbx, nby, nbz, NB;
     int cbx, cby, cbz, CB;
     int stage;   // 1: E (node block) and B (cell block) staged in shared memory too (h = 0 only)
-    int areal;   // bytes of an accumulator (and of a staged plane's value)
+    int areal, field;   // bytes of an accumulator, and of a staged node's or cell's three components
     // byte offsets in shared memory: 12 NB + 7 CB accumulators, the staged
     // fields (FP32 float4, FP64 three planes), then the warps' scratch
     __host__ __device__ size_t stage_at() const { return ((size_t)(12 * NB + 7 * CB) * areal + 15) & ~size_t(15); }
     __host__ __device__ size_t scratch_at() const {
-        return stage_at() + (stage ? (size_t)(NB + CB) * (areal == 4 ? 16 : 24) : 0);
+        return stage_at() + (stage ? (size_t)(NB + CB) * field : 0);
     }
 };
 
