@@ -1,5 +1,7 @@
 // boris_tile.cuh -- fused gather + Boris push + zigzag deposit, one CTA per
-// tile of cells (the whole-step path of the explicit Buneman/Tristan solver).
+// tile of cells (the whole-step path of the explicit Buneman/Tristan solver); in
+// small boxes several CTAs share a tile, along axes that 8 does not divide a CTA
+// takes a work tile made of several (kParts, kMerge).
 //
 // Particles are ordered by a tile-major cell key (sort.cuh), so tile t owns
 // the contiguous range [off[t*T3], off[(t+1)*T3]) of every species.  A CTA

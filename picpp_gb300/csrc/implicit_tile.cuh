@@ -3,7 +3,8 @@
 // 365-584, with the pressure tensor at the particle's own cells).
 //
 // Particles are ordered by the tile-major cell key (sort.cuh).  One CTA owns
-// a tile and accumulates, in shared memory,
+// a tile (right after a sort: a box of cells of its own) and accumulates, in
+// shared memory,
 //   * on nodes (tile + h halo + 1):  J-hat (3) and mu (9), 8 nodes/particle;
 //   * on cells (tile + h halo + 2):  rho-hat (1) and Pi (6 of the symmetric
 //     9), 8 of the 27 cells around the particle's cell.
@@ -11,8 +12,8 @@
 // Lanes holding the same (current) cell share one stencil base, so their
 // 96 node and 189 cell products (27 slots, zero weight outside the
 // particle's octant) are summed over the run before one shared-memory atomic
-// per sum: with FP32 accumulators as small TF32 tensor-core products at FP32
-// accuracy (tc_run_sums), with FP64 accumulators by a butterfly
+// per sum: FP32 particles as small TF32 tensor-core products at FP32
+// accuracy (tc_run_sums), FP64 ones by a butterfly
 // transpose-reduction (after five exchange rounds lane L holds the warp total
 // of product L of a 32-product pass).  Runs of only a few lanes add their
 // products directly; particles more than h cells
