@@ -101,20 +101,35 @@ __device__ __forceinline__ void gather3(const T* __restrict__ F, int plane, int 
         out[q] = fma(w[7], f[sz + sy + sx], v);
     }
 }
+// (x, y) in one packed FP32 multiply-add, z (and the unused fourth) in another:
+// the FP32 mover, bound by instruction issue, 448 -> 428 us at 64x64x16.
+__device__ __forceinline__ unsigned long long twice(float a) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+    return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ void split2(unsigned long long p, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p));
+}
 __device__ __forceinline__ void gather3(const float4* __restrict__ F, int base, int sx, int sy, int sz, const float w[8],
                                         float out[3]) {
-    const float4* f = F + base;
+    const ulonglong2* f = reinterpret_cast<const ulonglong2*>(F + base);
     const int at[8] = {0, sx, sy, sy + sx, sz, sz + sx, sz + sy, sz + sy + sx};
-    out[0] = out[1] = out[2] = 0.f;
+    unsigned long long xy = 0, z = 0;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-        const float4 v = f[at[q]];
-        out[0] = fmaf(w[q], v.x, out[0]);
-        out[1] = fmaf(w[q], v.y, out[1]);
-        out[2] = fmaf(w[q], v.z, out[2]);
+        const ulonglong2 v = f[at[q]];
+        const unsigned long long ww = twice(w[q]);
+        fma2(xy, ww, v.x);
+        fma2(z, ww, v.y);
     }
+    float none;
+    split2(xy, out[0], out[1]);
+    split2(z, out[2], none);
 }
-
 // ---- tensor-core reduction of one run (FP32 accumulators) -------------------
 // The 96 node sums  N[q][c] = sum_p QN_p[q] wn_p[c]  and 189 cell sums
 // C[s][q] = sum_p wc_p[s] QC_p[q]  of a run of particles are small matrix
@@ -814,16 +829,16 @@ struct MoverSet {
 // FP64 grids (the kernel itself calls nothing out of line, which would cost
 // its hot loop register spills).  Same arithmetic as k_implicit_push.
 // kRows: t holds work boxes of one or several of the sort's tiles o (some a tile
-// smaller than others, box_start; along an axis that 8 does not divide those tiles are 4, 2 or 1
-// cells wide, and their two-cell halo would be most of what a CTA stages), and
-// `nparts` CTAs share a box.  The particles are the box's rows of tiles along x,
+// smaller than others, box_start; along an axis that 8 does not divide those
+// tiles are 4, 2 or 1 cells wide, and their two-cell halo would be most of what
+// a CTA stages), and `nparts` CTAs share a box.  The particles are the box's rows of tiles along x,
 // one range of indices each and of all species one after the other, which the
 // warps take 32 at a time: in a small box, where a CTA has a few hundred
 // particles, all its warps work at once.  Without it: a CTA per tile, species by
 // species.
 // FP32 beams of 39x57x53 (tiles of one cell), 60 per species and cell: 3,170 ->
-// 802 us; shock of 112x51x5: 192 -> 135 us; FP64 pairs of 61x43x1: 525 -> 413 us;
-// of 32x32x1, 32 per species and cell (whole tiles, 19 CTAs each): 207 -> 108 us.
+// 762 us; shock of 112x51x5: 192 -> 135 us; FP64 pairs of 61x43x1: 525 -> 310 us;
+// of 32x32x1, 32 per species and cell (whole tiles, 19 CTAs each): 207 -> 82 us.
 // kFlat (FP64, one cell along z): gathers from four corners, where eight keep the
 // FP64 pipe busy with weights of 0 (32x32x1: 108 -> 82 us).
 template <typename T, bool kWall, bool kRows, bool kFlat>
