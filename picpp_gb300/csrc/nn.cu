@@ -430,23 +430,23 @@ void Net::backward(cudaStream_t s, NetBuffers& b) {
     auto back = [&](int li, const float* gy, const bf16* y, const bf16* x, float* gx, Dims d) {
         const NetLayer& l = L[li];
         const long long n = d.vox() * l.cout;
-        nn::k_relu_bwd<<<gs(n), 256, 0, s>>>(gy, l.relu ? y : nullptr, b.g16, n);
+        nn::k_relu_bwd<<<gs(n / 4), 256, 0, s>>>(gy, l.relu ? y : nullptr, b.g16, (unsigned)(n / 4));
         wgrad(s, l.cin, l.cout, x, b.g16, d, g_ + l.woff, g_ + l.boff);
         if (gx) conv(s, l.cout, l.cin, b.g16, wt + l.woff, nullptr, nullptr, gx, d, 0, tc_err_, wait_limit_);
     };
     back(HEAD, b.A0, nullptr, b.d0, b.B0, b.dm0);
     back(D0B, b.B0, b.d0, b.d0a, b.A0, b.dm0);
     back(D0A, b.A0, b.d0a, b.c0, b.B0, b.dm0);
-    nn::k_up_concat_bwd<<<gs(b.dm0.vox() * 16), 256, 0, s>>>(b.B0, b.A1, b.S0, b.dm0, 32, 16);
+    nn::k_up_concat_bwd<<<gs(b.dm0.vox() * 4), 256, 0, s>>>(b.B0, b.A1, b.S0, b.dm0, 32, 16);
     back(D1B, b.A1, b.d1, b.d1a, b.B1, b.dm1);
     back(D1A, b.B1, b.d1a, b.c1, b.A1, b.dm1);
-    nn::k_up_concat_bwd<<<gs(b.dm1.vox() * 32), 256, 0, s>>>(b.A1, b.A2, b.S1, b.dm1, 64, 32);
+    nn::k_up_concat_bwd<<<gs(b.dm1.vox() * 8), 256, 0, s>>>(b.A1, b.A2, b.S1, b.dm1, 64, 32);
     back(E2B, b.A2, b.e2, b.e2a, b.B2, b.dm2);
     back(E2A, b.B2, b.e2a, b.p2, b.A2, b.dm2);
-    nn::k_pool_bwd_add<<<gs(b.dm1.vox() * 32), 256, 0, s>>>(b.A2, b.S1, b.dm1, 32);
+    nn::k_pool_bwd_add<<<gs(b.dm1.vox() * 8), 256, 0, s>>>(b.A2, b.S1, b.dm1, 32);
     back(E1B, b.S1, b.e1, b.e1a, b.B1, b.dm1);
     back(E1A, b.B1, b.e1a, b.p1, b.A1, b.dm1);
-    nn::k_pool_bwd_add<<<gs(b.dm0.vox() * 16), 256, 0, s>>>(b.A1, b.S0, b.dm0, 16);
+    nn::k_pool_bwd_add<<<gs(b.dm0.vox() * 4), 256, 0, s>>>(b.A1, b.S0, b.dm0, 16);
     back(E0B, b.S0, b.e0, b.e0a, b.A0, b.dm0);
     back(E0A, b.A0, b.e0a, b.x0, nullptr, b.dm0);
 }
