@@ -356,7 +356,8 @@ pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
             {
                 Phase ph(ctx, PIC_PHASE_PUSH_DEPOSIT, 2);   // the fused kernel and its deferred pass
                 PK<T>::push_deposit_tiled(s, g, ctx->wg, ctx->tg, ctx->ws, S, ctx->E, ctx->B, (double*)ctx->Jpart,
-                                          ctx->Jfix, parts);
+                                          parts);
+                PK<T>::push_deposit_deferred(s, g, S, ctx->E, ctx->B, ctx->Jfix);
             }
             {
                 Phase ph(ctx, PIC_PHASE_FIELDS, 1);

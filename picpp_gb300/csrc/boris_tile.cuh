@@ -99,6 +99,52 @@ __device__ __forceinline__ float tri<float, float>(const float* __restrict__ F, 
     return lerp(a, b, wz);
 }
 
+// FP64: an offset within 2^-33 of its cell's lower face or 2^-21 of the upper one.
+// The zigzag split asks on which side of the face the old position, taken back
+// from the new one, lies; for a particle that started on the face the answer is
+// in the last bit, and the fused multiply-adds here round it another way than
+// the separate operations of the phase calls and the oracle.  The deferred pass,
+// compiled with separate operations, takes these particles (a few per million;
+// one electron on the other side moved E of a 64^3 box by 2e-8).  FP32: the
+// roundings are fixed.
+template <typename TP>
+__device__ __forceinline__ bool near_face(TP u) {
+    if constexpr (sizeof(TP) == sizeof(float)) return false;
+    else {
+        const int h = __double2hiint(u);
+        return h < 0x3de00000 || h >= 0x3fefffff;
+    }
+}
+
+// tri at node (i, j, k) of a global grid (periodic).
+template <typename TP, typename TF>
+__device__ __forceinline__ TP tri_global(const GridP& g, const TF* __restrict__ F, int i, int j, int k, TP wx, TP wy, TP wz) {
+    const int di = 1, dj = g.y3 ? 1 : 0, dk = g.z3 ? 1 : 0;
+    auto at = [&](int a, int b, int c) { return TP(F[linw(g, i + a, j + b, k + c)]); };
+    const TP a = lerp(lerp(at(0, 0, 0), at(di, 0, 0), wx), lerp(at(0, dj, 0), at(di, dj, 0), wx), wy);
+    const TP b = lerp(lerp(at(0, 0, dk), at(di, 0, dk), wx), lerp(at(0, dj, dk), at(di, dj, dk), wx), wy);
+    return lerp(a, b, wz);
+}
+// The fused kernel's gather from the global grids, in its order of operations.
+template <typename TP, typename TF>
+__device__ __forceinline__ void tri_gather(const GridP& g, int cell, TP ox, TP oy, TP oz, const TF* __restrict__ E,
+                                           const TF* __restrict__ B, TP e[3], TP b[3]) {
+    int i, j, k;
+    decode(g, cell, i, j, k);
+    const bool ey = g.y3, ez = g.z3;
+    const int ci = ox < TP(0.5) ? i - 1 : i, cj = ey && oy < TP(0.5) ? j - 1 : j, ck = ez && oz < TP(0.5) ? k - 1 : k;
+    const TP wcx = ox < TP(0.5) ? ox + TP(0.5) : ox - TP(0.5);
+    const TP wcy = ey ? (oy < TP(0.5) ? oy + TP(0.5) : oy - TP(0.5)) : TP(0);
+    const TP wcz = ez ? (oz < TP(0.5) ? oz + TP(0.5) : oz - TP(0.5)) : TP(0);
+    const TP wny = ey ? oy : TP(0), wnz = ez ? oz : TP(0);
+    e[0] = tri_global<TP, TF>(g, E, ci, j, k, wcx, wny, wnz);
+    e[1] = tri_global<TP, TF>(g, E + g.N, i, cj, k, ox, wcy, wnz);
+    e[2] = tri_global<TP, TF>(g, E + 2 * g.N, i, j, ck, ox, wny, wcz);
+    b[0] = tri_global<TP, TF>(g, B, i, cj, ck, ox, wcy, wcz);
+    b[1] = tri_global<TP, TF>(g, B + g.N, ci, j, ck, wcx, wny, wcz);
+    b[2] = tri_global<TP, TF>(g, B + 2 * g.N, ci, cj, k, wcx, wcy, wnz);
+}
+
 // The 24 zigzag terms of a particle straight into the FP64 correction grid.
 template <typename TP>
 __device__ __forceinline__ void deposit_global(const GridP& g, TP fcd, TP ox, TP oy, TP oz, const TP v[3], int ni,
@@ -479,7 +525,8 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
                     const int li = local(i, lox + px, otx, g.nx);
                     const int lj = ey ? local(j, loy + py, oty, g.ny) : 0;
                     const int lk = ez ? local(k, loz + pz, otz, g.nz) : 0;
-                    const bool fast = li >= -1 && li <= otx && lj >= -ey && lj <= oty * ey && lk >= -ez && lk <= otz * ez;
+                    const bool fast = li >= -1 && li <= otx && lj >= -ey && lj <= oty * ey && lk >= -ez && lk <= otz * ez &&
+                                      !(near_face(ox) || (ey && near_face(oy)) || (ez && near_face(oz)));
                     push_later = !fast;
                     if (fast) {
                         TP e3[3], b3[3];
@@ -673,7 +720,8 @@ __global__ void __launch_bounds__(256) k_push_deposit_deferred(GridP g, SpeciesS
                 TP v[3];
                 if (push) {
                     TP e3[3], b3[3];
-                    yee_gather<TP, TF>(g, P.cell[n], ox, oy, oz, E, B, e3, b3);
+                    if constexpr (sizeof(TP) == sizeof(float)) yee_gather<TP, TF>(g, P.cell[n], ox, oy, oz, E, B, e3, b3);
+                    else tri_gather<TP, TF>(g, P.cell[n], ox, oy, oz, E, B, e3, b3);
                     boris_t<TP>(q, m, dt, beta, e3, b3, mom);
                     velocity_t<TP>(mom, m, v);
                     if (g.wall) {

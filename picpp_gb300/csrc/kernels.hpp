@@ -61,13 +61,15 @@ struct PK {
     // each one or several tiles o of the sort, `parts` CTAs and partial blocks
     // per work tile (tile_parts)
     static void push_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileGeom& o, const TileShape& sh,
-                                   const SpeciesSet<T>& S, const void* E, const void* B, double* Jpart, double* Jfix,
-                                   int parts);
+                                   const SpeciesSet<T>& S, const void* E, const void* B, double* Jpart, int parts);
     // J from the tile partials and Jfix; inv_scale = 1 / fixed_scale for FP32
     // particles (integer partials), unused for FP64
     static void assemble_j(cudaStream_t s, const GridP& g, const TileGeom& t, const TileShape& sh, const double* Jpart,
                            const double* Jfix, double* J, double inv_scale, int parts);
     static float fixed_scale(const GridP& g, const SpeciesSet<T>& S);
+    // the particles it left over (in the translation unit of the phase calls)
+    static void push_deposit_deferred(cudaStream_t s, const GridP& g, const SpeciesSet<T>& S, const void* E, const void* B,
+                                      double* Jfix);
     static size_t tile_smem_bytes(const TileShape& sh, bool merge);
     static void implicit_deposit(cudaStream_t s, const GridP& g, PartView<T> p, double q, double m, double w,
                                  const double* E, const double* B, double* J, double* mu, double* rho, double* Pi,

@@ -4,7 +4,7 @@
 namespace pic {
 template size_t PK<double>::tile_smem_bytes(const TileShape&, bool);
 template void PK<double>::push_deposit_tiled(cudaStream_t, const GridP&, const TileGeom&, const TileGeom&, const TileShape&,
-                                             const SpeciesSet<double>&, const void*, const void*, double*, double*, int);
+                                             const SpeciesSet<double>&, const void*, const void*, double*, int);
 template float PK<double>::fixed_scale(const GridP&, const SpeciesSet<double>&);
 template void PK<double>::assemble_j(cudaStream_t, const GridP&, const TileGeom&, const TileShape&, const double*,
                                      const double*, double*, double, int);

@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cmath>
 #include "boris.cuh"
+#include "boris_tile.cuh"
 #include "diag.cuh"
 #include "implicit_particles.cuh"
 #include "kernels.hpp"
@@ -182,6 +183,17 @@ void PK<T>::implicit_deposit(cudaStream_t s, const GridP& g, PartView<T> p, doub
     if (p.n == 0) return;
     auto* kernel = compat ? k_implicit_deposit<T, true> : k_implicit_deposit<T, false>;
     kernel<<<grid_for(p.n, 128, 32), 128, 0, s>>>(g, p, q, m, w, E, B, J, mu, rho, Pi, ga);
+}
+
+template <typename T>
+void PK<T>::push_deposit_deferred(cudaStream_t s, const GridP& g, const SpeciesSet<T>& S, const void* E, const void* B,
+                                  double* Jfix) {
+    // one thread per mask word
+    long long words = 1;
+    for (int q = 0; q < S.ns; ++q) words = std::max(words, (S.p[q].n + 31) / 32 + 1);
+    // (few words hold set bits: small CTAs spread them; 128^3, 103 us per step with
+    // 256 threads, 80 us with 64)
+    k_push_deposit_deferred<T, T><<<grid_for(words, 64), 64, 0, s>>>(g, S, (const T*)E, (const T*)B, Jfix);
 }
 
 template <typename T>

@@ -23,8 +23,7 @@ size_t PK<T>::tile_smem_bytes(const TileShape& sh, bool merge) {
 
 template <typename T>
 void PK<T>::push_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileGeom& o, const TileShape& sh,
-                               const SpeciesSet<T>& S, const void* E, const void* B, double* Jpart, double* Jfix,
-                               int parts) {
+                               const SpeciesSet<T>& S, const void* E, const void* B, double* Jpart, int parts) {
     static bool attr_set = false;
     if (!attr_set) {
         for (auto* k : {k_push_deposit_tile<T, T, 8, false, false, false>, k_push_deposit_tile<T, T, 8, false, true, false>,
@@ -65,12 +64,6 @@ void PK<T>::push_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t
                                   : k_push_deposit_tile<T, T, 0, false, true, false>;
     auto* kernel = merge ? k_push_deposit_tile<T, T, 8, false, true, true> : (parts > 1 ? shared : whole);
     kernel<<<grid, kTileThreads, tile_smem_bytes(sh, merge), s>>>(g, t, o, sh, S, K, (const T*)E, (const T*)B, Jpart);
-    // the particles it left over: one thread per mask word
-    long long words = 1;
-    for (int q = 0; q < S.ns; ++q) words = std::max(words, (S.p[q].n + 31) / 32 + 1);
-    // (few words hold set bits: small CTAs spread them; 128^3, 103 us per step with
-    // 256 threads, 80 us with 64)
-    k_push_deposit_deferred<T, T><<<grid_for(words, 64), 64, 0, s>>>(g, S, (const T*)E, (const T*)B, Jfix);
 }
 
 // Fixed-point scale of the FP32 current block: the power of two with
