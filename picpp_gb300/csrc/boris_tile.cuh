@@ -342,19 +342,21 @@ struct MergeTable {
     unsigned first[kMergeTiles], count[kMergeTiles];
     int warp_total[kTileThreads / 32];
 };
-// Fills the table for one species (all threads; a thread per tile).
+// Fills the table for one species (all threads; a thread per tile, or with kRows
+// per row of tiles along x, whose particles are consecutive).
+template <bool kRows>
 __device__ __forceinline__ void merge_table(MergeTable* M, const int* __restrict__ off, const TileGeom& o, int ti, int tj,
                                             int tk) {
     static_assert(kTileThreads == kMergeTiles, "a thread per tile");
     const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
-    const int gx = 8 / o.tx, gy = 8 / o.ty, gz = 8 / o.tz;
-    const int a = ti * gx + e % gx, b = tj * gy + e / gx % gy, c = tk * gz + e / (gx * gy);
+    const int gx = kRows ? 1 : 8 / o.tx, gy = 8 / o.ty, gz = 8 / o.tz;
+    const int a = kRows ? ti * (8 / o.tx) : ti * gx + e % gx, b = tj * gy + e / gx % gy, c = tk * gz + e / (gx * gy);
     int first = 0, count = 0;
     if (e < gx * gy * gz && a < o.ntx && b < o.nty && c < o.ntz) {
         const int T3 = o.tx * o.ty * o.tz;
         const long long k0 = ((long long)(c * o.nty + b) * o.ntx + a) * T3;
         first = off[k0];
-        count = off[k0 + T3] - first;
+        count = off[k0 + T3 * (kRows ? min(8 / o.tx, o.ntx - a) : 1)] - first;
     }
     const int mine = (count + 31) / 32;
     int x = mine;
@@ -389,6 +391,9 @@ __device__ __forceinline__ void merge_table(MergeTable* M, const int* __restrict
 // one of the sort's tiles, counted from its first, and a particle's distance
 // is measured from that tile, so the sums of a run, and which particles are
 // left to the deferred pass, are those of a CTA per tile, bit for bit (FP32).
+// FP64 sums come in any order, so its chunks are cut from rows of tiles along x
+// (35x49x17, tiles of one cell, 5 per species: 15.3 -> 4.7 ms for five steps),
+// and distances are measured from the work tile.
 // At 100x60x54, 9 per species and cell (tiles of 4x4x2): 428 -> 273 us.
 template <typename TP, typename TF, int CT, bool kWall, bool kParts, bool kMerge>
 __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_tile(GridP g, TileGeom t, TileGeom o, TileShape s,
@@ -428,7 +433,8 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
     const TP idx = K.id[0], idy = K.id[1], idz = K.id[2];
     const int parts = kParts ? K.parts : 1;
     // extents of the sort's tiles
-    const int otx = kMerge ? o.tx : tx, oty = kMerge ? o.ty : ty, otz = kMerge ? o.tz : tz;
+    constexpr bool kPlace = kMerge && kFixed;   // where a chunk's tile lies in the work tile matters
+    const int otx = kPlace ? o.tx : tx, oty = kPlace ? o.ty : ty, otz = kPlace ? o.tz : tz;
     const int ey = CT ? 1 : (g.y3 ? 1 : 0), ez = CT ? 1 : (g.z3 ? 1 : 0);
     const int fsy = ey ? fx : 0, fsz = ez ? fx * fy : 0;
 
@@ -475,7 +481,7 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
                 pe = sM->first[at] + sM->count[at];
             };
             if constexpr (kMerge) {
-                merge_table(sM, S.off[sp], o, ti, tj, tk);
+                merge_table<!kFixed>(sM, S.off[sp], o, ti, tj, tk);
                 chunks = sM->before[kMergeTiles];
                 n0 = pe = 0;
                 if (c < chunks) seek();
@@ -490,9 +496,9 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
                 const unsigned nb = n0, n = n0 + lane;
                 const bool here = n < pe;
                 // the tile's place in the work tile
-                const int px = kMerge ? (at & (CT / otx - 1)) * otx : 0;
-                const int py = kMerge ? (at / (CT / otx) & (CT / oty - 1)) * oty : 0;
-                const int pz = kMerge ? at / (CT / otx * (CT / oty)) * otz : 0;
+                const int px = kPlace ? (at & (CT / otx - 1)) * otx : 0;
+                const int py = kPlace ? (at / (CT / otx) & (CT / oty - 1)) * oty : 0;
+                const int pz = kPlace ? at / (CT / otx * (CT / oty)) * otz : 0;
                 TP aB[12];
                 TP s1[6] = {TP(0), TP(0), TP(0), TP(0), TP(0), TP(0)};   // F1 and W1 of the old-side segment
                 int keyA = -1 - lane, keyB = -1 - lane;   // lanes outside a reduction keep unique keys
@@ -593,7 +599,7 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
                         const TP RZ = rz == 0 ? (Z + PZ) * TP(0.5) : TP(rz > 0 ? rz : 0) * dz;
                         const int ax = bx + rx, ay = by + ry, az = bz + rz;   // block cell of the old-side segment
                         // unsigned compares: (unsigned)x < n is 0 <= x < n
-                        const int ex_ = kMerge ? otx + 4 : jx, ey_ = kMerge ? oty + 4 : jy, ez_ = kMerge ? otz + 4 : jz;
+                        const int ex_ = kPlace ? otx + 4 : jx, ey_ = kPlace ? oty + 4 : jy, ez_ = kPlace ? otz + 4 : jz;
                         const bool inblock = nearx && (unsigned)(rx + 1) <= 2u && (unsigned)(ry + 1) <= 2u &&
                                              (unsigned)(rz + 1) <= 2u && (unsigned)ax < (unsigned)(ex_ - 1) &&
                                              (unsigned)bx < (unsigned)(ex_ - 1) && (unsigned)ay < (unsigned)(ey_ - ey) &&
