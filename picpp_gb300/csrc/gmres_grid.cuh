@@ -105,7 +105,10 @@ struct GmresCta {
         s = warp_sum(s);
         if ((threadIdx.x & 31) == 0) warp_row()[v] = s;
     }
-    // The CTA's sums of K values from its warps' to the partials of buffer `buf`.
+    // The CTA's sums of K values from its warps' to the partials of buffer `buf`
+    // (0: up to gmres_vals values, 1: up to two).  A CTA may be collecting from a
+    // buffer until it arrives at the next barrier, so between a collect and the
+    // next publish of the same buffer there is always one.
     __device__ void publish(int K, int buf) {
         const int kv = gmres_vals(A.cols);
         __syncthreads();
@@ -417,9 +420,9 @@ __global__ void __launch_bounds__(NW + 32) k_gmres_grid(const __grid_constant__ 
         }
     T.warp_sum1(sum, 0);
     T.warp_sum1(count, 1);
-    T.publish(2, 1);
+    T.publish(2, 0);   // (not buffer 1: the reference method's norm2 comes without a barrier between)
     if (!T.barrier()) return;
-    T.collect(2, 1);
+    T.collect(2, 0);
     if (T.sh[1] > 0) { T.finish(kGmNonFiniteSystem, 0, 0, 0); return; }
     const double bnorm = sqrt(T.sh[0]);
     if (bnorm == 0) {
