@@ -18,7 +18,7 @@
 //     order, so that all CTAs agree without another exchange.  All sums have
 //     a fixed order: a solve is reproducible bit for bit.
 // What it measured against the kernel-per-operation form stands at
-// launch_gmres_grid (grid.cu).
+// launch_gmres_grid (gmres_launch.cuh).
 #pragma once
 #include <algorithm>
 #include "common.cuh"

@@ -2,7 +2,7 @@
 // corrections, Maxwell right part and operator, field update, Krylov vectors.
 #include "implicit_grid.cuh"
 #include "kernels.hpp"
-#include "gmres_grid.cuh"
+#include "gmres_launch.cuh"
 #include "krylov.cuh"
 #include "sort.cuh"
 #include "wall.cuh"
@@ -329,45 +329,6 @@ void launch_combine(cudaStream_t s, double* x, const double* V, long long ld, in
 
 void launch_residual(cudaStream_t s, double* r, const double* b, const double* Ax, long long n) {
     k_residual<<<grid_for(n, 256), 256, 0, s>>>(r, b, Ax, n);
-}
-
-template <int NW, int KB, bool kNode, bool kRef>
-static cudaError_t gmres_grid(cudaStream_t s, const GmresArgs& a) {
-    const size_t smem = gmres_smem(a.cols, NW, kRef);
-    cudaError_t e = cudaFuncSetAttribute(k_gmres_grid<NW, KB, kNode, kRef>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-    const int grid = (int)std::min<long long>(kNumSM, ((kNode ? 1 : 3) * a.g.N + NW - 1) / NW);
-    void* args[] = {(void*)&a};
-    return cudaLaunchCooperativeKernel(k_gmres_grid<NW, KB, kNode, kRef>, grid, NW + 32, args, smem, s);
-}
-
-// Workers per CTA by the box: few, each with one element, while the barriers'
-// and reductions' latency is the time; many, each with whole nodes, once the
-// FP64 work is (more warps hide the loads of the basis).  Restarted GMRES(30)
-// to 1e-8, us per solve (16 iterations), the kernel-per-operation form first:
-//   32x32x1      26x20x18     64x64x32     128x128x32    256x256x64
-//   (1,750)      2,120        3,942        6,694         30,000
-//   128: 261     256: 384     480: 1,063   736: 3,075    992: 19,498
-// and the neighbours of each choice:
-//   256: 306     128: 435     736: 1,506   480: 3,292    736: 19,857
-// (128x64x32: 480 1,754, 736 2,007; 128x128x64: 736 5,720, 992 5,429.)
-cudaError_t launch_gmres_grid(cudaStream_t s, const GmresArgs& a) {
-    cudaError_t e = cudaMemsetAsync(a.bar, 0, 2 * sizeof(unsigned), s);
-    if (e != cudaSuccess) return e;
-    const long long n = a.g.N;
-    if (a.reference) {
-        if (n <= 4096) return gmres_grid<128, 8, false, true>(s, a);
-        if (n <= 24576) return gmres_grid<256, 8, false, true>(s, a);
-        if (n <= 393216) return gmres_grid<480, 4, true, true>(s, a);
-        if (n <= 786432) return gmres_grid<736, 4, true, true>(s, a);
-        return gmres_grid<992, 4, true, true>(s, a);
-    }
-    if (n <= 4096) return gmres_grid<128, 16, false, false>(s, a);
-    if (n <= 24576) return gmres_grid<256, 16, false, false>(s, a);
-    if (n <= 393216) return gmres_grid<480, 8, true, false>(s, a);
-    if (n <= 786432) return gmres_grid<736, 8, true, false>(s, a);
-    return gmres_grid<992, 8, true, false>(s, a);
 }
 
 // FP32 vectors: float4 accesses when the length is a multiple of 4 and the

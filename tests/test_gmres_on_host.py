@@ -1,6 +1,7 @@
 """The one-launch GMRES kernel (csrc/gmres_grid.cuh) on host threads
 (cpp/gmres_on_host.cpp): its solution, and that no CTA overwrites partial sums
-that another, held up, has yet to collect.  No GPU."""
+that another, held up, has yet to collect; its launch against a CUDA runtime
+of the test's own (cpp/gmres_launch_on_host.cpp).  No GPU."""
 import os
 import shutil
 import subprocess
@@ -17,7 +18,8 @@ CUDA = next((d for d in ("/usr/local/cuda/include",) if os.path.exists(os.path.j
 
 
 @pytest.fixture(scope="module")
-def exe(tmp_path_factory):
+def headers(tmp_path_factory):
+    """A folder with the kernel's header as the host compiles it."""
     if shutil.which("g++") is None or CUDA is None:
         pytest.skip("needs g++ and the CUDA headers")
     d = tmp_path_factory.mktemp("gmres")
@@ -30,10 +32,28 @@ def exe(tmp_path_factory):
         assert text.count(gpu) == 1, gpu
         text = text.replace(gpu, host)
     (d / "gmres_grid_host.cuh").write_text(text)
-    out = str(d / "gmres_on_host")
-    subprocess.run(["g++", "-std=c++20", "-O1", "-w", "-pthread", "-I", str(d), "-I", CSRC, "-I", CUDA,
-                    os.path.join(ROOT, "tests", "cpp", "gmres_on_host.cpp"), "-o", out], check=True)
+    return str(d)
+
+
+def compiled(headers, name, *extra):
+    out = os.path.join(headers, name)
+    subprocess.run(["g++", "-std=c++20", "-O1", "-w", "-pthread", "-I", headers, "-I", CSRC, "-I", CUDA,
+                    os.path.join(ROOT, "tests", "cpp", name + ".cpp"), "-o", out, *extra], check=True)
     return out
+
+
+@pytest.fixture(scope="module")
+def exe(headers):
+    return compiled(headers, "gmres_on_host")
+
+
+@pytest.fixture(scope="module")
+def launcher(headers):
+    # (kernels and the methods that no test here reaches stay unresolved; gmres_launch.cuh
+    # finds the host's form of the kernel in gmres_grid.cuh's place)
+    with open(os.path.join(headers, "gmres_launch.cuh"), "w") as f:
+        f.write(open(os.path.join(CSRC, "gmres_launch.cuh")).read().replace('"gmres_grid.cuh"', '"gmres_grid_host.cuh"'))
+    return compiled(headers, "gmres_launch_on_host", "-Wl,--unresolved-symbols=ignore-all")
 
 
 N = (4, 3, 3)
@@ -78,3 +98,10 @@ def test_a_late_cta_changes_nothing(exe, tmp_path, reference):
         for nth in range(1, 5):
             i2, x2 = solve(exe, tmp_path, reference, late, nth)
             assert np.array_equal(info, i2) and np.array_equal(x, x2), (late, nth)
+
+
+def test_solves_of_two_threads_do_not_refuse_each_other(launcher):
+    """The shared memory that a kernel may take is set for the function, not for a
+    thread: a solve with few columns between another's preparation and launch."""
+    r = subprocess.run([launcher, "threads"], check=True, capture_output=True, text=True, timeout=60)
+    assert r.stdout.split() == ["0", "0"]
