@@ -15,7 +15,17 @@ static cudaError_t gmres_grid(cudaStream_t s, const GmresArgs& a) {
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)gmres_smem(kGmresMaxCols, NW, kRef));
     if (e != cudaSuccess) return e;
-    const int grid = (int)std::min<long long>(kNumSM, ((kNode ? 1 : 3) * a.g.N + NW - 1) / NW);
+    // as many CTAs as run at once on the SMs that this process sees, at most one
+    // per SM of a whole GB300 (what the partial sums have room for)
+    int device = 0, sms = 0, per_sm = 0;
+    if ((e = cudaGetDevice(&device)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess ||
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_gmres_grid<NW, KB, kNode, kRef>, NW + 32,
+                                                           smem)) != cudaSuccess)
+        return e;
+    const long long most = std::min<long long>(kNumSM, (long long)sms * per_sm);
+    if (most < 1) return cudaErrorCooperativeLaunchTooLarge;
+    const int grid = (int)std::min<long long>(most, ((kNode ? 1 : 3) * a.g.N + NW - 1) / NW);
     void* args[] = {(void*)&a};
     return cudaLaunchCooperativeKernel((const void*)k_gmres_grid<NW, KB, kNode, kRef>, grid, NW + 32, args, smem, s);
 }

@@ -93,6 +93,11 @@ bool one_launch(const GridP& g, const pic_solve_opts& o) {
     return o.method == PIC_GMRES_REFERENCE && (o.max_iter > 0 ? o.max_iter : 50) <= kGmresMaxCols + 2;
 }
 
+pic_status gmres_reference(SolveCtx& c, const OpCoef& oc, const double* rhs, double* x, const pic_solve_opts& o,
+                           pic_solve_info* info);
+pic_status gmres_restarted(SolveCtx& c, const OpCoef& oc, const double* b, double* x, const pic_solve_opts& o,
+                           pic_solve_info* info, Net* pc = nullptr, int inner = 0);
+
 pic_status gmres_one_launch(SolveCtx& c, const OpCoef& oc, const double* rhs, double* x, const pic_solve_opts& o,
                             pic_solve_info* info) {
     const GridP& g = *c.g;
@@ -121,7 +126,14 @@ pic_status gmres_one_launch(SolveCtx& c, const OpCoef& oc, const double* rhs, do
     a.mu = c.mu; a.b = rhs; a.x = x;
     a.V = k.V; a.mx = k.mx; a.w = k.w; a.r = k.r;
     a.part = k.part; a.bar = k.bar; a.out = k.scal;
-    CKS(launch_gmres_grid(c.s, a));
+    const cudaError_t launched = launch_gmres_grid(c.s, a);
+    if (launched == cudaErrorCooperativeLaunchTooLarge || launched == cudaErrorNotSupported) {
+        // the device does not run all its CTAs at once: operation by operation
+        cudaGetLastError();   // (cleared)
+        if ((st = check_finite(c, rhs, L)) != PIC_OK || (st = check_finite(c, c.mu, 3 * L)) != PIC_OK) return st;
+        return ref ? gmres_reference(c, oc, rhs, x, o, info) : gmres_restarted(c, oc, rhs, x, o, info);
+    }
+    CKS(launched);
     double out[kGmOutLen] = {};
     unsigned bar[2] = {};
     CKS(cudaMemcpyAsync(out, k.scal, sizeof(out), cudaMemcpyDeviceToHost, c.s));
@@ -312,7 +324,7 @@ pic_status inner_apply(SolveCtx& c, const OpCoef& oc, int S, double tol, const d
 // rest of the solve to plain GMRES from the current iterate.  With inner > 0
 // the right preconditioner is instead the FP32 inner solve of inner steps.
 pic_status gmres_restarted(SolveCtx& c, const OpCoef& oc, const double* b, double* x, const pic_solve_opts& o,
-                           pic_solve_info* info, Net* pc = nullptr, int inner = 0) {
+                           pic_solve_info* info, Net* pc, int inner) {
     const GridP& g = *c.g;
     Net* const net = pc;   // pc becomes nullptr on a fallback
     bool have = pc != nullptr || inner > 0;   // a right preconditioner is in use

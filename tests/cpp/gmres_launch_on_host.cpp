@@ -5,7 +5,11 @@
 //
 //   gmres_launch_on_host threads   two threads' solves, the second one's launch
 //                                  between the first one's preparation and launch
-// Prints the solves' statuses and the grid of the last launch.
+//   gmres_launch_on_host device SMS COOPERATIVE   a solve of each plain method on a
+//                                  device of SMS multiprocessors, which takes cooperative
+//                                  launches or does not
+// Prints the solves' statuses and, of a device, the grid of the last launch (0: none)
+// and how many dot products were launched by themselves.
 #include "host_cuda.hpp"
 
 #include <cstdio>
@@ -26,7 +30,7 @@ namespace {
 std::mutex lock;
 std::map<const void*, size_t> most_smem;          // opted-in dynamic shared memory
 std::function<void()> after_attribute;            // called once, after an attribute is set
-int launches = 0, last_grid = 0;
+int last_grid = 0, dots = 0, multiprocessors = 152, cooperative = 1;
 }  // namespace
 
 extern "C" {
@@ -43,12 +47,19 @@ cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute, int v) {
 cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3 grid, dim3, void** args, size_t smem, cudaStream_t) {
     std::lock_guard<std::mutex> l(lock);
     if (smem > std::max<size_t>(48 * 1024, most_smem[f])) return cudaErrorInvalidValue;
-    ++launches;
+    if (!cooperative) return cudaErrorNotSupported;
+    if ((int)grid.x > multiprocessors) return cudaErrorCooperativeLaunchTooLarge;   // one CTA of these per SM
     last_grid = (int)grid.x;
     const GmresArgs& a = *static_cast<const GmresArgs*>(args[0]);
     for (int i = 0; i < kGmOutLen; ++i) a.out[i] = 0;
     return cudaSuccess;
 }
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr what, int) {
+    *v = what == cudaDevAttrMultiProcessorCount ? multiprocessors : 0;
+    return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int, size_t) { *n = 1; return cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t n) { *p = std::calloc(n, 1); return cudaSuccess; }
 cudaError_t cudaFree(void* p) { std::free(p); return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t) { std::memset(p, v, n); return cudaSuccess; }
@@ -62,6 +73,15 @@ cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 0; return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 }
+
+// The operations that a solve of a right part 0 takes by themselves.
+namespace pic {
+void launch_nonfinite(cudaStream_t, const double*, long long, int*) {}
+void launch_dot(cudaStream_t, const double*, const double*, long long, double*, int, double* out, int) {
+    ++dots;
+    *out = 0;
+}
+}  // namespace pic
 
 // A box, its system (right part 0) and a workspace of its own.
 struct Caller {
@@ -98,6 +118,14 @@ int main(int argc, char** argv) {
         };
         const int first = one.solve(PIC_GMRES_RESTARTED, 128);
         std::printf("%d %d\n", first, second.get());
+        return 0;
+    }
+    if (what == "device" && argc == 4) {
+        multiprocessors = std::atoi(argv[2]);
+        cooperative = std::atoi(argv[3]);
+        Caller one(20, 20, 20);
+        const int a = one.solve(PIC_GMRES_REFERENCE, 0), b = one.solve(PIC_GMRES_RESTARTED, 30);
+        std::printf("%d %d %d %d\n", a, b, last_grid, dots);
         return 0;
     }
     return 2;

@@ -105,3 +105,13 @@ def test_solves_of_two_threads_do_not_refuse_each_other(launcher):
     thread: a solve with few columns between another's preparation and launch."""
     r = subprocess.run([launcher, "threads"], check=True, capture_output=True, text=True, timeout=60)
     assert r.stdout.split() == ["0", "0"]
+
+
+# 20^3 nodes on 256 workers a CTA: 94 CTAs
+@pytest.mark.parametrize("sms,cooperative,grid,dots", [(152, 1, 94, 0), (76, 1, 76, 0), (3, 1, 3, 0), (152, 0, 0, 2)])
+def test_a_smaller_device_solves_too(launcher, sms, cooperative, grid, dots):
+    """As many CTAs as the device runs at once; operation by operation where it takes no
+    cooperative launch."""
+    r = subprocess.run([launcher, "device", str(sms), str(cooperative)], check=True, capture_output=True, text=True,
+                       timeout=60)
+    assert [int(v) for v in r.stdout.split()] == [0, 0, grid, dots]
