@@ -26,10 +26,6 @@
 
 namespace pic {
 
-// Polls of a barrier before it gives up (about ten seconds; CTAs of a
-// cooperative launch all run at once, so only a fault reaches it).
-constexpr unsigned kGmresPolls = 1u << 24;
-
 // Values of one dot-product phase at most.
 __host__ __device__ inline int gmres_vals(int cols) { return 2 * (cols + 2); }
 inline size_t gmres_smem(int cols, int workers, bool reference) {
@@ -68,7 +64,7 @@ struct GmresCta {
             unsigned polls = 0, seen;
             do {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(A.bar) : "memory");
-            } while ((int)(seen - target) < 0 && ++polls < kGmresPolls);
+            } while ((int)(seen - target) < 0 && ++polls < A.polls);
             *bad = (int)(seen - target) < 0;
             if (*bad) A.bar[1] = 1u;
             __threadfence();

@@ -167,6 +167,9 @@ void launch_combine(cudaStream_t s, double* x, const double* V, long long ld, in
                     int accumulate, long long n);
 // A whole FP64 GMRES solve in one cooperative launch (gmres_grid.cuh)
 constexpr int kGmresMaxCols = 128;    // Krylov columns its shared-memory triangles reach
+// Polls of a grid barrier before it gives up (about ten seconds; CTAs of a
+// cooperative launch all run at once, so only a fault reaches it).
+constexpr unsigned kGmresPolls = 1u << 24;
 struct GmresArgs {
     GridP g;
     OpCoef oc;
@@ -184,6 +187,7 @@ struct GmresArgs {
     int cols;         // columns per cycle (restarted) / most columns (reference)
     int max_iter;     // restarted: iterations in all; reference: its limit on n
     int reference;
+    unsigned polls;   // kGmresPolls
 };
 enum GmresOut { kGmStatus = 0, kGmIterations, kGmRestarts, kGmRel, kGmOutLen };
 enum GmresStatus { kGmOk = 0, kGmNotConverged, kGmNonFiniteSystem, kGmNonFiniteResidual };

@@ -105,6 +105,7 @@ pic_status gmres_one_launch(SolveCtx& c, const OpCoef& oc, const double* rhs, do
     const bool ref = o.method == PIC_GMRES_REFERENCE;
     GmresArgs a{};
     a.reference = ref ? 1 : 0;
+    a.polls = kGmresPolls;
     pic_status st;
     if (ref) {
         const int maxIter = o.max_iter > 0 ? o.max_iter : 50;

@@ -8,6 +8,7 @@
 //   gmres_launch_on_host device SMS COOPERATIVE   a solve of each plain method on a
 //                                  device of SMS multiprocessors, which takes cooperative
 //                                  launches or does not
+//   gmres_launch_on_host runs-out  a solve one of whose barriers gave up, then another
 // Prints the solves' statuses and, of a device, the grid of the last launch (0: none)
 // and how many dot products were launched by themselves.
 #include "host_cuda.hpp"
@@ -30,7 +31,7 @@ namespace {
 std::mutex lock;
 std::map<const void*, size_t> most_smem;          // opted-in dynamic shared memory
 std::function<void()> after_attribute;            // called once, after an attribute is set
-int last_grid = 0, dots = 0, multiprocessors = 152, cooperative = 1;
+int last_grid = 0, dots = 0, multiprocessors = 152, cooperative = 1, runs_out = 0;
 }  // namespace
 
 extern "C" {
@@ -51,7 +52,9 @@ cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3 grid, dim3, void** a
     if ((int)grid.x > multiprocessors) return cudaErrorCooperativeLaunchTooLarge;   // one CTA of these per SM
     last_grid = (int)grid.x;
     const GmresArgs& a = *static_cast<const GmresArgs*>(args[0]);
-    for (int i = 0; i < kGmOutLen; ++i) a.out[i] = 0;
+    if (runs_out) a.bar[1] = 1;
+    else
+        for (int i = 0; i < kGmOutLen; ++i) a.out[i] = 0;
     return cudaSuccess;
 }
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
@@ -126,6 +129,14 @@ int main(int argc, char** argv) {
         Caller one(20, 20, 20);
         const int a = one.solve(PIC_GMRES_REFERENCE, 0), b = one.solve(PIC_GMRES_RESTARTED, 30);
         std::printf("%d %d %d %d\n", a, b, last_grid, dots);
+        return 0;
+    }
+    if (what == "runs-out") {
+        Caller one(20, 20, 20);
+        runs_out = 1;
+        const int a = one.solve(PIC_GMRES_REFERENCE, 0);
+        runs_out = 0;
+        std::printf("%d %s\n%d\n", a, one.text.c_str(), one.solve(PIC_GMRES_REFERENCE, 0));
         return 0;
     }
     return 2;

@@ -5,10 +5,11 @@
 // kernel's header with shared memory and the acquiring load given by functions of
 // host_cuda.hpp.
 //
-//   gmres_on_host SYSTEM OUT late nth
+//   gmres_on_host SYSTEM OUT late nth polls
 // SYSTEM: int32 nx ny nz reference cols max_iter ctas, float64 dx dy dz dt theta
 // cfix tol, then mu (9N) and b (3N).  CTA `late` waits between the nth barrier and the
-// collection of partial sums that follows it (-1: none does).  OUT: float64 status, iterations, restarts, residual, x (3N).
+// collection of partial sums that follows it (-1: none does); a barrier of the grid gives
+// up after `polls` polls (0: as many as the library takes).  OUT: float64 status, iterations, restarts, residual, x (3N).
 #include "host_cuda.hpp"
 
 #include <cstdio>
@@ -38,7 +39,7 @@ static void run(const GmresArgs& a, int ctas) {
 }
 
 int main(int argc, char** argv) {
-    if (argc != 5) return 2;
+    if (argc != 6) return 2;
     std::FILE* f = std::fopen(argv[1], "rb");
     int n[7];
     double d[7];
@@ -65,11 +66,12 @@ int main(int argc, char** argv) {
     std::fclose(f);
     a.mu = mu.data(); a.b = b.data(); a.x = x.data(); a.V = V.data(); a.mx = mx.data(); a.w = w.data(); a.r = r.data();
     a.part = part.data(); a.bar = bar; a.out = out.data();
+    a.polls = std::atoi(argv[5]) > 0 ? (unsigned)std::atoi(argv[5]) : kGmresPolls;
     late_cta = std::atoi(argv[3]);
     late_at = std::atoi(argv[4]);
     if (a.reference) run<true>(a, ctas);
     else run<false>(a, ctas);
-    if (bar[1]) return 3;
+    if (bar[1]) out[kGmStatus] = -1;   // a barrier gave up
     f = std::fopen(argv[2], "wb");
     if (!f) return 2;
     std::fwrite(out.data(), 8, kGmOutLen, f);

@@ -70,7 +70,7 @@ def system():
     return mu.reshape(-1), rng.standard_normal(3 * n)
 
 
-def solve(exe, tmp_path, reference, late=-1, nth=0):
+def solve(exe, tmp_path, reference, late=-1, nth=0, polls=0):
     mu, b = system()
     src, dst = str(tmp_path / "system"), str(tmp_path / "out")
     with open(src, "wb") as f:
@@ -78,7 +78,7 @@ def solve(exe, tmp_path, reference, late=-1, nth=0):
         np.array([BOX.dx, BOX.dy, BOX.dz, BOX.dt, BOX.theta, BOX.cfix, 1e-15 if reference else 1e-4]).tofile(f)
         mu.tofile(f)
         b.tofile(f)
-    subprocess.run([exe, src, dst, str(late), str(nth)], check=True, timeout=120)
+    subprocess.run([exe, src, dst, str(late), str(nth), str(polls)], check=True, timeout=120)
     r = np.fromfile(dst)
     return r[:4], r[4:]
 
@@ -100,11 +100,26 @@ def test_a_late_cta_changes_nothing(exe, tmp_path, reference):
             assert np.array_equal(info, i2) and np.array_equal(x, x2), (late, nth)
 
 
+@pytest.mark.parametrize("reference", [0, 1])
+@pytest.mark.parametrize("late,nth", [(2, 1), (0, 2), (1, 3)])
+def test_a_barrier_that_runs_out_ends_the_solve(exe, tmp_path, reference, late, nth):
+    """One CTA held up, and barriers of few polls: every thread leaves, with an
+    error and the solution as it was."""
+    info, x = solve(exe, tmp_path, reference, late, nth, polls=2)
+    assert info[0] == -1 and (x == -1.0).all()
+
+
 def test_solves_of_two_threads_do_not_refuse_each_other(launcher):
     """The shared memory that a kernel may take is set for the function, not for a
     thread: a solve with few columns between another's preparation and launch."""
     r = subprocess.run([launcher, "threads"], check=True, capture_output=True, text=True, timeout=60)
     assert r.stdout.split() == ["0", "0"]
+
+
+def test_a_barrier_that_ran_out_is_an_error_of_that_solve_only(launcher):
+    """PIC_ERR_CUDA from the solve whose kernel says so; the next one succeeds."""
+    r = subprocess.run([launcher, "runs-out"], check=True, capture_output=True, text=True, timeout=60)
+    assert r.stdout.split("\n")[:2] == ["2 a grid barrier of the field solve ran out", "0"]
 
 
 # 20^3 nodes on 256 workers a CTA: 94 CTAs
