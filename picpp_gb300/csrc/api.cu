@@ -424,7 +424,8 @@ TileGeom deposit_boxes(const GridP& g, const TileGeom& t, int ns, ImpBlock& bk) 
     for (;;) {
         TileGeom w{e[0], e[1], e[2], m[0], m[1], m[2], -1, -1, -1};
         // FP32 sums of several of the sort's tiles meet in FP64, as in the grids
-        const bool wide = sizeof(T) == 4 && (e[0] > t.tx || e[1] > t.ty || e[2] > t.tz);
+        bool wide = false;
+        for (int a = 0; a < 3; ++a) wide = wide || (sizeof(T) == 4 && !boxes_in_tiles(n[a], m[a], tile[a]));
         bk = PK<T>::implicit_block(g, w, 0, wide);
         bk.stage = 1;
         const bool fits = PK<T>::implicit_tile_smem(bk, e[0] * e[1] * e[2], ns) <= (size_t)(227 * 1024) / 2 - 1024;

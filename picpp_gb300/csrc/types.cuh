@@ -28,6 +28,10 @@ __host__ __device__ __forceinline__ int box_start(int n, int b, int m) {
     return b * q + (b < r ? b : r);
 }
 
+// Whether each of m boxes along an axis of n cells (box_start) lies within one of
+// the tiles of t cells that divide it; ragged boxes of several tiles count as not.
+inline bool boxes_in_tiles(int n, int m, int t) { return t >= n || (n % m == 0 && t % (n / m) == 0); }
+
 // Sort key of cell (i, j, k): tile by tile, x fastest in a tile.
 __device__ __forceinline__ int cell_key(const TileGeom& t, int i, int j, int k) {
     int ti, tj, tk;
