@@ -104,17 +104,19 @@ __device__ __forceinline__ float tri<float, float>(const float* __restrict__ F, 
 // from the new one, lies; for a particle that started on the face the answer is
 // in the last bit, and the fused multiply-adds here round it another way than
 // the separate operations of the phase calls and the oracle.  The deferred pass,
-// compiled with separate operations, takes these particles (a few per million;
-// one electron on the other side moved E of a 64^3 box by 2e-8).  FP32: the
-// roundings are fixed.
-template <typename TP>
-__device__ __forceinline__ bool near_face(TP u) {
-    if constexpr (sizeof(TP) == sizeof(float)) return false;
-    else {
-        const int h = __double2hiint(u);
-        return h < 0x3de00000 || h >= 0x3fefffff;
-    }
+// compiled with separate operations, takes these particles (a few per million of a
+// thermal plasma; one electron on the other side moved E of a 64^3 box by 2e-8).
+// FP32: the roundings are fixed.
+__device__ __forceinline__ bool near_face(double u) {
+    const int h = __double2hiint(u);
+    return h < 0x3de00000 || h >= 0x3fefffff;
 }
+// Of a load on a lattice they may be all.  A chunk takes as long here with one
+// particle as with 32, and the deferred pass about as long per particle: from a sixth
+// of the lanes on it takes the chunk (64^3, 8 per species and cell, a step with no
+// particle on a face 3.6 ms; seven of eight on one 7.5 ms with the others pushed here,
+// 5.5 ms so; 7.5 ms in the separately rounded fused kernel that this one replaced).
+constexpr int kNearMin = 6;
 
 // tri at node (i, j, k) of a global grid (periodic).
 template <typename TP, typename TF>
@@ -518,6 +520,14 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
                 }
                 if (n0 + lane < pe) stage_particle(sBuf, P, n0 + lane, lane);
                 cp_async_commit();
+                // FP64: particles near a face, and with kNearMin of them the whole
+                // chunk, are left to the deferred pass
+                bool near = false;
+                if constexpr (!kFixed) {
+                    near = here && (near_face(ox) || (ey && near_face(oy)) || (ez && near_face(oz)));
+                    const unsigned all = __ballot_sync(0xffffffffu, near);
+                    near = near || __popc(all) >= kNearMin;
+                }
                 // (an escaped particle of a wall box waits with cell -1 for the sort)
                 if (here && (!kWall || cell >= 0)) {
                     int i, j, k;
@@ -531,8 +541,7 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
                     const int li = local(i, lox + px, otx, g.nx);
                     const int lj = ey ? local(j, loy + py, oty, g.ny) : 0;
                     const int lk = ez ? local(k, loz + pz, otz, g.nz) : 0;
-                    const bool fast = li >= -1 && li <= otx && lj >= -ey && lj <= oty * ey && lk >= -ez && lk <= otz * ez &&
-                                      !(near_face(ox) || (ey && near_face(oy)) || (ez && near_face(oz)));
+                    const bool fast = li >= -1 && li <= otx && lj >= -ey && lj <= oty * ey && lk >= -ez && lk <= otz * ez && !near;
                     push_later = !fast;
                     if (fast) {
                         TP e3[3], b3[3];
@@ -694,6 +703,9 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas<TP>()) k_push_deposit_
 //     block): the zigzag current of the stored new position and velocity.
 // The current goes into Jfix with FP64 global atomics; a particle that left a
 // wall box is marked (cell -1) once its current is in.
+// FP32: a thread per word (few of which hold a bit).  FP64, where every particle of
+// a lattice load may start on a face (near_face): the bits dealt to the lanes, so
+// that neighbours move neighbouring particles.
 template <typename TP, typename TF>
 __global__ void __launch_bounds__(256) k_push_deposit_deferred(GridP g, SpeciesSet<TP> S, const TF* __restrict__ E,
                                                                const TF* __restrict__ B, double* __restrict__ Jfix) {
@@ -708,45 +720,78 @@ __global__ void __launch_bounds__(256) k_push_deposit_deferred(GridP g, SpeciesS
         unsigned* mp = S.defer[sp];
         unsigned* md = mp + S.dwords[sp];
         const long long words = (P.n + 31) / 32 + 1;
-        for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < words;
-             w += (long long)gridDim.x * blockDim.x) {
-            unsigned bp = mp[w], bd = md[w];
-            if (!(bp | bd)) continue;
-            mp[w] = 0u;
-            md[w] = 0u;
-            while (bp | bd) {
-                const bool push = bp != 0u;
-                unsigned& bits = push ? bp : bd;
-                const long long n = w * 32 + (__ffs(bits) - 1);
-                bits &= bits - 1u;
-                TP ox = P.ox[n], oy = P.oy[n], oz = P.oz[n];
-                TP mom[3] = {P.px[n], P.py[n], P.pz[n]};
-                int ni, nj, nk;
-                decode(g, P.cell[n], ni, nj, nk);
-                TP v[3];
-                if (push) {
-                    TP e3[3], b3[3];
-                    if constexpr (sizeof(TP) == sizeof(float)) yee_gather<TP, TF>(g, P.cell[n], ox, oy, oz, E, B, e3, b3);
-                    else tri_gather<TP, TF>(g, P.cell[n], ox, oy, oz, E, B, e3, b3);
-                    boris_t<TP>(q, m, dt, beta, e3, b3, mom);
-                    velocity_t<TP>(mom, m, v);
-                    if (g.wall) {
-                        if (tristan_wall_x<TP>(g, ni, ox, (v[0] * dt) * idx) & 1) {   // reflectMomentumX
-                            mom[0] = -mom[0];
-                            v[0] = -v[0];
-                        }
-                    } else {
-                        advance_axis<TP>(ox, ni, (v[0] * dt) * idx, g.nx);
+        auto one = [&](long long n, bool push) {
+            TP ox = P.ox[n], oy = P.oy[n], oz = P.oz[n];
+            TP mom[3] = {P.px[n], P.py[n], P.pz[n]};
+            int ni, nj, nk;
+            decode(g, P.cell[n], ni, nj, nk);
+            TP v[3];
+            if (push) {
+                TP e3[3], b3[3];
+                if constexpr (sizeof(TP) == sizeof(float)) yee_gather<TP, TF>(g, P.cell[n], ox, oy, oz, E, B, e3, b3);
+                else tri_gather<TP, TF>(g, P.cell[n], ox, oy, oz, E, B, e3, b3);
+                boris_t<TP>(q, m, dt, beta, e3, b3, mom);
+                velocity_t<TP>(mom, m, v);
+                if (g.wall) {
+                    if (tristan_wall_x<TP>(g, ni, ox, (v[0] * dt) * idx) & 1) {   // reflectMomentumX
+                        mom[0] = -mom[0];
+                        v[0] = -v[0];
                     }
-                    advance_axis<TP>(oy, nj, (v[1] * dt) * idy, g.ny);
-                    advance_axis<TP>(oz, nk, (v[2] * dt) * idz, g.nz);
-                    P.px[n] = mom[0]; P.py[n] = mom[1]; P.pz[n] = mom[2];
-                    P.ox[n] = ox; P.oy[n] = oy; P.oz[n] = oz;
                 } else {
-                    velocity_t<TP>(mom, m, v);
+                    advance_axis<TP>(ox, ni, (v[0] * dt) * idx, g.nx);
                 }
-                deposit_global<TP>(g, fcd, ox, oy, oz, v, ni, nj, nk, Jfix);
-                P.cell[n] = (g.wall && tristan_escaped<TP>(g, ni, ox)) ? -1 : (int)lin(g, ni, nj, nk);
+                advance_axis<TP>(oy, nj, (v[1] * dt) * idy, g.ny);
+                advance_axis<TP>(oz, nk, (v[2] * dt) * idz, g.nz);
+                P.px[n] = mom[0]; P.py[n] = mom[1]; P.pz[n] = mom[2];
+                P.ox[n] = ox; P.oy[n] = oy; P.oz[n] = oz;
+            } else {
+                velocity_t<TP>(mom, m, v);
+            }
+            deposit_global<TP>(g, fcd, ox, oy, oz, v, ni, nj, nk, Jfix);
+            P.cell[n] = (g.wall && tristan_escaped<TP>(g, ni, ox)) ? -1 : (int)lin(g, ni, nj, nk);
+        };
+        if constexpr (sizeof(TP) == sizeof(float)) {
+            for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < words;
+                 w += (long long)gridDim.x * blockDim.x) {
+                unsigned bp = mp[w], bd = md[w];
+                if (!(bp | bd)) continue;
+                mp[w] = 0u;
+                md[w] = 0u;
+                while (bp | bd) {
+                    const bool push = bp != 0u;
+                    unsigned& bits = push ? bp : bd;
+                    const long long n = w * 32 + (__ffs(bits) - 1);
+                    bits &= bits - 1u;
+                    one(n, push);
+                }
+            }
+        } else {
+            // 16 words of either mask per warp, lane by lane, their set bits dealt to the lanes
+            const int lane = threadIdx.x & 31, at = lane & 15;
+            const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+            for (long long w0 = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * 16; w0 < words; w0 += warps * 16) {
+                unsigned* const mine = (lane < 16 ? mp : md) + w0 + at;
+                const unsigned bits = w0 + at < words ? *mine : 0u;
+                if (bits) *mine = 0u;
+                if (!__any_sync(0xffffffffu, bits != 0u)) continue;
+                int upto = __popc(bits);   // bits of the lanes up to this one
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, upto, d);
+                    if (lane >= d) upto += y;
+                }
+                const int total = __shfl_sync(0xffffffffu, upto, 31);
+                for (int k0 = 0; k0 < total; k0 += 32) {
+                    const int k = min(k0 + lane, total - 1);
+                    int l = 0;   // the lane that holds bit k
+#pragma unroll
+                    for (int d = 16; d > 0; d >>= 1)
+                        if (__shfl_sync(0xffffffffu, upto, l + d - 1) <= k) l += d;
+                    const unsigned word = __shfl_sync(0xffffffffu, bits, l);
+                    const int before = __shfl_sync(0xffffffffu, upto, l) - __popc(word);
+                    if (k0 + lane < total) one((w0 + (l & 15)) * 32 + (int)__fns(word, 0, k - before + 1), l < 16);
+                    __syncwarp();
+                }
             }
         }
     }

@@ -188,12 +188,13 @@ void PK<T>::implicit_deposit(cudaStream_t s, const GridP& g, PartView<T> p, doub
 template <typename T>
 void PK<T>::push_deposit_deferred(cudaStream_t s, const GridP& g, const SpeciesSet<T>& S, const void* E, const void* B,
                                   double* Jfix) {
-    // one thread per mask word
+    // FP32: one thread per mask word; FP64: one warp per 16
     long long words = 1;
     for (int q = 0; q < S.ns; ++q) words = std::max(words, (S.p[q].n + 31) / 32 + 1);
+    const long long threads = sizeof(T) == sizeof(float) ? words : 2 * words;
     // (few words hold set bits: small CTAs spread them; 128^3, 103 us per step with
     // 256 threads, 80 us with 64)
-    k_push_deposit_deferred<T, T><<<grid_for(words, 64), 64, 0, s>>>(g, S, (const T*)E, (const T*)B, Jfix);
+    k_push_deposit_deferred<T, T><<<grid_for(threads, 64), 64, 0, s>>>(g, S, (const T*)E, (const T*)B, Jfix);
 }
 
 template <typename T>
