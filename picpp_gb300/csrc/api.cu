@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/picpp_gb300.h"
+#include "explicit_split.hpp"
 #include "kernels.hpp"
 #include "nn.hpp"
 #include "solver.hpp"
@@ -269,10 +270,6 @@ pic_status smooth_moments(pic_ctx* ctx) {
 }
 
 // -------------------------------------------------------------- explicit
-// CTAs per tile of the fused kernel: two CTAs per SM run at once with FP32
-// particles, one with FP64 ones.
-int explicit_parts(const TileGeom& t, int preal) { return tile_parts(t, preal ? kNumSM : 2 * kNumSM, preal != 0); }
-
 // Work tiles of the fused explicit kernel: 8^3 cells, several of the sort's
 // tiles each, where the caller left the tiles to the library and some axis is
 // no multiple of 8 (its default tile is then smaller).  At 100x60x54 (4x4x2
@@ -352,7 +349,9 @@ pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
                 S.defer[q] = ctx->sp[q].defer;
                 S.dwords[q] = ctx->sp[q].dwords;
             }
-            const int parts = explicit_parts(ctx->wg, ctx->preal);
+            long long particles = 0;
+            for (const auto& sp : ctx->sp) particles += sp.n;
+            const int parts = explicit_parts(ctx->wg, ctx->preal, particles);
             {
                 Phase ph(ctx, PIC_PHASE_PUSH_DEPOSIT, 2);   // the fused kernel and its deferred pass
                 PK<T>::push_deposit_tiled(s, g, ctx->wg, ctx->tg, ctx->ws, S, ctx->E, ctx->B, (double*)ctx->Jpart,
@@ -680,7 +679,7 @@ pic_status pic_create(const pic_config* cfg, pic_ctx** out) {
         ok = ok && A(&ctx->J, sizeof(double) * 3 * N);
         ok = ok && A(&ctx->Jfix, sizeof(double) * 3 * N);
         ok = ok && A(&ctx->Jpart, sizeof(double) * 3 * (size_t)ctx->ws.jcells * ctx->wg.ntx * ctx->wg.nty * ctx->wg.ntz *
-                                   explicit_parts(ctx->wg, ctx->preal));
+                                   explicit_parts(ctx->wg, ctx->preal, LLONG_MAX));
     } else {
         ctx->pi_len = c.pressure_compat ? 9LL * ga.cex * ga.cey * ga.cez : 9 * N;
         ctx->jg_len = c.pressure_compat ? 3LL * ctx->nex * ctx->ney * ctx->nez : 3 * N;

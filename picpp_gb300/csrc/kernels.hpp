@@ -30,24 +30,6 @@ inline int red_blocks(long long n) {
     return (int)b;
 }
 
-// CTAs that share one tile's particles in the fused explicit kernel, of which
-// `slots` run at once.  A box with fewer tiles than that
-// would leave SMs idle: its tiles are cut into as many parts as still run in
-// one wave.  `even`: larger boxes are cut too where that fills the last wave
-// (the FP64 explicit kernel, milliseconds per tile: staging a tile again costs
-// nothing beside them), by the fewest parts up to 4 that leave 6% of it idle.
-inline int tile_parts(const TileGeom& t, int slots, bool even) {
-    const int n = t.ntx * t.nty * t.ntz;
-    if (n < slots) return slots / n;
-    int best = 1;
-    double most = 0;
-    for (int p = 1; even && p <= 4 && most < 0.94; ++p) {
-        const double waves = (double)n * p / slots, use = waves / std::ceil(waves);
-        if (use > most + 0.02) { most = use; best = p; }
-    }
-    return best;
-}
-
 template <typename T>
 struct PK {
     // with GridP::wall the B half step first sets the ghost column left of
@@ -59,7 +41,7 @@ struct PK {
     static void zigzag(cudaStream_t s, const GridP& g, PartView<T> p, double q, double m, double w, double* J);
     // fused gather/push/deposit over work tiles t of shape sh (boris_tile.cuh),
     // each one or several tiles o of the sort, `parts` CTAs and partial blocks
-    // per work tile (tile_parts)
+    // per work tile (explicit_split.hpp)
     static void push_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t, const TileGeom& o, const TileShape& sh,
                                    const SpeciesSet<T>& S, const void* E, const void* B, double* Jpart, int parts);
     // J from the tile partials and Jfix; inv_scale = 1 / fixed_scale for FP32
