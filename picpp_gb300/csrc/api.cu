@@ -51,7 +51,7 @@ struct pic_ctx {
     GridP g{};
     TileGeom tg{};
     TileShape ts{};
-    TileGeom wg{};          // work tiles of the fused explicit kernel (merge_geom) and their shape
+    TileGeom wg{};          // work tiles of the fused explicit kernel (work_tiles; else the sort's) and their shape
     TileShape ws{};
     TileGeom mg{};          // work boxes of the implicit mover (mover_boxes)
     GhostAxes ga{};
@@ -270,27 +270,6 @@ pic_status smooth_moments(pic_ctx* ctx) {
 }
 
 // -------------------------------------------------------------- explicit
-// Work tiles of the fused explicit kernel: 8^3 cells, several of the sort's
-// tiles each, where the caller left the tiles to the library and some axis is
-// no multiple of 8 (its default tile is then smaller).  At 100x60x54 (4x4x2
-// tiles of 288 particles per species) a CTA per tile spent its time staging
-// and flushing halo: 428 us per step, 273 us with work tiles.  Axes below 8 cells
-// keep the sort's tiles: a work tile would wrap onto itself.
-void merge_geom(const pic_config& c, const TileGeom& t, TileGeom& w, TileShape& ws) {
-    const int n[3] = {c.nx, c.ny, c.nz}, e[3] = {t.tx, t.ty, t.tz};
-    bool small = false;
-    for (int a = 0; a < 3; ++a) {
-        if (c.tile[a] > 0 || n[a] < 8 || 8 % e[a] != 0) return;
-        small = small || e[a] < 8;
-    }
-    if (!small || c.boundary_x != PIC_BOUNDARY_PERIODIC) return;
-    w.tx = w.ty = w.tz = 8;
-    w.ntx = (n[0] + 7) / 8; w.nty = (n[1] + 7) / 8; w.ntz = (n[2] + 7) / 8;
-    w.lx = w.ly = w.lz = 3;
-    ws.fx = ws.fy = ws.fz = ws.jx = ws.jy = ws.jz = 12;
-    ws.jcells = 12 * 12 * 12;
-}
-
 // Work boxes of the implicit mover: as even as the axes allow, up to 8 cells per
 // axis in whole tiles of the sort, where the caller left the tiles to the
 // library (k_implicit_push_tile has both sides' times).  FP64 fields of 8^3 cells
@@ -351,11 +330,14 @@ pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
             }
             long long particles = 0;
             for (const auto& sp : ctx->sp) particles += sp.n;
-            const int parts = explicit_parts(ctx->wg, ctx->preal, particles);
+            const long long filled = g.wall ? (long long)std::max(1, g.nx - 2 - kTristanWallNode) * g.ny * g.nz : g.N;
+            const ExplicitSplit split = explicit_split(ctx->tg, ctx->wg, filled, ctx->preal, S.ns, particles);
+            const TileGeom& wg = split.work ? ctx->wg : ctx->tg;
+            const TileShape& ws = split.work ? ctx->ws : ctx->ts;
+            const int parts = split.parts;
             {
                 Phase ph(ctx, PIC_PHASE_PUSH_DEPOSIT, 2);   // the fused kernel and its deferred pass
-                PK<T>::push_deposit_tiled(s, g, ctx->wg, ctx->tg, ctx->ws, S, ctx->E, ctx->B, (double*)ctx->Jpart,
-                                          parts);
+                PK<T>::push_deposit_tiled(s, g, wg, ctx->tg, ws, S, ctx->E, ctx->B, (double*)ctx->Jpart, parts);
                 PK<T>::push_deposit_deferred(s, g, S, ctx->E, ctx->B, ctx->Jfix);
             }
             {
@@ -364,7 +346,7 @@ pic_status buneman_steps(pic_ctx* ctx, int nsteps) {
             }
             {
                 Phase ph(ctx, PIC_PHASE_ASSEMBLE, 1);
-                PK<T>::assemble_j(s, g, ctx->wg, ctx->ws, (const double*)ctx->Jpart, ctx->Jfix, ctx->J,
+                PK<T>::assemble_j(s, g, wg, ws, (const double*)ctx->Jpart, ctx->Jfix, ctx->J,
                                   1.0 / (double)PK<T>::fixed_scale(g, S), parts);
             }
         } else {
@@ -651,7 +633,7 @@ pic_status pic_create(const pic_config* cfg, pic_ctx** out) {
     }
     ctx->wg = t;
     ctx->ws = ts;
-    merge_geom(c, t, ctx->wg, ctx->ws);
+    work_tiles(c, t, ctx->wg, ctx->ws);
     ctx->mg = mover_boxes(c, t);
     GhostAxes& ga = ctx->ga;
     ga.cex = c.nx > 1 ? c.nx + 4 : 1; ga.cey = c.ny > 1 ? c.ny + 4 : 1; ga.cez = c.nz > 1 ? c.nz + 4 : 1;
@@ -678,8 +660,7 @@ pic_status pic_create(const pic_config* cfg, pic_ctx** out) {
         ok = ok && A(&ctx->B, ctx->rsz * 3 * N);
         ok = ok && A(&ctx->J, sizeof(double) * 3 * N);
         ok = ok && A(&ctx->Jfix, sizeof(double) * 3 * N);
-        ok = ok && A(&ctx->Jpart, sizeof(double) * 3 * (size_t)ctx->ws.jcells * ctx->wg.ntx * ctx->wg.nty * ctx->wg.ntz *
-                                   explicit_parts(ctx->wg, ctx->preal, LLONG_MAX));
+        ok = ok && A(&ctx->Jpart, sizeof(double) * partial_cells(t, ts, ctx->wg, ctx->ws, ctx->preal));
     } else {
         ctx->pi_len = c.pressure_compat ? 9LL * ga.cex * ga.cey * ga.cez : 9 * N;
         ctx->jg_len = c.pressure_compat ? 3LL * ctx->nex * ctx->ney * ctx->nez : 3 * N;

@@ -33,7 +33,7 @@ void PK<T>::push_deposit_tiled(cudaStream_t s, const GridP& g, const TileGeom& t
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
         attr_set = true;
     }
-    const bool merge = t.tx != o.tx || t.ty != o.ty || t.tz != o.tz;   // (merge_geom: 8^3 work tiles)
+    const bool merge = t.tx != o.tx || t.ty != o.ty || t.tz != o.tz;   // (work_tiles: 8^3 cells)
     const bool cube8 = t.tx == 8 && t.ty == 8 && t.tz == 8 && g.y3 && g.z3 && sh.fx == 12 && sh.fy == 12 &&
                        sh.fz == 12 && sh.jx == 12 && sh.jy == 12 && sh.jz == 12;
     const int grid = std::min(t.ntx * t.nty * t.ntz * parts, kNumSM * 8);
