@@ -12,7 +12,12 @@ namespace pic {
 // clock): the products are factored, six for the eight weights' parts and five
 // per corner, and the one division is by a constant (4.2 million particles:
 // 852 us with each corner's weights multiplied out and p^2 divided by m^2).
-template <typename T>
+// kTurn, for boxes of few cells with many particles each, where the adds to the few
+// addresses are the time: each warp of a CTA begins at another corner (8^3 cells, 1,000
+// per species and cell, FP32 and FP64: 1,277 and 1,346 us; all from the first corner 1,558 and
+// 1,632, and with the weights multiplied out, which left more time between the
+// adds, 1,387 and 1,395.  8^3 with 100: 115, 126, 130).
+template <typename T, bool kTurn>
 __global__ void __launch_bounds__(256) k_density_deposit(GridP g, PartView<T> p, double m, double w,
                                                          double* __restrict__ conc, double* __restrict__ energy,
                                                          double* __restrict__ mom) {
@@ -31,9 +36,10 @@ __global__ void __launch_bounds__(256) k_density_deposit(GridP g, PartView<T> p,
         const double yz[4] = {y0 * z0, y1 * z0, y0 * z1, y1 * z1};
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            if ((!g.y3 && (q & 2)) || (!g.z3 && (q & 4))) continue;
-            const long long id = lin(g, X[q & 1], Y[(q >> 1) & 1], Z[q >> 2]);
-            const double s = (q & 1 ? x1 : x0) * yz[q >> 1];
+            const int c = kTurn ? (q + (int)(threadIdx.x >> 5)) & 7 : q;
+            if ((!g.y3 && (c & 2)) || (!g.z3 && (c & 4))) continue;
+            const long long id = lin(g, c & 1 ? X[1] : X[0], c & 2 ? Y[1] : Y[0], c & 4 ? Z[1] : Z[0]);
+            const double s = (c & 1 ? x1 : x0) * (c & 4 ? (c & 2 ? yz[3] : yz[2]) : (c & 2 ? yz[1] : yz[0]));
             atomicAdd(&conc[id], s);
             atomicAdd(&energy[id], s * gm);
             atomicAdd(&mom[id], s * px);
