@@ -209,9 +209,10 @@ template <typename T>
 void PK<T>::density_deposit(cudaStream_t s, const GridP& g, PartView<T> p, double m, double w, double* conc,
                             double* energy, double* mom) {
     if (p.n == 0) return;
-    // (from 32^3 cells on the adds meet seldom enough: 64 per species and cell, 1,139 us
-    // either way; 64^3 with 8, 761 us, 847 with the corners turned)
-    auto* kernel = g.N <= 4096 && p.n >= 100 * g.N ? k_density_deposit<T, true> : k_density_deposit<T, false>;
+    // (with fewer particles, and from 32^3 cells on, the adds meet seldom enough: 32^3 with
+    // 64 per species and cell 1,139 us, 1,132 with the corners turned, with 16 251 and
+    // 259; 64^3 with 8 761 and 847; 16^3 with 30 136 and 120)
+    auto* kernel = g.N <= 4096 && p.n >= 20 * g.N ? k_density_deposit<T, true> : k_density_deposit<T, false>;
     kernel<<<grid_for(p.n, 256, 32), 256, 0, s>>>(g, p, m, w, conc, energy, mom);
 }
 
