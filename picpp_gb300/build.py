@@ -3,8 +3,9 @@
     python -m picpp_gb300.build        (or picpp_gb300.build.build())
 
 Translation units compile in parallel with nvcc; the FP64 particle kernels
-(but the per-tile ones) use --fmad=false so that their arithmetic rounds like
-the CPU oracle.
+(but the per-tile ones) use --fmad=false: every multiply and add rounds by
+itself, as in the CPU oracle.  (The implicit path's quotients are products with
+a reciprocal in FP64 too, and its Picard tests compare squares.)
 """
 from __future__ import annotations
 

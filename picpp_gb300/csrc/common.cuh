@@ -90,7 +90,8 @@ template <> __device__ __forceinline__ float divd<float>(float a, float, float i
 // rounded, whatever code stands around them.  Left to the compiler, the
 // choice of which product of a sum is fused changes with the surrounding code,
 // and a particle within a rounding of a cell face then takes the other zigzag
-// path.  (FP64: separate operations, as the oracle's.)
+// path.  (FP64: plain operations, rounded as their translation unit says, each by
+// itself in kernels_f64.cu, fused where the compiler can in kernels_f64_tile.cu.)
 template <typename T> __device__ __forceinline__ T fmadd(T a, T b, T c) { return a * b + c; }
 template <> __device__ __forceinline__ float fmadd<float>(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 template <typename T> __device__ __forceinline__ T mulr(T a, T b) { return a * b; }

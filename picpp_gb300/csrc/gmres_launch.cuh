@@ -40,6 +40,15 @@ static cudaError_t gmres_grid(cudaStream_t s, const GmresArgs& a) {
 // and the neighbours of each choice:
 //   256: 306     128: 435     736: 1,506   480: 3,292    736: 19,857
 // (128x64x32: 480 1,754, 736 2,007; 128x128x64: 736 5,720, 992 5,429.)
+// The reference method to its own stop (20 to 31 columns; two dot products per
+// vector, so half as many vectors per pass: with KB doubled every box takes 1% to
+// 17% longer), us per solve:
+//   32x32x1      32x32x24     64x64x32     128x128x32    256x256x64
+//   128: 397     256: 881     480: 2,325   736: 7,574    992: 55,209
+//   256: 443     128: 1,269   736: 3,321   480: 7,831    736: 58,282
+// (16x16x16: 128 592, 256 617; 26x20x18: 256 682, 128 851; 40x40x40: 480 1,442, 256
+// 1,540; 96x64x64: 480 6,053, 736 6,224; 128x128x48: 736 11,683, 480 10,781, 992
+// 11,605; 128x128x64: 992 14,120, 736 15,356.)
 cudaError_t launch_gmres_grid(cudaStream_t s, const GmresArgs& a) {
     cudaError_t e = cudaMemsetAsync(a.bar, 0, 2 * sizeof(unsigned), s);
     if (e != cudaSuccess) return e;

@@ -182,7 +182,14 @@ bool PK<T>::implicit_push_tiled(cudaStream_t s, const GridP& g, const TileGeom& 
     // for staging the box.  FP64 particles, ten times as long in work, are cut as
     // fine as that allows (pairs of 61x43x1: 6 CTAs per box 511 us, 25 413 us);
     // FP32 as little (40x56x56: one CTA per box 806 us, five 760 us; 64x64x16: 2
-    // 475 us, 7 435 us).
+    // 475 us, 7 435 us).  192 and 4,096 particles: what a CTA moves in the time that it
+    // stages its box; p goes to four waves, and a dozen more where a box is one of few.
+    // us of a call (with its launch) by p, (p) the choice:
+    //   FP64 32x32x1, 32 per species and cell: 1 625, 4 175, 8 102, (19) 104, 64 116
+    //        16x16x16, 8: 1 1,653, 8 239, 16 137, (38) 148, 64 166;  61x43x1, 32: 1 630, 8 254, (18) 229
+    //        26x20x18, 16: 1 640, 8 489, (14) 444, 64 537
+    //   FP32 26x20x18, 16: 1 153, (8) 59, 16 69, 64 144;  16x16x16, 8: 1 111, 8 48, 16 43, (38) 44, 64 57
+    //        39x57x53, 20: (1) 302, 2 307, 8 390;  112x51x5, 24: 1 189, (3) 104, 4 148, 8 140
     const int n = t.ntx * t.nty * t.ntz, slots = (int)std::min<size_t>(2, 228 * 1024 / (most_smem + 1024)) * kNumSM;
     long long total = 0;
     for (int q = 0; q < S.ns; ++q) total += S.p[q].n;
