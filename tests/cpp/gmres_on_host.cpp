@@ -67,6 +67,7 @@ int main(int argc, char** argv) {
     a.mu = mu.data(); a.b = b.data(); a.x = x.data(); a.V = V.data(); a.mx = mx.data(); a.w = w.data(); a.r = r.data();
     a.part = part.data(); a.bar = bar; a.out = out.data();
     a.polls = std::atoi(argv[5]) > 0 ? (unsigned)std::atoi(argv[5]) : kGmresPolls;
+    if (a.polls != kGmresPolls) late_ms = 1000;   // longer than the others take for their polls
     late_cta = std::atoi(argv[3]);
     late_at = std::atoi(argv[4]);
     if (a.reference) run<true>(a, ctas);
